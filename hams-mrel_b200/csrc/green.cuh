@@ -209,17 +209,16 @@ struct TableModes {
   __device__ __forceinline__ double fldt(int i) const { return t.fldt[(size_t)i * t.tn + f]; }
 };
 
-// EIGEN, FinGreen3D.f90:281-362 (R/h >= 0.5)
-template <class MD>
-__device__ inline void eigen(double r, double zf, double zp, double wk, const double* __restrict__ wvn, double h,
-                             cplx g[3], const MD& md) {
-  double zfh = zf + h, zph = zp + h;
-  prop_mode(r, zfh, zph, wk, h, g);
+// The evanescent modes of EIGEN, FinGreen3D.f90:324-347; bk supplies K0 and
+// K1 of km r for mode i.
+template <class MD, class BK>
+__device__ __forceinline__ void eigen_modes(double r, const double* __restrict__ wvn, cplx g[3], const MD& md,
+                                            const BK& bk) {
   for (int i = 2; i <= 10; ++i) {
     double km = wvn[i - 1];
     double pm = md.pm(i);
     double k0, k1, skzf, ckzf;
-    ik01a(km * r, k0, k1);
+    bk(i, km, r, k0, k1);
     md.src(i, skzf, ckzf);
     double ckzp = md.fld(i);
     double rm0 = pm * k0 * ckzf * ckzp, rm1 = -pm * km * k1 * ckzf * ckzp, rm2 = -pm * km * k0 * skzf * ckzp;
@@ -228,6 +227,21 @@ __device__ inline void eigen(double r, double zf, double zp, double wk, const do
     g[2].re += rm2;
     if (fabs(rm0) < HAMS_F4(1.E-6) && fabs(rm1) < HAMS_F4(1.E-6) && fabs(rm2) < HAMS_F4(1.E-6)) break;
   }
+}
+
+struct BesselInline {
+  __device__ __forceinline__ void operator()(int, double km, double r, double& k0, double& k1) const {
+    ik01a(km * r, k0, k1);
+  }
+};
+
+// EIGEN, FinGreen3D.f90:281-362 (R/h >= 0.5)
+template <class MD>
+__device__ inline void eigen(double r, double zf, double zp, double wk, const double* __restrict__ wvn, double h,
+                             cplx g[3], const MD& md) {
+  double zfh = zf + h, zph = zp + h;
+  prop_mode(r, zfh, zph, wk, h, g);
+  eigen_modes(r, wvn, g, md, BesselInline{});
   remove_rankine(r, zf, zp, g);
 }
 
@@ -294,13 +308,18 @@ __device__ inline void pidcock_images(double r, double zf, double zp, double h, 
     p2[m] = pow(t2, 2.0 * m);
     p3[m] = pow(t3, 2.0 * m);
   }
+  double o1[5], o23[5];
+  for (int m = 1; m <= 4; ++m) {
+    o1[m] = pow(t1, 2.0 * m - 1.0);
+    o23[m] = pow(t2, 2.0 * m - 1.0) + pow(t3, 2.0 * m - 1.0);
+  }
   double q0 = 0.0, q1 = 0.0, q2 = 0.0;
   for (int m = 0; m <= 4; ++m)
     for (int n = 0; n <= 4; ++n) {
       double amn = c_amn[m + 5 * n];
       q0 += amn * p1[m] * (p2[n] + p3[n]);
-      if (m >= 1) q1 += 2.0 * m * amn * pow(t1, 2.0 * m - 1.0) * (p2[n] + p3[n]);
-      if (n >= 1) q2 += 2.0 * n * amn * p1[m] * (pow(t2, 2.0 * n - 1.0) + pow(t3, 2.0 * n - 1.0));
+      if (m >= 1) q1 += 2.0 * m * amn * o1[m] * (p2[n] + p3[n]);
+      if (n >= 1) q2 += 2.0 * n * amn * p1[m] * o23[n];
     }
   gs = (s0 - 2.0 + q0) / h;
   gr = (-s1 + q1) / (h * h);

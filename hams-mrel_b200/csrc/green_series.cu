@@ -8,54 +8,329 @@
 // transcendental functions inside them come from detmath.h.  The remaining
 // kernels (hams_gpu.cu) keep fused multiply-adds.
 #include "kernels.cuh"
+#include "epsilon.h"
 #include "rankine.cuh"
 
-// 128 threads and at most 64 registers per thread (8 blocks per SM): the
-// series are latency-bound, and the extra resident warps outweigh the few
-// spills (measured on the 5,400-panel array: EIGENE 54 ms at 116 registers,
-// 38 ms at 64).
-template <int BR, int N>
-__global__ void __launch_bounds__(128, 8) k_green_series(DevGeom g, WaveDev w, const double* __restrict__ wvn,
-                                                      hams::ModeTab mt, const uint32_t* __restrict__ pairs,
-                                                      long long count, const double* __restrict__ rs,
-                                                      const double* __restrict__ rd, double2* __restrict__ A,
-                                                      double2* __restrict__ S, int* ovf) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  size_t p = pairs[t];
-  int i = (int)(p % (size_t)g.tn), j = (int)(p / (size_t)g.tn);
-  int flag = near_flag(g, i, j);
-  double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], zp = g.fxyz[i + 2 * g.tn];
-  double xq = g.xq[j], yq = g.xq[j + g.n], zq = g.xq[j + 2 * g.n];
-  grn4 G;
-  if (w.limit) {
-    G = hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag);
-  } else {
-    hams::SeriesScratchN<N> sc;
-    hams::TableModes md{mt, j, i};
-    int o = 0;
-    G = hams::fingreen3d<BR>(xq, xp, yq, yp, zq, zp, w.v, wvn, w.h, flag, &sc, &o, md);
-    if (o) atomicOr(ovf, 1);
-  }
-  store_pair(g, p, i, j, G, rs, rd, A, S);
+// Horizontal distance of a pair, as fingreen3d of this file rounds it.
+__device__ __forceinline__ double pair_distance(const DevGeom& g, uint32_t p) {
+  const uint32_t tn = (uint32_t)g.tn;
+  const int j = (int)(p / tn), i = (int)(p - (uint32_t)j * tn);
+  const double xpq = g.xq[j] - g.fxyz[i], ypq = g.xq[j + g.n] - g.fxyz[i + g.tn];
+  return sqrt(xpq * xpq + ypq * ypq);
 }
 
-void launch_green_series(int br, unsigned blocks, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,
-                         const hams::ModeTab& mt, const uint32_t* pairs, long long count, const double* rs,
-                         const double* rd, double2* A, double2* S, int* ovf) {
+__global__ void k_series_distance(DevGeom g, const uint32_t* __restrict__ pairs, long long count,
+                                  double* __restrict__ r) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < count) r[t] = pair_distance(g, pairs[t]);
+}
+
+void launch_series_distance(cudaStream_t st, DevGeom g, const uint32_t* pairs, long long count, double* r) {
+  k_series_distance<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(g, pairs, count, r);
+}
+
+// Series length of a distance (FinGreen3D.f90:434, :592)
+template <int BR>
+__device__ __forceinline__ int series_terms(double r, double h) {
+  const double rhp = fabs(r / h);
+  return BR == hams::kPidcock ? (int)(HAMS_F4(-1010.10) * rhp + HAMS_F4(100.50))
+                              : (int)(HAMS_F4(-88.89) * rhp + HAMS_F4(54.45));
+}
+template <int BR>
+constexpr int series_max() {
+  return BR == hams::kPidcock ? hams::kPidcockMax : hams::kEigenEMax;
+}
+
+// The radial table of a branch: one thread per (distance, mode), blockIdx.y
+// the mode (0: the propagating mode's J and Y).  The threads of a warp hold
+// neighbouring distances of one mode, so the loops of ik01a end together.
+template <int BR>
+__global__ void __launch_bounds__(128) k_rad_series(DevGeom g, WaveDev w, const double* __restrict__ wvn,
+                                                    const double* __restrict__ ur, const uint32_t* __restrict__ pairs,
+                                                    long long count, double* __restrict__ kt,
+                                                    double4* __restrict__ jy) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const double r = ur ? ur[t] : pair_distance(g, pairs[t]);
+  if (blockIdx.y == 0) {
+    double4 v;
+    hams::jy01b(wvn[0] * r, v.x, v.y, v.z, v.w);
+    jy[t] = v;
+    return;
+  }
+  const int i = blockIdx.y + 1;
+  if (i > min(series_terms<BR>(r, w.h), series_max<BR>())) return;
+  double k0, k1;
+  hams::ik01a(wvn[i - 1] * r, k0, k1);
+  if (BR == hams::kPidcock) {
+    const double umt = (i - 1) * 3.141592653589793 / w.h;
+    double k0t, k1t;
+    hams::ik01a(umt * r, k0t, k1t);
+    reinterpret_cast<double2*>(kt)[(size_t)t * (rad_stride(BR) / 2) + 2 * (i - 2)] = make_double2(k0, k1);
+    reinterpret_cast<double2*>(kt)[(size_t)t * (rad_stride(BR) / 2) + 2 * (i - 2) + 1] = make_double2(k0t, k1t);
+  } else {
+    reinterpret_cast<double2*>(kt)[(size_t)t * (rad_stride(BR) / 2) + (i - 2)] = make_double2(k0, k1);
+  }
+}
+
+void launch_rad_series(int br, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, const double* ur,
+                       const uint32_t* pairs, long long count, double* kt, double4* jy) {
   if (br == hams::kPidcock)
-    k_green_series<hams::kPidcock, hams::kPidcockMax>
-        <<<blocks, 128, 0, st>>>(g, w, wvn, mt, pairs, count, rs, rd, A, S, ovf);
+    k_rad_series<hams::kPidcock><<<dim3((unsigned)((count + 127) / 128), hams::kPidcockMax), 128, 0, st>>>(
+        g, w, wvn, ur, pairs, count, kt, jy);
   else
-    k_green_series<hams::kEigenE, hams::kEigenEMax>
-        <<<blocks, 128, 0, st>>>(g, w, wvn, mt, pairs, count, rs, rd, A, S, ovf);
+    k_rad_series<hams::kEigenE><<<dim3((unsigned)((count + 127) / 128), hams::kEigenEMax), 128, 0, st>>>(
+        g, w, wvn, ur, pairs, count, kt, jy);
+}
+
+// One term of table T (0: G, 1: dG/dR, 2: dG/dz) of mode i, FinGreen3D.f90:
+// 446-470 (EIGENE) and :597-627 (PIDCOCK).
+template <int BR>
+struct SeriesTerm {
+  const double* __restrict__ wvn;
+  const double* __restrict__ pm;
+  const double* __restrict__ ac;
+  const double* __restrict__ kt;    // the pair's radial row, at K0 or K1
+  const double* __restrict__ src;   // the source panel's sin or cos of mode 0, stride sn
+  const double* __restrict__ srct;
+  const double* __restrict__ fld;   // the field point's cos of mode 0, stride fn
+  const double* __restrict__ fldt;
+  size_t sn, fn;
+  double h;
+  int table;
+  __device__ __forceinline__ double operator()(int i) const {
+    if (BR == hams::kEigenE) {
+      const double p = pm[i], c = table == 0 ? p : -p * wvn[i - 1];
+      return c * kt[2 * (i - 2)] * src[i * sn] * fld[i * fn];
+    }
+    const double um = wvn[i - 1], umt = (i - 1) * 3.141592653589793 / h, a = ac[i];
+    const double su = src[i * sn], sut = srct[i * sn], cup = fld[i * fn], cutp = fldt[i * fn];
+    const double k = kt[4 * (i - 2)], kk = kt[4 * (i - 2) + 2];
+    if (table == 2) {
+      const double dam = -um * a * su * cup, damt = -umt * sut * cutp / h;
+      return dam * k - damt * kk;
+    }
+    const double am = a * su * cup, amt = sut * cutp / h;
+    return table == 0 ? am * k - amt * kk : -um * am * k + umt * amt * kk;
+  }
+};
+
+// The same table in the reference's column order, for the rare sequences whose
+// row-ordered pass asks for it (epsilon.h).
+template <int BR>
+__device__ __noinline__ double series_columns(const SeriesTerm<BR>& term, int nt) {
+  double s[series_max<BR>()], a[series_max<BR>()];
+  s[0] = 0.0;
+  for (int i = 2; i <= nt; ++i) s[i - 1] = s[i - 2] + term(i);
+  return hams::limes(nt - 1, s, a);
+}
+
+// Pidcock's image sum of one table (IMGS/DGSR/DGSZ), as pidcock_images.
+__device__ __noinline__ double pidcock_image(int table, double r, double zf, double zp, double h) {
+  const double t1 = r / h, t2 = (zf - zp) / h, t3 = (zf + zp + 2.0 * h) / h;
+  double s = 0.0, q = 0.0;
+  for (int l = -1; l <= 1; ++l) {
+    const double a = t2 + 2.0 * l, b = t3 + 2.0 * l;
+    const double ra = sqrt(t1 * t1 + a * a), rb = sqrt(t1 * t1 + b * b);
+    if (table == 0) s += 1.0 / ra + 1.0 / rb;
+    else if (table == 1) s += t1 / (ra * ra * ra) + t1 / (rb * rb * rb);
+    else s += a / (ra * ra * ra) + b / (rb * rb * rb);
+  }
+  double p1[5], p23[5];
+  for (int m = 0; m <= 4; ++m) {
+    p1[m] = table == 1 ? pow(t1, 2.0 * m - 1.0) : pow(t1, 2.0 * m);
+    p23[m] = table == 2 ? pow(t2, 2.0 * m - 1.0) + pow(t3, 2.0 * m - 1.0) : pow(t2, 2.0 * m) + pow(t3, 2.0 * m);
+  }
+  for (int m = 0; m <= 4; ++m)
+    for (int n = 0; n <= 4; ++n) {
+      const double amn = hams::c_amn[m + 5 * n];
+      if (table == 0) q += amn * p1[m] * p23[n];
+      else if (table == 1 && m >= 1) q += 2.0 * m * amn * p1[m] * p23[n];
+      else if (table == 2 && n >= 1) q += 2.0 * n * amn * p1[m] * p23[n];
+    }
+  return table == 0 ? (s - 2.0 + q) / h : (-s + q) / (h * h);
+}
+
+// EIGENE and PIDCOCK pairs.  Three warps share 32 pairs, one per epsilon table
+// (G, dG/dR, dG/dz): a table's chain of reciprocals is the pair's latency, and
+// the three are independent.  The partial sums go through the epsilon table in
+// blocks of 8 rows kept in registers (epsilon.h), so that 8 reciprocals are in
+// flight per thread; the last row of each block (8 bytes per column) and the
+// largest |a| per column pair (4 bytes) are in shared memory, sized for the
+// launch's longest series (rows terms).
+// Issue-bound: about 18 instructions per table entry, 8 of them FP64 (the FP64
+// pipe is at half its rate).  Against one thread per pair with the Bessel
+// functions in the loop and the tables column by column in local memory
+// (5,400 panels, every pair): EIGENE 36.8 -> 13.3 ms for 11.2 M pairs, PIDCOCK
+// 16.0 -> 7.8 ms for 0.63 M.  Blocks of 4 or 6 rows (more warps, more columns
+// read and written per entry) measured the same within 3 %, one loop body for
+// all columns (less code, idle rows computed) 6-20 % slower.
+constexpr int kSerThreads = 96;
+template <int BR>
+__global__ void __launch_bounds__(kSerThreads, 5) k_green_series(DevGeom g, WaveDev w, const double* __restrict__ wvn,
+                                                                 hams::ModeTab mt, RadTab rt,
+                                                                 const uint32_t* __restrict__ pairs, long long count,
+                                                                 const double* __restrict__ rs,
+                                                                 const double* __restrict__ rd,
+                                                                 double2* __restrict__ A, double2* __restrict__ S,
+                                                                 int* ovf, int rows) {
+  extern __shared__ double sm[];
+  __shared__ double2 dz[32];
+  const int table = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the list is sorted by series length: the longest first
+  const long long t0 = ((long long)gridDim.x - 1 - blockIdx.x) * 32 + lane;
+  const bool live = t0 < count;
+  const long long t = live ? t0 : count - 1;
+  const uint32_t p = pairs[t], tn = (uint32_t)g.tn;
+  const int j = (int)(p / tn), i = (int)(p - (uint32_t)j * tn);
+  const int flag = near_flag(g, i, j);
+  const double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], zp = g.fxyz[i + 2 * g.tn];
+  const double xq = g.xq[j], yq = g.xq[j + g.n], zq = g.xq[j + 2 * g.n];
+  if (w.limit) {
+    if (table == 0 && live)
+      store_pair(g, p, i, j, hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag), rs, rd, A, S);
+    return;
+  }
+  const double xpq = xq - xp, ypq = yq - yp, zpq = zq + zp, h = w.h;
+  const double rr = sqrt(xpq * xpq + ypq * ypq);
+  const uint32_t row = rt.rid ? rt.rid[t] - rt.base : (uint32_t)t;
+
+  // the extrapolated sum of this warp's table
+  int nt = series_terms<BR>(rr, h);
+  if (nt > rows) {  // outside the branch's range of R/h
+    atomicOr(ovf, 1);
+    nt = rows;
+  }
+  SeriesTerm<BR> term;
+  term.wvn = wvn;
+  term.pm = mt.pm;
+  term.ac = mt.ac;
+  term.kt = rt.kt + (size_t)row * rad_stride(BR) + (table == 1 ? 1 : 0);
+  term.src = reinterpret_cast<const double*>(mt.src + j) + (table == 2 ? 0 : 1);
+  term.srct = reinterpret_cast<const double*>(mt.srct + j) + (table == 2 ? 0 : 1);
+  term.fld = mt.fld + i;
+  term.fldt = mt.fldt + i;
+  term.sn = 2 * (size_t)g.n;
+  term.fn = (size_t)g.tn;
+  term.h = h;
+  term.table = table;
+  double l;
+  {
+    double* e = sm + threadIdx.x;
+    uint32_t* m = reinterpret_cast<uint32_t*>(sm + (size_t)hams::eps_columns(rows) * kSerThreads) + threadIdx.x;
+    hams::EpsBest best;
+    // the first block holds the rows that full blocks do not divide; a row's
+    // sum s_q adds mode q + 1, and s_0 = 0
+    const int r0 = (nt - 1) % hams::kEpsRows + 1, pad = hams::kEpsRows - r0;
+    double x[hams::kEpsRows], s = 0.0;
+#pragma unroll
+    for (int k = 0; k < hams::kEpsRows; ++k) {
+      if (k > pad) s += term(k - pad + 1);
+      x[k] = s;
+    }
+    hams::eps_block(x, 0, pad, e, m, kSerThreads, r0 < nt, best);
+    for (int q = r0; q < nt; q += hams::kEpsRows) {
+#pragma unroll
+      for (int k = 0; k < hams::kEpsRows; ++k) x[k] = term(q + k + 1);
+#pragma unroll
+      for (int k = 0; k < hams::kEpsRows; ++k) {
+        s += x[k];
+        x[k] = s;
+      }
+      hams::eps_block(x, q, 0, e, m, kSerThreads, q + hams::kEpsRows < nt, best);
+    }
+    l = best.redo ? series_columns<BR>(term, nt) : hams::eps_result(best, s);
+  }
+
+  // this table's component of G: the propagating mode, the series, minus the
+  // Rankine terms, plus the point sources (FINGREEN3D)
+  const double wk = wvn[0], czp = mt.fld[g.tn + i];
+  const double2 szf = mt.src[g.n + j];  // sinh, cosh of k0 (zq + h)
+  const double4 jy = rt.jy[row];
+  const double p0 = mt.pm[1] * szf.y * czp;
+  // the distances to the source and its image, with which FINGREEN3D both
+  // removes and adds the point sources
+  const double r = sqrt(rr * rr + (zq - zp) * (zq - zp)), r1 = sqrt(rr * rr + zpq * zpq);
+  cplx v;
+  if (BR == hams::kEigenE) {
+    if (table == 0) v = hams::cmk(-p0 * jy.z, p0 * jy.x);
+    else if (table == 1) v = hams::cmk(wk * p0 * jy.w, -wk * p0 * jy.y);
+    else {
+      const double dp0 = mt.pm[1] * szf.x * czp;
+      v = hams::cmk(-wk * dp0 * jy.z, wk * dp0 * jy.x);
+    }
+    v.re += l;
+  } else {
+    if (table == 0) v = hams::cmk(-p0 * jy.z + 2.0 / h * (0.5772156649015328 + log(rr / 4.0 / h)), p0 * jy.x);
+    else if (table == 1) v = hams::cmk(wk * p0 * jy.w + 2.0 / (rr * h), -wk * p0 * jy.y);
+    else {
+      const double dp0 = mt.ac[1] * szf.x * czp;
+      v = hams::cmk(-dp0 * jy.z, dp0 * jy.x);
+    }
+    v.re = v.re + 4.0 * l + pidcock_image(table, rr, zq, zp, h);
+  }
+  const double ir1 = 1.0 / r1, ir13 = ir1 * ir1 * ir1, ir = 1.0 / r, ir3 = ir * ir * ir;
+  if (table == 0) {
+    v.re -= (ir + ir1);
+    v.re += flag == 1 ? ir1 : ir1 + ir;
+    if (live) {
+      const double ds = g.ds[j];
+      S[p] = make_double2(rs[p] + v.re * ds, v.im * ds);
+    }
+  } else if (table == 2) {
+    v.re += ((zq - zp) / r / (r * r) + zpq / r1 / (r1 * r1));
+    v.re -= flag == 1 ? zpq * ir13 : zpq * ir13 + (zq - zp) * ir3;
+    dz[lane] = make_double2(v.re, v.im);
+  }
+  __syncthreads();
+  if (table == 1 && live) {
+    v.re += (rr / r / (r * r) + rr / r1 / (r1 * r1));
+    cplx gx = hams::cmk(0.0, 0.0), gy = hams::cmk(0.0, 0.0);
+    if (rr > HAMS_F4(1.E-6)) {
+      gx = v * (xpq / rr);
+      gy = v * (ypq / rr);
+    }
+    gx.re -= flag == 1 ? xpq * ir13 : xpq * ir13 + xpq * ir3;
+    gy.re -= flag == 1 ? ypq * ir13 : ypq * ir13 + ypq * ir3;
+    const double2 gz = dz[lane];
+    const double ds = g.ds[j], n1 = g.nrm[j], n2 = g.nrm[j + g.n], n3 = g.nrm[j + 2 * g.n];
+    double are = rd[p] + ds * (gx.re * n1 + gy.re * n2 + gz.x * n3);
+    const double aim = ds * (gx.im * n1 + gy.im * n2 + gz.y * n3);
+    if (i == j) are += 2.0 * 3.141592653589793;
+    A[p] = make_double2(are, aim);
+  }
+}
+
+// Shared memory of a launch whose longest series has rows terms.
+static size_t series_smem(int rows) {
+  return ((size_t)hams::eps_columns(rows) * 8 + (size_t)hams::eps_pairs(rows) * 4) * kSerThreads;
+}
+
+int series_kernels_init() {
+  return cudaFuncSetAttribute(k_green_series<hams::kPidcock>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)series_smem(hams::kPidcockMax)) != cudaSuccess ||
+         cudaFuncSetAttribute(k_green_series<hams::kEigenE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)series_smem(hams::kEigenEMax)) != cudaSuccess;
+}
+
+void launch_green_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,
+                         const hams::ModeTab& mt, RadTab rt, const uint32_t* pairs, long long count, const double* rs,
+                         const double* rd, double2* A, double2* S, int* ovf) {
+  const unsigned blocks = (unsigned)((count + 31) / 32);
+  const size_t sh = series_smem(ntmax);
+  if (br == hams::kPidcock)
+    k_green_series<hams::kPidcock>
+        <<<blocks, kSerThreads, sh, st>>>(g, w, wvn, mt, rt, pairs, count, rs, rd, A, S, ovf, ntmax);
+  else
+    k_green_series<hams::kEigenE>
+        <<<blocks, kSerThreads, sh, st>>>(g, w, wvn, mt, rt, pairs, count, rs, rd, A, S, ovf, ntmax);
 }
 
 // Per-frequency mode tables (ModeTab) for modes 2..nmode-1: one thread per
 // (mode, panel) entry, the expressions of InlineModes (green.cuh), compiled
 // here without fused multiply-adds like the series that read them.  Slot 1
-// holds the propagating mode's factors for the surrogate kernel: pm[1] =
-// pi / NM0, src = (sinh, cosh) of k0 (zq + h), fld = cosh of k0 (zp + h).
+// holds the propagating mode's factors: pm[1] = pi / NM0, ac[1] = k0 pi / NM0,
+// src = (sinh, cosh) of k0 (zq + h), fld = cosh of k0 (zp + h).
 __global__ void k_mode_tables(DevGeom g, WaveDev w, const double* __restrict__ wvn, int nmode, double* pm, double* ac,
                               double2* src, double2* srct, double* fld, double* fldt) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -69,7 +344,11 @@ __global__ void k_mode_tables(DevGeom g, WaveDev w, const double* __restrict__ w
       src[g.n + k] = make_double2(sinh(wk * zfh), cosh(wk * zfh));
     }
     if (k < g.tn) fld[g.tn + k] = cosh(wk * (g.fxyz[k + 2 * g.tn] + h));
-    if (k == 0) pm[1] = 3.141592653589793 / (h / 2.0 * (1.0 + sinh(2.0 * wk * h) / (2.0 * wk * h)));
+    if (k == 0) {
+      const double nm0 = h / 2.0 * (1.0 + sinh(2.0 * wk * h) / (2.0 * wk * h));
+      pm[1] = 3.141592653589793 / nm0;
+      ac[1] = wk * 3.141592653589793 / nm0;
+    }
     return;
   }
   if (k < g.n) {

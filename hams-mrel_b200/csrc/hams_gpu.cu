@@ -148,11 +148,12 @@ __global__ void k_pair_keys(DevGeom g, double h, int sg_on, double far, const un
   idx[p] = (uint32_t)p;
 }
 
-// First index of each bin b = 0..nbins in the sorted keys (key >> 8 is the bin).
-__global__ void k_bin_offsets(const uint32_t* __restrict__ keys, long long np, int nbins, long long* off) {
+// First index of each of nv key values in the sorted keys.
+__global__ void k_bin_offsets(const uint32_t* __restrict__ keys, long long np, const uint32_t* __restrict__ vals,
+                              int nv, long long* off) {
   const int b = threadIdx.x;
-  if (b > nbins) return;
-  const uint32_t v = (uint32_t)b << 8;
+  if (b >= nv) return;
+  const uint32_t v = vals[b];
   long long lo = 0, hi = np;
   while (lo < hi) {
     const long long mid = lo + (hi - lo) / 2;
@@ -163,12 +164,58 @@ __global__ void k_bin_offsets(const uint32_t* __restrict__ keys, long long np, i
 }
 
 // ---------------------------------------------------------------------------
+// distinct distances: the radial tables' rows (RadTab)
+// ---------------------------------------------------------------------------
+// Horizontal distance of a pair, as fingreen3d of this file rounds it (the
+// EIGEN pairs; those of the epsilon series come from green_series.cu).
+__device__ __forceinline__ double eigen_distance(const DevGeom& g, uint32_t p) {
+  const uint32_t tn = (uint32_t)g.tn;
+  const int j = (int)(p / tn), i = (int)(p - (uint32_t)j * tn);
+  const double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], xq = g.xq[j], yq = g.xq[j + g.n];
+  const double xpq = xq - xp, ypq = yq - yp;
+  return sqrt(xpq * xpq + ypq * ypq);
+}
+__global__ void k_eigen_distance(DevGeom g, const uint32_t* __restrict__ pairs, long long count,
+                                 double* __restrict__ r) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < count) r[t] = eigen_distance(g, pairs[t]);
+}
+__global__ void k_iota(uint32_t* __restrict__ v, long long count) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < count) v[t] = (uint32_t)t;
+}
+// 1 at the first of equal sorted distances
+__global__ void k_distance_heads(const double* __restrict__ r, long long count, uint32_t* __restrict__ head) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < count) head[t] = t == 0 || r[t] != r[t - 1];
+}
+// rid of every pair, the distinct distances ur, and each branch's first and
+// last distance number (lim[2 br], lim[2 br + 1]); cut0..cut4 are the
+// positions where bins 2..6 start, counted from bin 1.
+__device__ __forceinline__ int series_class(long long pos, long long c2, long long c3, long long c4, long long c5) {
+  if (pos < c2) return hams::kPidcock;
+  if (pos < c3) return hams::kEigenE;
+  if (pos < c4) return hams::kEigen;
+  return pos < c5 ? hams::kEigenE : hams::kEigen;
+}
+__global__ void k_distance_rows(const double* __restrict__ r, const uint32_t* __restrict__ idx,
+                                const uint32_t* __restrict__ rank, long long count, long long c2, long long c3,
+                                long long c4, long long c5, uint32_t* __restrict__ rid, double* __restrict__ ur,
+                                uint32_t* __restrict__ lim) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t k = rank[t] - 1;
+  rid[idx[t]] = k;
+  if (t == 0 || rank[t - 1] != rank[t]) ur[k] = r[t];
+  const int br = series_class(idx[t], c2, c3, c4, c5);
+  if (t == 0 || series_class(idx[t - 1], c2, c3, c4, c5) != br) atomicMin(&lim[2 * br], k);
+  if (t == count - 1 || series_class(idx[t + 1], c2, c3, c4, c5) != br) atomicMax(&lim[2 * br + 1], k);
+}
+
+// ---------------------------------------------------------------------------
 // per-frequency assembly: Green function fused with the pair algebra
 // ---------------------------------------------------------------------------
-// LINTON (BR = 0) and EIGEN (BR = 3) pairs; the epsilon-series branches are
-// in green_series.cu.
-// EIGEN runs at 8 blocks per SM like the series kernels; LINTON's adaptive
-// quadrature keeps its registers.
+// LINTON and EIGEN pairs; the epsilon-series branches are in green_series.cu.
 // ---------------------------------------------------------------------------
 // the series' judgement of the surrogate
 // ---------------------------------------------------------------------------
@@ -377,12 +424,83 @@ __global__ void __launch_bounds__(kPrThreads) k_probe_apply(DevGeom g, const uns
   }
 }
 
-template <int BR>
-__global__ void __launch_bounds__(128, BR == hams::kEigen ? 8 : 1) k_green_fin(DevGeom g, WaveDev w, const double* __restrict__ wvn,
-                                                   hams::ModeTab mt, const uint32_t* __restrict__ pairs,
-                                                   long long count, const double* __restrict__ rs,
-                                                   const double* __restrict__ rd, double2* __restrict__ A,
-                                                   double2* __restrict__ S, int* ovf) {
+// The radial table of EIGEN: one thread per distance.  Past the mode whose
+// terms are below the series' truncation threshold for any depths (|sin|,
+// |cos| <= 1) no pair reads on.
+__global__ void __launch_bounds__(128) k_rad_eigen(DevGeom g, const double* __restrict__ wvn, hams::ModeTab mt,
+                                                   const double* __restrict__ ur, const uint32_t* __restrict__ pairs,
+                                                   long long count, double* __restrict__ kt,
+                                                   double4* __restrict__ jy) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const double r = ur ? ur[t] : eigen_distance(g, pairs[t]);
+  double4 v;
+  hams::jy01b(wvn[0] * r, v.x, v.y, v.z, v.w);
+  jy[t] = v;
+  double2* row = reinterpret_cast<double2*>(kt) + (size_t)t * (rad_stride(hams::kEigen) / 2);
+  for (int i = 2; i <= 10; ++i) {
+    const double km = wvn[i - 1], pm = mt.pm[i];
+    double k0, k1;
+    hams::ik01a(km * r, k0, k1);
+    row[i - 2] = make_double2(k0, k1);
+    if (pm * k0 < HAMS_F4(1.E-6) && pm * km * k1 < HAMS_F4(1.E-6) && pm * km * k0 < HAMS_F4(1.E-6)) break;
+  }
+}
+
+// EIGEN pairs: the propagating mode and at most nine modes from the pair's
+// radial row.  Memory-bound: 56 bytes per pair and the table rows it gathers;
+// 17.3 M pairs take 0.89 ms with 0.08 ms of table, against 9.3 ms with the
+// Bessel functions evaluated per pair.
+struct BesselRow {
+  const double2* __restrict__ row;
+  __device__ __forceinline__ void operator()(int i, double, double, double& k0, double& k1) const {
+    const double2 k = row[i - 2];
+    k0 = k.x;
+    k1 = k.y;
+  }
+};
+__global__ void __launch_bounds__(128, 8) k_green_eigen(DevGeom g, WaveDev w, const double* __restrict__ wvn,
+                                                        hams::ModeTab mt, RadTab rt,
+                                                        const uint32_t* __restrict__ pairs, long long count,
+                                                        const double* __restrict__ rs, const double* __restrict__ rd,
+                                                        double2* __restrict__ A, double2* __restrict__ S) {
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t p = pairs[t], tn = (uint32_t)g.tn;
+  const int j = (int)(p / tn), i = (int)(p - (uint32_t)j * tn);
+  int flag = near_flag(g, i, j);
+  double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], zp = g.fxyz[i + 2 * g.tn];
+  double xq = g.xq[j], yq = g.xq[j + g.n], zq = g.xq[j + 2 * g.n];
+  grn4 G;
+  if (w.limit) {
+    G = hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag);
+  } else {
+    const double xpq = xq - xp, ypq = yq - yp, zpq = zq + zp, wk = wvn[0];
+    const double rr = sqrt(xpq * xpq + ypq * ypq);
+    const double r = sqrt(rr * rr + (zp - zq) * (zp - zq)), r1 = sqrt(rr * rr + zpq * zpq);
+    const uint32_t row = rt.rid ? rt.rid[t] - rt.base : (uint32_t)t;
+    const double4 jy = rt.jy[row];
+    const double2 szf = mt.src[g.n + j];  // sinh, cosh of k0 (zq + h)
+    const double czp = mt.fld[g.tn + i], p0 = mt.pm[1] * szf.y * czp, dp0 = mt.pm[1] * szf.x * czp;
+    cplx fg[3];
+    fg[0] = hams::cmk(-p0 * jy.z, p0 * jy.x);
+    fg[1] = hams::cmk(wk * p0 * jy.w, -wk * p0 * jy.y);
+    fg[2] = hams::cmk(-wk * dp0 * jy.z, wk * dp0 * jy.x);
+    hams::TableModes md{mt, j, i};
+    const BesselRow bk{reinterpret_cast<const double2*>(rt.kt) + (size_t)row * (rad_stride(hams::kEigen) / 2)};
+    hams::eigen_modes(rr, wvn, fg, md, bk);
+    hams::remove_rankine(rr, zq, zp, fg);
+    G = hams::finish_green(fg, xpq, ypq, zq, zp, rr, r, r1, flag);
+  }
+  store_pair(g, p, i, j, G, rs, rd, A, S);
+}
+
+// LINTON pairs, a thread each.
+__global__ void __launch_bounds__(128) k_green_linton_threads(DevGeom g, WaveDev w, const double* __restrict__ wvn,
+                                                              hams::ModeTab mt, const uint32_t* __restrict__ pairs,
+                                                              long long count, const double* __restrict__ rs,
+                                                              const double* __restrict__ rd, double2* __restrict__ A,
+                                                              double2* __restrict__ S, int* ovf) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   size_t p = pairs[t];
@@ -396,7 +514,7 @@ __global__ void __launch_bounds__(128, BR == hams::kEigen ? 8 : 1) k_green_fin(D
   } else {
     int o = 0;
     hams::TableModes md{mt, j, i};
-    G = hams::fingreen3d<BR>(xq, xp, yq, yp, zq, zp, w.v, wvn, w.h, flag, (void*)nullptr, &o, md);
+    G = hams::fingreen3d<hams::kLinton>(xq, xp, yq, yp, zq, zp, w.v, wvn, w.h, flag, (void*)nullptr, &o, md);
     if (o) atomicOr(ovf, 1);
   }
   store_pair(g, p, i, j, G, rs, rd, A, S);
@@ -972,6 +1090,16 @@ struct hams_ctx {
   // EIGEN), 4-5 (surrogate pairs of EIGENE, EIGEN), 6 (pairs of copied body
   // blocks); bin_off[7] = total
   long long bin_off[kBins + 1] = {};
+  // radial tables: the distance number of every pair of bins 1-5 (from bin 1
+  // on), the distinct distances, and each branch's first and number of
+  // distances; a branch without distance numbers (rad_n = 0) gives every pair
+  // its own row, a chunk of pairs at a time
+  DBuf<uint32_t> rid;
+  DBuf<double> ur;
+  uint32_t rad_base[4] = {}, rad_n[4] = {};
+  // positions where the series of bins 1, 2 and 4 get longer than the two
+  // lengths of kNtCut (launch_series)
+  long long nt_cut[kBins][2] = {};
   // identical body blocks (hams_opts.body_blocks): per (field, source) body
   // pair 1 when copied, and the copies (6 ints each, k_copy_blocks)
   DBuf<unsigned char> blk_copied;
@@ -994,6 +1122,10 @@ struct hams_ctx {
   DBuf<double> mt_pm, mt_ac, mt_fld, mt_fldt;  // per-frequency mode tables (finite depth)
   DBuf<double2> mt_src, mt_srct;
   hams::ModeTab mt{};
+  // this frequency's radial tables per branch (rad_ready: filled)
+  DBuf<double> rad_k[4];
+  DBuf<double4> rad_j[4];
+  bool rad_ready[4] = {};
   DBuf<int> ipiv, info, ovf;
   DBuf<char> work;
   DBuf<char> work32;
@@ -1116,6 +1248,84 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
 
 static int ctx_frequency_buffers(hams_ctx* c);
 
+// Series lengths (EIGENE, then PIDCOCK) at which a bin's launch is split, so
+// that its shared memory fits the lengths it holds (launch_series).
+constexpr int kNtCut[2][2] = {{26, 38}, {66, 82}};
+// Least cap on the radial table of a numbered branch (otherwise half the bytes
+// of A), and the table bytes of a chunk of pairs where distances are not
+// numbered: small enough to stay in L2 between the two kernels.
+constexpr size_t kRadMin = (size_t)64 << 20;
+
+// The distinct distances of the series bins (RadTab): the pairs' distances
+// sorted, numbered where they change, the numbers scattered back to the
+// pairs.  A branch whose table would exceed half the bytes of A (a mesh
+// with few equal distances) keeps no numbers.
+static int build_distances(hams_ctx* c) {
+  const long long o1 = c->bin_off[1], ns = c->bin_off[6] - o1;
+  for (int br = 0; br < 4; ++br) c->rad_base[br] = c->rad_n[br] = 0;
+  c->rid.release(true);
+  if (ns <= 0) return 0;
+  DBuf<double> r, r2;
+  DBuf<uint32_t> idx, idx2, rank, lim;
+  // without the memory for the sort, every pair has its own row
+  if (r.alloc(ns) || r2.alloc(ns) || idx.alloc(ns) || idx2.alloc(ns) || rank.alloc(ns) || lim.alloc(8) ||
+      c->rid.alloc(ns)) {
+    g_err.clear();
+    c->rid.release(true);
+    return 0;
+  }
+  for (int b = 1; b < 6; ++b) {
+    const long long n = c->bin_off[b + 1] - c->bin_off[b];
+    if (n <= 0) continue;
+    const uint32_t* lst = c->pairs.p + c->bin_off[b];
+    double* out = r.p + (c->bin_off[b] - o1);
+    if (b == 3 || b == 5) k_eigen_distance<<<(unsigned)((n + 255) / 256), 256, 0, c->st>>>(c->g, lst, n, out);
+    else launch_series_distance(c->st, c->g, lst, n, out);
+    TRY(launch_check(c));
+  }
+  const unsigned nb = (unsigned)((ns + 255) / 256);
+  k_iota<<<nb, 256, 0, c->st>>>(idx.p, ns);
+  size_t t1 = 0, t2 = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, t1, r.p, r2.p, idx.p, idx2.p, (size_t)ns, 0, 64, c->st);
+  cub::DeviceScan::InclusiveSum(nullptr, t2, rank.p, rank.p, (size_t)ns, c->st);
+  DBuf<char> tbuf;
+  if (tbuf.alloc(std::max(t1, t2))) {
+    g_err.clear();
+    c->rid.release();
+    return 0;
+  }
+  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, t1, r.p, r2.p, idx.p, idx2.p, (size_t)ns, 0, 64, c->st));
+  k_distance_heads<<<nb, 256, 0, c->st>>>(r2.p, ns, rank.p);
+  CU(cub::DeviceScan::InclusiveSum(tbuf.p, t2, rank.p, rank.p, (size_t)ns, c->st));
+  c->lib_calls += 2;
+  TRY(launch_check(c, 2));
+  uint32_t nu = 0, l[8];
+  CU(cudaMemcpyAsync(&nu, rank.p + ns - 1, 4, cudaMemcpyDeviceToHost, c->st));
+  CU(cudaStreamSynchronize(c->st));
+  c->ur.release(true);
+  TRY(c->ur.alloc(nu));
+  for (int q = 0; q < 8; ++q) l[q] = q % 2 ? 0u : 0xffffffffu;
+  CU(cudaMemcpyAsync(lim.p, l, sizeof l, cudaMemcpyHostToDevice, c->st));
+  k_distance_rows<<<nb, 256, 0, c->st>>>(r2.p, idx2.p, rank.p, ns, c->bin_off[2] - o1, c->bin_off[3] - o1,
+                                         c->bin_off[4] - o1, c->bin_off[5] - o1, c->rid.p, c->ur.p, lim.p);
+  TRY(launch_check(c));
+  CU(cudaMemcpyAsync(l, lim.p, sizeof l, cudaMemcpyDeviceToHost, c->st));
+  CU(cudaStreamSynchronize(c->st));
+  for (DBuf<uint32_t>* d : {&idx, &idx2, &rank, &lim}) d->release(true);
+  r.release(true);
+  r2.release(true);
+  tbuf.release(true);
+  const size_t cap = std::max(kRadMin, (size_t)c->tn * c->n * 8);
+  for (int br = 1; br < 4; ++br) {
+    if (l[2 * br] > l[2 * br + 1]) continue;  // no pair
+    const uint32_t n = l[2 * br + 1] - l[2 * br] + 1;
+    if ((size_t)n * rad_stride(br) * 8 > cap) continue;
+    c->rad_base[br] = l[2 * br];
+    c->rad_n[br] = n;
+  }
+  return 0;
+}
+
 // Sorted pair list and bin offsets (finite depth); rebuilt when the surrogate
 // is switched on or off.
 static int build_pairs(hams_ctx* c) {
@@ -1134,15 +1344,32 @@ static int build_pairs(hams_ctx* c) {
   TRY(tbuf.alloc(tmp));
   CU(cub::DeviceRadixSort::SortPairs(tbuf.p, tmp, keys.p, keys2.p, idx.p, c->pairs.p, np, 0, 11, c->st));
   c->lib_calls += 1;
-  // bin boundaries: first index of each bin in the sorted keys, found on the
-  // device (a binary search per bin) so that only kBins + 1 numbers come back
+  // bin boundaries, and where the series of bins 1, 2 and 4 pass kNtCut:
+  // first index of each key in the sorted keys, found on the device (a binary
+  // search each) so that only these numbers come back
+  std::vector<uint32_t> vals;
+  for (int b = 0; b <= kBins; ++b) vals.push_back((uint32_t)b << 8);
+  for (int b : {1, 2, 4})
+    for (int q = 0; q < 2; ++q) vals.push_back(((uint32_t)b << 8) + kNtCut[b == 1][q] + 1);
   DBuf<long long> offs;
-  TRY(offs.alloc(kBins + 1));
-  k_bin_offsets<<<1, 32, 0, c->st>>>(keys2.p, (long long)np, kBins, offs.p);
+  DBuf<uint32_t> dvals;
+  TRY(offs.alloc(vals.size()));
+  TRY(dvals.alloc(vals.size()));
+  std::vector<long long> got(vals.size());
+  CU(cudaMemcpyAsync(dvals.p, vals.data(), vals.size() * 4, cudaMemcpyHostToDevice, c->st));
+  k_bin_offsets<<<1, 32, 0, c->st>>>(keys2.p, (long long)np, dvals.p, (int)vals.size(), offs.p);
   TRY(launch_check(c));
-  CU(cudaMemcpyAsync(c->bin_off, offs.p, (kBins + 1) * sizeof(long long), cudaMemcpyDeviceToHost, c->st));
+  CU(cudaMemcpyAsync(got.data(), offs.p, got.size() * sizeof(long long), cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
-  return 0;
+  for (int b = 0; b <= kBins; ++b) c->bin_off[b] = got[b];
+  int k = kBins + 1;
+  for (int b : {1, 2, 4})
+    for (int q = 0; q < 2; ++q) c->nt_cut[b][q] = got[k++];
+  keys.release(true);
+  keys2.release(true);
+  idx.release(true);
+  tbuf.release(true);
+  return build_distances(c);
 }
 
 static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
@@ -1253,6 +1480,15 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
   return 0;
 }
 
+static int rad_buffers(hams_ctx* c) {
+  for (int br = 1; br < 4; ++br)
+    if (c->rad_n[br]) {
+      TRY(c->rad_k[br].alloc((size_t)c->rad_n[br] * rad_stride(br)));
+      TRY(c->rad_j[br].alloc(c->rad_n[br]));
+    }
+  return 0;
+}
+
 // Buffers of one frequency in flight: mode tables, A and S, roots, flags.
 static int ctx_frequency_buffers(hams_ctx* c) {
   const int n = c->n, tn = c->tn;
@@ -1266,6 +1502,7 @@ static int ctx_frequency_buffers(hams_ctx* c) {
     int nmode = 11;
     if (c->bin_off[3] > c->bin_off[2] || c->bin_off[5] > c->bin_off[4]) nmode = hams::kEigenEMax + 1;
     if (c->bin_off[2] > c->bin_off[1]) nmode = hams::kPidcockMax + 1;
+    TRY(rad_buffers(c));
     c->mt = hams::ModeTab{n, tn, nmode, c->mt_pm.p, c->mt_ac.p, c->mt_src.p, c->mt_srct.p, c->mt_fld.p, c->mt_fldt.p};
   }
   TRY(c->A.alloc(np));
@@ -1351,6 +1588,7 @@ static void release_handle_pool() {
 // Stream, library handles and events of a context, on its device.
 static int ctx_handles(hams_ctx* c) {
   if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice(%d) failed", c->dev);
+  if (series_kernels_init()) return fail(HAMS_ERR_CUDA, "series kernels: shared memory size refused");
   if (handles_from_pool(c)) {
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev);
     return 0;
@@ -1368,6 +1606,16 @@ static int ctx_handles(hams_ctx* c) {
   CU(cudaEventCreate(&c->evf));
   CU(cudaEventCreate(&c->evc));
   return 0;
+}
+
+// The pair lists and distances of c as l's.
+static void view_pairs(hams_ctx* l, hams_ctx* c) {
+  for (int b = 0; b <= kBins; ++b) l->bin_off[b] = c->bin_off[b];
+  l->pairs.view(c->pairs);
+  l->rid.view(c->rid);
+  l->ur.view(c->ur);
+  for (int br = 0; br < 4; ++br) l->rad_base[br] = c->rad_base[br], l->rad_n[br] = c->rad_n[br];
+  for (int b = 0; b < kBins; ++b) l->nt_cut[b][0] = c->nt_cut[b][0], l->nt_cut[b][1] = c->nt_cut[b][1];
 }
 
 // A batch lane of c: its own stream, handles and per-frequency buffers; the
@@ -1392,12 +1640,12 @@ static int make_lane(hams_ctx* c, hams_ctx** out) {
   if (!rc) {
     l->xq.view(c->xq); l->fxyz.view(c->fxyz); l->ds.view(c->ds); l->pnsz.view(c->pnsz); l->nrm.view(c->nrm);
     l->vtx.view(c->vtx); l->ncn.view(c->ncn); l->body.view(c->body); l->bstart.view(c->bstart);
-    l->rs.view(c->rs); l->rd.view(c->rd); l->pairs.view(c->pairs); l->chunks.view(c->chunks);
+    l->rs.view(c->rs); l->rd.view(c->rd); l->chunks.view(c->chunks);
     l->chunk_body.view(c->chunk_body);
     l->blk_copied.view(c->blk_copied); l->blk_list.view(c->blk_list);
     l->nblk = c->nblk; l->blk_rows = c->blk_rows; l->blk_cols = c->blk_cols; l->blk_pairs = c->blk_pairs;
     l->g = c->g;
-    for (int b = 0; b <= kBins; ++b) l->bin_off[b] = c->bin_off[b];
+    view_pairs(l, c);
     l->sg_on = c->sg_on;
     l->sg_far = c->sg_far;
     l->sg_kmin = c->sg_kmin;
@@ -1581,21 +1829,78 @@ static WaveDev wave_dev(const hams_ctx* c, const hams_wave* w) {
   return d;
 }
 
-// Assemble A (tn x n) and the right-hand sides B (tn x (6nb+nbeta)) on the
-// device; force_series keeps the series for the far pairs of a surrogate
-// context (the re-solve of a frequency the series judged).
+// The pairs of one bin from the EIGENE / PIDCOCK / EIGEN series (br); pos is
+// the list's place in c->pairs, or -1 for a list without distance numbers.
+// bin is the bin the list is (its launch is split by series length), or 0.
+static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* lst, long long cnt, long long pos,
+                        int bin) {
+  if (cnt <= 0) return 0;
+  const int ntmax = br == hams::kPidcock ? hams::kPidcockMax : hams::kEigenEMax;
+  auto launch = [&](RadTab rt, const uint32_t* l, long long n, int nt) {
+    if (br == hams::kEigen)
+      k_green_eigen<<<(unsigned)((n + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->mt, rt, l, n, c->rs.p,
+                                                                    c->rd.p, c->A.p, c->S.p);
+    else
+      launch_green_series(br, nt, c->st, c->g, wd, c->wvn.p, c->mt, rt, l, n, c->rs.p, c->rd.p, c->A.p, c->S.p,
+                          c->ovf.p);
+    return launch_check(c);
+  };
+  auto table = [&](const double* ur, const uint32_t* l, long long n) {
+    if (br == hams::kEigen)
+      k_rad_eigen<<<(unsigned)((n + 127) / 128), 128, 0, c->st>>>(c->g, c->wvn.p, c->mt, ur, l, n, c->rad_k[br].p,
+                                                                  c->rad_j[br].p);
+    else
+      launch_rad_series(br, c->st, c->g, wd, c->wvn.p, ur, l, n, c->rad_k[br].p, c->rad_j[br].p);
+    return launch_check(c);
+  };
+  if (wd.limit) return launch(RadTab{}, lst, cnt, 8);
+  if (pos >= 0 && c->rad_n[br]) {
+    if (!c->rad_ready[br]) {
+      TRY(table(c->ur.p + c->rad_base[br], nullptr, c->rad_n[br]));
+      c->rad_ready[br] = true;
+    }
+    const uint32_t* rid = c->rid.p + (pos - c->bin_off[1]);
+    // the longest series first, each launch with the shared memory of its own
+    // lengths (and one more: the keys round distances with fused multiply-adds);
+    // a list that one wave of blocks holds stays one launch
+    long long cut[4] = {0, 0, 0, cnt};
+    if (br != hams::kEigen && bin && cnt > (long long)c->sms * 32 * 16) {
+      cut[1] = c->nt_cut[bin][0] - c->bin_off[bin];
+      cut[2] = c->nt_cut[bin][1] - c->bin_off[bin];
+    }
+    for (int q = 2; q >= 0; --q) {
+      const long long n = cut[q + 1] - cut[q];
+      if (n <= 0) continue;
+      const RadTab rt{rid + cut[q], c->rad_base[br], c->rad_k[br].p, c->rad_j[br].p};
+      TRY(launch(rt, lst + cut[q], n, q == 2 ? ntmax : kNtCut[br == hams::kPidcock][q] + 1));
+    }
+    return 0;
+  }
+  // a row per pair, a chunk of pairs at a time; c->rad_k may hold the table
+  // of the numbered distances, which is then filled again
+  const long long per = std::min<long long>(cnt, kRadMin / (rad_stride(br) * 8));
+  TRY(c->rad_k[br].alloc((size_t)per * rad_stride(br)));
+  TRY(c->rad_j[br].alloc(per));
+  c->rad_ready[br] = false;
+  for (long long t = 0; t < cnt; t += per) {
+    const long long n = std::min(per, cnt - t);
+    TRY(table(nullptr, lst + t, n));
+    TRY(launch(RadTab{nullptr, 0, c->rad_k[br].p, c->rad_j[br].p}, lst + t, n, ntmax));
+  }
+  return 0;
+}
+// The pairs of bin b (1-5) of the context's list.
+static int series_bin(hams_ctx* c, const WaveDev& wd, int b) {
+  static const int branch[6] = {hams::kLinton, hams::kPidcock, hams::kEigenE, hams::kEigen, hams::kEigenE, hams::kEigen};
+  return series_pairs(c, wd, branch[b], c->pairs.p + c->bin_off[b], c->bin_off[b + 1] - c->bin_off[b], c->bin_off[b],
+                      b);
+}
+
 // The far pairs (bins 4 and 5 of k_pair_keys) from the series: EIGENE and
 // EIGEN, as their own bins would (FinGreen3D.f90:413-660).
 static int far_series(hams_ctx* c, const WaveDev& wd) {
-  const long long ce = c->bin_off[5] - c->bin_off[4], cg = c->bin_off[6] - c->bin_off[5];
-  if (ce > 0)
-    launch_green_series(hams::kEigenE, (unsigned)((ce + 127) / 128), c->st, c->g, wd, c->wvn.p, c->mt,
-                        c->pairs.p + c->bin_off[4], ce, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p);
-  if (cg > 0)
-    k_green_fin<3><<<(unsigned)((cg + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->mt,
-                                                                    c->pairs.p + c->bin_off[5], cg, c->rs.p, c->rd.p,
-                                                                    c->A.p, c->S.p, c->ovf.p);
-  return launch_check(c, (ce > 0) + (cg > 0));
+  TRY(series_bin(c, wd, 4));
+  return series_bin(c, wd, 5);
 }
 
 // The copies of the identical body blocks, then the right-hand sides B from S
@@ -1614,6 +1919,9 @@ static int copy_blocks_and_rhs(hams_ctx* c, int nbeta) {
   return launch_check(c, 2);
 }
 
+// Assemble A (tn x n) and the right-hand sides B (tn x (6nb+nbeta)) on the
+// device; force_series keeps the series for the far pairs of a surrogate
+// context (the re-solve of a frequency the series judged).
 static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_series = false) {
   const int n = c->n, tn = c->tn, nb = c->nb, nrhs = 6 * nb + nbeta;
   WaveDev wd = wave_dev(c, w);
@@ -1631,27 +1939,25 @@ static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_s
                          c->mt_fld.p, c->mt_fldt.p);
       TRY(launch_check(c));
     }
+    for (bool& r : c->rad_ready) r = false;
     for (int br = 0; br < 4; ++br) {
       long long cnt = c->bin_off[br + 1] - c->bin_off[br];
       CU(cudaEventRecord(c->evb[br], c->st));
       if (cnt <= 0) continue;
-      const uint32_t* lst = c->pairs.p + c->bin_off[br];
-      unsigned blocks = (unsigned)((cnt + 127) / 128);
-      switch (br) {
-        case 0:
-          // few pairs (body blocks): a warp per pair for latency; many: a thread per pair, whose
-          // one wave over the GPU costs less than the warps' redundant lanes
-          if (cnt < (long long)c->sms * kLintonWarpPairsPerSm)
-            k_green_linton<<<(unsigned)((cnt + kLintonWarps - 1) / kLintonWarps), 32 * kLintonWarps, 0, c->st>>>(
-                c->g, wd, c->wvn.p, lst, cnt, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p);
-          else
-            k_green_fin<0><<<blocks, 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->mt, lst, cnt, c->rs.p, c->rd.p, c->A.p,
-                                                      c->S.p, c->ovf.p);
-          break;
-        case 1:
-        case 2: launch_green_series(br, blocks, c->st, c->g, wd, c->wvn.p, c->mt, lst, cnt, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p); break;
-        default: k_green_fin<3><<<blocks, 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->mt, lst, cnt, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p); break;
+      if (br > 0) {
+        TRY(series_bin(c, wd, br));
+        continue;
       }
+      // few pairs (body blocks): a warp per pair for latency; many: a thread per pair, whose
+      // one wave over the GPU costs less than the warps' redundant lanes
+      const uint32_t* lst = c->pairs.p;
+      if (cnt < (long long)c->sms * kLintonWarpPairsPerSm)
+        k_green_linton<<<(unsigned)((cnt + kLintonWarps - 1) / kLintonWarps), 32 * kLintonWarps, 0, c->st>>>(
+            c->g, wd, c->wvn.p, lst, cnt, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p);
+      else
+        k_green_linton_threads<<<(unsigned)((cnt + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->mt, lst, cnt,
+                                                                                 c->rs.p, c->rd.p, c->A.p, c->S.p,
+                                                                                 c->ovf.p);
       TRY(launch_check(c));
     }
     CU(cudaEventRecord(c->evb[4], c->st));
@@ -1675,14 +1981,8 @@ static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_s
           const unsigned gb = (unsigned)((ns + 255) / 256);
           k_gather_pairs<<<gb, 256, 0, c->st>>>(c->sg_samp.p, ns, c->A.p, c->S.p, c->sg_g1.p);
           TRY(launch_check(c));
-          if (c->sg_ns4 > 0)
-            launch_green_series(hams::kEigenE, (unsigned)((c->sg_ns4 + 127) / 128), c->st, c->g, wd, c->wvn.p, c->mt,
-                                c->sg_samp.p, c->sg_ns4, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p);
-          if (c->sg_ns5 > 0)
-            k_green_fin<3><<<(unsigned)((c->sg_ns5 + 127) / 128), 128, 0, c->st>>>(
-                c->g, wd, c->wvn.p, c->mt, c->sg_samp.p + c->sg_ns4, c->sg_ns5, c->rs.p, c->rd.p, c->A.p, c->S.p,
-                c->ovf.p);
-          TRY(launch_check(c, (c->sg_ns4 > 0) + (c->sg_ns5 > 0)));
+          TRY(series_pairs(c, wd, hams::kEigenE, c->sg_samp.p, c->sg_ns4, -1, 0));
+          TRY(series_pairs(c, wd, hams::kEigen, c->sg_samp.p + c->sg_ns4, c->sg_ns5, -1, 0));
           k_gather_pairs<<<gb, 256, 0, c->st>>>(c->sg_samp.p, ns, c->A.p, c->S.p, c->sg_g2.p);
           k_sample_err<<<1, 1024, 0, c->st>>>(c->sg_g1.p, c->sg_g2.p, ns, c->sg_red.p);
           TRY(c->sg_cells.alloc(4 * kJCells));
@@ -2756,6 +3056,7 @@ extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t 
     c->sg_on = 0;
   }
   TRY(build_pairs(c));
+  TRY(rad_buffers(c));
   TRY(build_judge_samples(c));
   if (c->sg_on) {
     TRY(c->sg_map.alloc((size_t)c->tn * c->n));
@@ -2766,8 +3067,8 @@ extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t 
   if (c->bin_off[3] > c->bin_off[2] || c->bin_off[5] > c->bin_off[4]) nmode = std::max(nmode, hams::kEigenEMax + 1);
   c->mt.nmode = nmode;
   for (hams_ctx* l : c->lanes) {
-    for (int b = 0; b <= kBins; ++b) l->bin_off[b] = c->bin_off[b];
-    l->pairs.view(c->pairs);
+    view_pairs(l, c);
+    TRY(rad_buffers(l));
     l->sg_on = c->sg_on;
     l->sg_far = c->sg_far;
     l->sg_kmin = c->sg_kmin;

@@ -55,14 +55,37 @@ __device__ __forceinline__ void store_pair(const DevGeom& g, size_t p, int i, in
 }
 
 
+// Radial factors of the eigenfunction series: the Bessel functions of a pair
+// depend on its horizontal distance R only, and a deck has far fewer distinct
+// distances than pairs (G is even in R, columns of panels share theirs, bodies
+// repeat), so each branch evaluates them once per distinct R and frequency
+// into a table.  Without rid the pairs of a launch are numbered by their place
+// in its list: every pair its own table row.
+struct RadTab {
+  const uint32_t* rid;  // distance number of each pair of the list, or null
+  uint32_t base;        // the branch's first distance number
+  const double* kt;     // (distance, stride): EIGENE/EIGEN K0, K1 of wvn[i-1] R for modes i = 2..; PIDCOCK K0, K1
+                        // of wvn[i-1] R and of (i-1) pi/h R
+  const double4* jy;    // J0, J1, Y0, Y1 of k0 R
+};
+// Doubles of a table row: EIGEN 9 modes, EIGENE 49, PIDCOCK 98 with two pairs.
+__host__ __device__ constexpr int rad_stride(int br) {
+  return br == hams::kPidcock ? 4 * (hams::kPidcockMax - 1) : br == hams::kEigenE ? 2 * (hams::kEigenEMax - 1) : 18;
+}
+
 // Launchers of the kernels compiled without implicit fused multiply-adds
 // (green_series.cu): the EIGENE (br = 2) and PIDCOCK (br = 1) branches, whose
 // epsilon-extrapolated series must see the same operation sequence as the
-// CPU checker, the per-frequency mode tables they read, and the batch
-// evaluator.
-void launch_green_series(int br, unsigned blocks, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,
-                         const hams::ModeTab& mt, const uint32_t* pairs, long long count, const double* rs,
+// CPU checker, their radial tables (from the distances ur, or from the pairs
+// of the list where ur is null), the distances themselves, the per-frequency
+// mode tables, and the batch evaluator.
+void launch_green_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,
+                         const hams::ModeTab& mt, RadTab rt, const uint32_t* pairs, long long count, const double* rs,
                          const double* rd, double2* A, double2* S, int* ovf);
+void launch_rad_series(int br, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, const double* ur,
+                       const uint32_t* pairs, long long count, double* kt, double4* jy);
+void launch_series_distance(cudaStream_t st, DevGeom g, const uint32_t* pairs, long long count, double* r);
+int series_kernels_init();
 void launch_mode_tables(cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, int nmode, double* pm, double* ac,
                         double2* src, double2* srct, double* fld, double* fldt);
 void launch_eval_green(unsigned blocks, cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w,
