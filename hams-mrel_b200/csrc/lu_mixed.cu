@@ -9,9 +9,9 @@
 //
 //   for each panel of kPB = 4 diagonal blocks (256 columns):
 //     for each diagonal block k (kNB = 64 rows) of the panel:
-//       k_diag_lu    one CTA factors A_kk = P_k^T L_kk U_kk in shared memory
-//                    with partial pivoting inside the block, and forms
-//                    L_kk^-1 and U_kk^-1;
+//       k_diag_lu    one CTA factors A_kk = P_k^T L_kk U_kk in registers with
+//                    partial pivoting inside the block, and forms L_kk^-1 and
+//                    U_kk^-1 on the way;
 //       k_perm_expand applies P_k to the rest of block row k and expands the
 //                    block column below for the GEMMs;
 //       GEMM         L_ik = A_ik U_kk^-1 below the block, U_kj = L_kk^-1 A_kj
@@ -45,6 +45,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdint>
 
 #include "gemm_tf32.h"
 #include "lu_mixed.h"
@@ -53,7 +54,6 @@ namespace {
 
 constexpr int kNB = 64;
 constexpr int kPB = 4;   // diagonal blocks per panel: the trailing update runs once per kPB kNB columns
-constexpr int kLd = kNB + 1;  // padded shared-memory leading dimension
 
 // Real expansion of complex matrices.  A complex p x q matrix X becomes the
 // real 2p x 2q matrix X^ with the 2 x 2 block [[xr, -xi], [xi, xr]] in place
@@ -61,14 +61,7 @@ constexpr int kLd = kNB + 1;  // padded shared-memory leading dimension
 // float2) is, viewed as floats, the real 2q x r matrix with rows re, im.
 // Then (X B) viewed as floats = X^ B_real and (X Y)^ = X^ Y^, so every
 // complex product of the factorisation is one real GEMM on tensor cores.
-__device__ __forceinline__ void put_expanded(float* E, int lde, int i, int k, float2 x) {
-  E[(size_t)(2 * k) * lde + 2 * i] = x.x;
-  E[(size_t)(2 * k) * lde + 2 * i + 1] = x.y;
-  E[(size_t)(2 * k + 1) * lde + 2 * i] = -x.y;
-  E[(size_t)(2 * k + 1) * lde + 2 * i + 1] = x.x;
-}
-
-// The same expansion stored row-major (E[row * lde + col]): the K-major
+// Entry (i, k) of the expansion stored row-major (E[row * lde + col]): the K-major
 // layout of a left operand of the tensor-core GEMM.
 __device__ __forceinline__ void put_expanded_rm(float* E, int lde, int i, int k, float2 x) {
   *reinterpret_cast<float2*>(E + (size_t)(2 * i) * lde + 2 * k) = make_float2(x.x, -x.y);
@@ -80,186 +73,210 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 }
 
 __device__ __forceinline__ float2 cmac(float2 s, float2 a, float2 b) {
-  return make_float2(s.x + a.x * b.x - a.y * b.y, s.y + a.x * b.y + a.y * b.x);
+  return make_float2(fmaf(-a.y, b.y, fmaf(a.x, b.x, s.x)), fmaf(a.y, b.x, fmaf(a.x, b.y, s.y)));
 }
 
-// Barrier of one 128-thread half of the block (named barrier bar, 1 or 2).
-__device__ __forceinline__ void group_sync(int bar) { asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory"); }
-
-// Inverse of the unit lower (lower) or the upper triangle of T (kNB x kNB,
-// ld kLd) into X: the 8 x 8 diagonal blocks by substitution, then three
-// doubling levels X21 = -X22 (L21 X11) (lower) or X12 = -X11 (U12 X22)
-// (upper), each product spread over 128 threads (tid 0..127 of one half of
-// the block, synchronised by the named barrier bar, so that the two halves
-// form the two inverses at once); W holds the inner products of one level
-// (at most 32 columns).
-__device__ void tri_inverse(const float2* T, float2* X, float2* W, bool lower, int tid, int bar) {
-  for (int e = tid; e < kNB * kNB; e += 128) X[(e / kNB) * kLd + e % kNB] = make_float2(0.0f, 0.0f);
-  group_sync(bar);
-  if (tid < kNB) {
-    const int c = tid, b0 = c & ~7;
-    if (lower) {
-      X[c * kLd + c] = make_float2(1.0f, 0.0f);
-      for (int i = c + 1; i < b0 + 8; ++i) {
-        float2 acc = make_float2(0.0f, 0.0f);
-        for (int k = c; k < i; ++k) acc = cmac(acc, T[k * kLd + i], X[c * kLd + k]);
-        X[c * kLd + i] = make_float2(-acc.x, -acc.y);
-      }
-    } else {
-      for (int i = c; i >= b0; --i) {
-        float2 acc = make_float2(i == c ? 1.0f : 0.0f, 0.0f);
-        for (int k = i + 1; k <= c; ++k) {
-          float2 t = cmac(make_float2(0.0f, 0.0f), T[k * kLd + i], X[c * kLd + k]);
-          acc.x -= t.x;
-          acc.y -= t.y;
-        }
-        const float2 d = T[i * kLd + i];
-        const float dd = d.x * d.x + d.y * d.y;
-        X[c * kLd + i] = dd > 0.0f ? make_float2((acc.x * d.x + acc.y * d.y) / dd, (acc.y * d.x - acc.x * d.y) / dd)
-                                   : make_float2(0.0f, 0.0f);
-      }
-    }
-  }
-  group_sync(bar);
-  for (int sz = 8; sz < kNB; sz *= 2) {
-    const int tot = (kNB / (2 * sz)) * sz * sz;
-    for (int e = tid; e < tot; e += 128) {
-      const int q = e / (sz * sz), rem = e % (sz * sz), c = rem / sz, i = rem % sz, b0 = 2 * sz * q;
-      float2 acc = make_float2(0.0f, 0.0f);
-      if (lower)  // W = L21 X11
-        for (int k = c; k < sz; ++k) acc = cmac(acc, T[(b0 + k) * kLd + b0 + sz + i], X[(b0 + c) * kLd + b0 + k]);
-      else  // W = U12 X22
-        for (int k = 0; k <= c; ++k) acc = cmac(acc, T[(b0 + sz + k) * kLd + b0 + i], X[(b0 + sz + c) * kLd + b0 + sz + k]);
-      W[(q * sz + c) * kLd + i] = acc;
-    }
-    group_sync(bar);
-    for (int e = tid; e < tot; e += 128) {
-      const int q = e / (sz * sz), rem = e % (sz * sz), c = rem / sz, i = rem % sz, b0 = 2 * sz * q;
-      float2 acc = make_float2(0.0f, 0.0f);
-      if (lower) {  // X21 = -X22 W
-        for (int k = 0; k <= i; ++k) acc = cmac(acc, X[(b0 + sz + k) * kLd + b0 + sz + i], W[(q * sz + c) * kLd + k]);
-        X[(b0 + c) * kLd + b0 + sz + i] = make_float2(-acc.x, -acc.y);
-      } else {  // X12 = -X11 W
-        for (int k = i; k < sz; ++k) acc = cmac(acc, X[(b0 + k) * kLd + b0 + i], W[(q * sz + c) * kLd + k]);
-        X[(b0 + sz + c) * kLd + b0 + i] = make_float2(-acc.x, -acc.y);
-      }
-    }
-    group_sync(bar);
-  }
-}
-
-// One CTA of 256 threads: LU with partial pivoting of the nbk x nbk
-// diagonal block at (k0, k0), written back in place (unit L below, U on and
-// above the diagonal); the block's row permutation as global source rows in
-// perm; the expansions of L^-1 (row-major) and U^-1 (column-major), 2nbk x
-// 2nbk with ld 2 kNB, in invL, invU -- the K-major layouts of a left and a
-// right GEMM operand; and the complex kNB x kNB inverses (column-major, the
+// LU with partial pivoting of the nbk x nbk diagonal block at (k0, k0), in one
+// CTA: the block's row permutation as global source rows in perm; the
+// expansions of L^-1 (row-major) and U^-1 (column-major), 2nbk x 2nbk with ld
+// 2 kNB, in invL, invU -- the K-major layouts of a left and a right GEMM
+// operand; and the complex kNB x kNB inverses (column-major, the
 // identity-padded block for a partial last block) in invLc, invUc for the
-// triangular solves.  info gets 1 + the first global column whose pivot is
-// zero.  A partial last block is padded with the identity to kNB.
-__global__ void __launch_bounds__(256) k_diag_lu(float2* A, int lda, int k0, int nbk, int* perm, float* invL,
-                                                 float* invU, float2* invLc, float2* invUc, int* info) {
-  extern __shared__ float2 sm[];
-  float2* T = sm;                  // [col * kLd + row]
-  float2* X = sm + kNB * kLd;      // L^-1
-  float2* Y = sm + 2 * kNB * kLd;  // U^-1
-  float2* W = sm + 3 * kNB * kLd;  // inversion scratch (32 columns for each inverse)
-  __shared__ int piv[kNB];
-  __shared__ int prm[kNB];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  for (int e = tid; e < kNB * kNB; e += 256) {
-    int r = e % kNB, c = e / kNB;
-    T[c * kLd + r] = (r < nbk && c < nbk) ? A[(size_t)(k0 + c) * lda + k0 + r]
-                                          : make_float2(r == c ? 1.0f : 0.0f, 0.0f);
-  }
-  __syncthreads();
-  for (int j = 0; j < nbk; ++j) {
-    if (tid < 32) {
-      float best = -1.0f;
-      int bi = j;
-      for (int r = j + tid; r < nbk; r += 32) {
-        float2 v = T[j * kLd + r];
-        float a = fabsf(v.x) + fabsf(v.y);
-        if (a > best) {
-          best = a;
-          bi = r;
-        }
+// triangular solves.  The block itself stays in A: nothing reads its factors.
+// info gets 1 + the first global column whose pivot is zero.
+//
+// A chain of 64 dependent columns on one SM, so what counts is the time per
+// column: one barrier, one pass.  Two threads of warps 0-3 hold a row in
+// registers, and rows never move: the pivot row is the one of largest |re| +
+// |im| among those not taken yet.  Each warp offers its own best row (a
+// warp-wide maximum, then the two lanes write the row to shared memory, with
+// the reciprocal of its entry) before the barrier; after it every thread knows
+// the pivot row and updates its own.  The row operations are applied to
+// [A | I], whose right half becomes L^-1: a column of A that is done makes room
+// for the new column of L^-1, so a row keeps 64 entries.  An entry's place is
+// fixed for four columns (places 4q..4q+3; at column j the current one is place
+// j % 4), then the row moves down by four: no register is indexed at run time.
+// So place x of the pivot row of column j, j0 = 4 (j / 4), holds
+//   L^-1(j, j0 + x) for x < j - j0, U(j, j0 + x) for j - j0 <= x < 64 - j0,
+//   L^-1(j, x - (64 - j0)) from there on (t < j0),
+// which warps 4-11 keep in R, one row per column, while they form column j of
+// U^-1: U^-1(i, j) = -sum_t U^-1(i, t) U(t, j) / U(j, j), four threads per row
+// i, a quarter of the t each.
+// Bound by the chain of a column (about 1,400 cycles: the maximum, the row
+// through shared memory, the update); one block takes 52 us, against 112 us
+// with the block in shared memory, three barriers per column and the inverses
+// after the factorisation.  A layout of 4 x 4 entries per thread on twice the
+// warps (a shorter chain, more instructions) takes 62 us.
+constexpr int kLuRowWarps = 4, kLuInvWarps = 8;
+constexpr int kLuThreads = 32 * (kLuRowWarps + kLuInvWarps);
+// row strides of R and U^-1 in shared memory, so that the four threads of a
+// row read from different banks
+constexpr int kRLd = kNB + 1, kUiLd = kNB + 8;
+constexpr int kDiagSmem = (kNB * (kRLd + kUiLd) + 2 * kLuRowWarps * kNB) * (int)sizeof(float2);
+
+__global__ void __launch_bounds__(kLuThreads) k_diag_lu(const float2* __restrict__ A, int lda, int k0, int nbk,
+                                                        int* perm, float* invL, float* invU, float2* invLc,
+                                                        float2* invUc, int* info) {
+  extern __shared__ __align__(16) float2 sm[];
+  float2* offer = sm;                                // [j & 1][warp][place]: each warp's best row
+  float2* Ui = sm + 2 * kLuRowWarps * kNB;           // [column j][row i]: U^-1
+  float2* R = Ui + kNB * kUiLd;                      // [column j][place]: the pivot rows
+  __shared__ __align__(16) uint32_t okey[2][kLuRowWarps];
+  __shared__ __align__(16) int orow[2][kLuRowWarps];
+  __shared__ float2 orcp[2][kLuRowWarps];  // reciprocal of the offered row's entry
+  __shared__ int prow[kNB];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the pivot of column j among the offers: the largest, the first warp of equal ones
+  static_assert(kLuRowWarps == 4, "the offers are compared as four");
+  auto winner = [&](int j) {
+    const uint4 k = *reinterpret_cast<const uint4*>(okey[j & 1]);
+    const bool a = k.y > k.x, b = k.w > k.z;
+    return max(k.z, k.w) > max(k.x, k.y) ? (b ? 3 : 2) : (a ? 1 : 0);
+  };
+  auto reciprocal = [](float2 d) {
+    const float dd = d.x * d.x + d.y * d.y, r = __frcp_rn(dd);
+    return dd > 0.0f ? make_float2(d.x * r, -d.y * r) : make_float2(0.0f, 0.0f);
+  };
+  auto minus = [](float2 a, float2 l, float ux, float uy) {  // a - l u
+    return make_float2(fmaf(-l.x, ux, fmaf(l.y, uy, a.x)), fmaf(-l.x, uy, fmaf(-l.y, ux, a.y)));
+  };
+  if (warp < kLuRowWarps) {
+    const int row = warp * 16 + (lane >> 1), h = lane & 1;  // places 4q + 2h, 4q + 2h + 1 of this row
+    float2 a[16][2];
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const int c = 4 * q + 2 * h + v;
+        a[q][v] = (row < nbk && c < nbk) ? A[(size_t)(k0 + c) * lda + k0 + row] : make_float2(0.0f, 0.0f);
       }
-      for (int o = 16; o; o >>= 1) {
-        float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (tid == 0) {
-        piv[j] = bi;
-        if (!(best > 0.0f)) atomicMin(info, k0 + j + 1);
-      }
-    }
-    __syncthreads();
-    // row swap j <-> p and the multipliers of column j in one pass, from the
-    // values before the swap: thread t swaps column t (t != j) and scales
-    // row t of column j (t > j, t != p); thread j handles rows j and p of
-    // column j
-    {
-      const int p = piv[j];
-      const float2 d = T[j * kLd + p];  // the pivot
-      const float dd = d.x * d.x + d.y * d.y;
-      const float2 rcp = dd > 0.0f ? make_float2(d.x / dd, -d.y / dd) : make_float2(0.0f, 0.0f);
-      if (tid < nbk) {
-        if (tid != j) {
-          if (p != j) {
-            float2 t = T[tid * kLd + j];
-            T[tid * kLd + j] = T[tid * kLd + p];
-            T[tid * kLd + p] = t;
+    bool taken = row >= nbk;
+    float2 cur = a[0][0];  // the row's entry of the current column, in both of its lanes
+    cur.x = __shfl_sync(0xffffffffu, cur.x, lane & ~1);
+    cur.y = __shfl_sync(0xffffffffu, cur.y, lane & ~1);
+#pragma unroll 1
+    for (int j0 = 0; j0 < nbk; j0 += 4) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int j = j0 + s;
+        if (j < nbk) {  // uniform
+          // offer this warp's best row and the reciprocal of its entry
+          const uint32_t mine = taken ? 0u : __float_as_uint(fabsf(cur.x) + fabsf(cur.y)) + 1u;
+          const uint32_t best = __reduce_max_sync(0xffffffffu, mine);
+          const float2 rcp = reciprocal(cur);
+          float2* of = offer + ((j & 1) * kLuRowWarps + warp) * kNB;
+          const unsigned at = __ballot_sync(0xffffffffu, mine == best);
+          if (lane >> 1 == (__ffs(at) - 1) >> 1) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              *reinterpret_cast<float4*>(of + 4 * q + 2 * h) = make_float4(a[q][0].x, a[q][0].y, a[q][1].x, a[q][1].y);
+            if (h == 0) {
+              okey[j & 1][warp] = best;
+              orow[j & 1][warp] = row;
+              orcp[j & 1][warp] = rcp;
+            }
           }
-          if (tid > j && tid != p && dd > 0.0f) T[j * kLd + tid] = cmul(T[j * kLd + tid], rcp);
-        } else {
-          const float2 old = T[j * kLd + j];
-          T[j * kLd + j] = d;
-          if (p != j) T[j * kLd + p] = dd > 0.0f ? cmul(old, rcp) : old;
+          __syncthreads();
+          const int w = winner(j);
+          const float2* u = offer + ((j & 1) * kLuRowWarps + w) * kNB;
+          const float2 l = cmul(cur, orcp[j & 1][w]);
+          if (tid == 0 && okey[j & 1][w] <= 1u) atomicMin(info, k0 + j + 1);  // zero pivot
+          if (row == orow[j & 1][w]) taken = true;
+          if (!taken) {
+            float2 first[2];  // quad 0 after the update: it moves to the end with s = 3
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              const float4 uu = *reinterpret_cast<const float4*>(u + 4 * q + 2 * h);
+              float2 n0 = minus(a[q][0], l, uu.x, uu.y), n1 = minus(a[q][1], l, uu.z, uu.w);
+              if (q == 0 && h == s / 2) (s & 1 ? n1 : n0) = make_float2(-l.x, -l.y);  // the new column of L^-1
+              if (s < 3) {
+                a[q][0] = n0;
+                a[q][1] = n1;
+              } else if (q == 0) {
+                first[0] = n0;
+                first[1] = n1;
+              } else {
+                a[q - 1][0] = n0;
+                a[q - 1][1] = n1;
+              }
+            }
+            if (s == 3) {
+              a[15][0] = first[0];
+              a[15][1] = first[1];
+            }
+          }
+          // the next column's entry, from the lane that holds it
+          constexpr int kNext[4] = {1, 2, 3, 0};
+          const int sn = kNext[s];
+          cur = a[0][sn & 1];
+          cur.x = __shfl_sync(0xffffffffu, cur.x, (lane & ~1) | (sn / 2));
+          cur.y = __shfl_sync(0xffffffffu, cur.y, (lane & ~1) | (sn / 2));
         }
       }
     }
-    __syncthreads();
-    // rank-1 update: tx walks rows (consecutive in shared memory), ty columns
-    for (int c = j + 1 + ty; c < nbk; c += 16) {
-      float2 u = T[c * kLd + j];
-      for (int r = j + 1 + tx; r < nbk; r += 16) {
-        float2 l = T[j * kLd + r], t = T[c * kLd + r];
-        T[c * kLd + r] = make_float2(t.x - (l.x * u.x - l.y * u.y), t.y - (l.x * u.y + l.y * u.x));
+  } else {
+    const int iw = warp - kLuRowWarps, g = lane >> 3, i = iw * 8 + (lane & 7);  // row of U^-1, quarter of the sum
+    const int place = tid - 32 * kLuRowWarps;
+    float2 v[16];  // U^-1(i, 4q + g)
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int jq = 0; jq < 16; ++jq) {  // columns 4 jq .. 4 jq + 3: the registers are indexed at compile time
+#pragma unroll 1
+      for (int s = 0; s < 4 && 4 * jq + s < nbk; ++s) {
+        const int j = 4 * jq + s;
+        __syncthreads();
+        const int w = winner(j);
+        if (place < kNB) R[j * kRLd + place] = offer[((j & 1) * kLuRowWarps + w) * kNB + place];
+        if (place == 0) prow[j] = orow[j & 1][w];
+        const float2 rcp = orcp[j & 1][w];
+        // U(t, j), t < j, sits in row t of R at place j - 4 (t / 4)
+        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+        for (int q = 0; q < jq; ++q) {
+          float2& t = q & 1 ? s1 : s0;
+          t = cmac(t, v[q], R[(4 * q + g) * kRLd + j - 4 * q]);
+        }
+        if (g < s) s0 = cmac(s0, v[jq], R[(4 * jq + g) * kRLd + s]);
+        s0.x += s1.x;
+        s0.y += s1.y;
+#pragma unroll
+        for (int o = 8; o <= 16; o *= 2) {
+          s0.x += __shfl_xor_sync(0xffffffffu, s0.x, o);
+          s0.y += __shfl_xor_sync(0xffffffffu, s0.y, o);
+        }
+        float2 x = cmul(make_float2(-s0.x, -s0.y), rcp);
+        if (i == j) x = rcp;
+        if (i > j) x = make_float2(0.0f, 0.0f);
+        if (g == s) v[jq] = x;
       }
     }
-    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16; ++q) Ui[(4 * q + g) * kUiLd + i] = v[q];
   }
-  if (tid == 0) {  // the block permutation: the same swaps applied to row indices
-    for (int i = 0; i < nbk; ++i) prm[i] = i;
-    for (int j = 0; j < nbk; ++j) {
-      int t = prm[j];
-      prm[j] = prm[piv[j]];
-      prm[piv[j]] = t;
-    }
-  }
-  __syncthreads();  // the factors and prm are complete
-  if (tid < 128)
-    tri_inverse(T, X, W, true, tid, 1);
-  else
-    tri_inverse(T, Y, W + 32 * kLd, false, tid - 128, 2);
   __syncthreads();
-  for (int e = tid; e < nbk * nbk; e += 256) {
-    int r = e % nbk, c = e / nbk;
-    A[(size_t)(k0 + c) * lda + k0 + r] = T[c * kLd + r];
-    put_expanded_rm(invL, 2 * kNB, r, c, X[c * kLd + r]);
-    put_expanded(invU, 2 * kNB, r, c, Y[c * kLd + r]);
+  auto linv = [&](int r, int c) {  // L^-1(r, c), r, c < nbk
+    if (c >= r) return make_float2(c == r ? 1.0f : 0.0f, 0.0f);
+    const int r0 = r & ~3;
+    return R[r * kRLd + (c < r0 ? 64 - r0 + c : c - r0)];
+  };
+  constexpr int K2 = 2 * kNB;
+  for (int e = tid; e < kNB * kNB; e += kLuThreads) {  // row by row: the row-major expansion of L^-1
+    const int r = e / kNB, c = e % kNB;
+    if (r < nbk && c < nbk) put_expanded_rm(invL, K2, r, c, linv(r, c));
   }
-  for (int e = tid; e < kNB * kNB; e += 256) {
-    int r = e % kNB, c = e / kNB;
-    invLc[e] = X[c * kLd + r];
-    invUc[e] = Y[c * kLd + r];
+  for (int e = tid; e < kNB * kNB; e += kLuThreads) {  // column by column
+    const int r = e % kNB, c = e / kNB;
+    const bool in = r < nbk && c < nbk;
+    const float2 id = make_float2(r == c ? 1.0f : 0.0f, 0.0f), x = in ? Ui[c * kUiLd + r] : id;
+    if (in) {
+      *reinterpret_cast<float2*>(invU + (size_t)(2 * c) * K2 + 2 * r) = x;
+      *reinterpret_cast<float2*>(invU + (size_t)(2 * c + 1) * K2 + 2 * r) = make_float2(-x.y, x.x);
+    }
+    invLc[e] = in ? linv(r, c) : id;
+    invUc[e] = x;
   }
-  for (int i = tid; i < nbk; i += 256) perm[k0 + i] = k0 + prm[i];
+  for (int i = tid; i < nbk; i += kLuThreads) perm[k0 + i] = k0 + prow[i];
 }
 
 
@@ -536,8 +553,7 @@ size_t mixed_lu_workspace_elems(int n, int nrhs) { return Layout(n, nrhs).total 
 
 int mixed_lu_factor(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasComputeType_t ct, int n, int lda,
                     float2* A, int* perm, float2* work, int* dinfo, long long* launches, long long* lib_calls) {
-  const int smem = (3 * kNB + 64) * kLd * (int)sizeof(float2);  // T, L^-1, U^-1, two 32-column scratches
-  if (cudaFuncSetAttribute(k_diag_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 1;
+  if (cudaFuncSetAttribute(k_diag_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiagSmem) != cudaSuccess) return 1;
   if (lda < n || (lda & 1)) return 1;
   const int K2 = 2 * kNB, PW = kPB * kNB;
   const Layout L(n, 0);
@@ -572,7 +588,7 @@ int mixed_lu_factor(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasC
                 k2 = 2 * nbk;
       float* iL = invL + (size_t)s * K2 * K2;
       float* iU = invU + (size_t)s * K2 * K2;
-      k_diag_lu<<<1, 256, smem, st>>>(A, lda, k0, nbk, perm, iL, iU, invLc + (size_t)b * kNB * kNB,
+      k_diag_lu<<<1, kLuThreads, kDiagSmem, st>>>(A, lda, k0, nbk, perm, iL, iU, invLc + (size_t)b * kNB * kNB,
                                       invUc + (size_t)b * kNB * kNB, dinfo);
       {  // the block's permutation and the expansion of its column below, one launch
         const int pb = (n + 31) / 32, nex = wr > 0 ? ((wr + 31) / 32) * ((nbk + 31) / 32) : 0;

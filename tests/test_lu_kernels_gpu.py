@@ -111,3 +111,25 @@ def test_block_lu_recorded_graphs_give_the_same_bits():
     assert "not recorded" not in graph.note(), graph.note()
     direct.close()
     graph.close()
+
+
+# 61, 62, 63, 64, 65, 66, 191, 74, 255, 256, 257 and 259 panels: around the 64-row diagonal blocks
+# and the 256-column panels
+@pytest.mark.parametrize("nl,nb,nz", [(3, 7, 2), (2, 9, 2), (3, 5, 3), (4, 4, 3), (5, 5, 2), (2, 3, 6), (7, 9, 4),
+                                      (2, 11, 2), (7, 9, 6), (8, 8, 6), (11, 7, 5), (11, 9, 4)],
+                         ids=lambda v: str(v))
+def test_block_lu_at_block_edges(nl, nb, nz):
+    """The block LU's diagonal blocks whole, nearly whole and with 1-3 columns left: no fallback to
+    the library's LU, a refinement that contracts, and the FP64 form's results.  Residuals of 1e-12
+    (mixed) and rounding (fp64) at the condition of these systems (below 1e3) leave 1e-9."""
+    xyz, ncn, ncon, cnt = meshgen.combine([meshgen.box(12.0, 7.0, 4.0, nl, nb, nz)])
+    geom = hams_b200.prepare_geometry(xyz, ncn, ncon, cnt, np.zeros((1, 3)))
+    res = {}
+    for prec in (hams_b200.PREC_FP64, hams_b200.PREC_MIXED):
+        ctx = hams_b200.Context(geom, 40.0, rho=1025.0, g=9.81, precision=prec)
+        res[prec] = ctx.solve_frequency(ctx.wave(0.8), [0.3])
+        if prec == hams_b200.PREC_MIXED:
+            assert ctx.note() == "" and ctx.timings()["ir_rate"] < 0.05
+        ctx.close()
+    for a, b in zip(res[hams_b200.PREC_FP64], res[hams_b200.PREC_MIXED]):
+        assert np.linalg.norm(a - b) < 1e-9 * np.linalg.norm(a)
