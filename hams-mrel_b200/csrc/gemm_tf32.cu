@@ -29,6 +29,7 @@
 #include <mutex>
 
 #include "gemm_tf32.h"
+#include "pdl.cuh"
 
 namespace {
 
@@ -133,6 +134,8 @@ __global__ void __launch_bounds__(kThreads, BN <= 128 ? 2 : 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = *reinterpret_cast<volatile uint32_t*>(tslot);
+  pdl_wait();  // the operands and C are the predecessors' results
+  pdl_next();
 
   if (warp == 0) {
     if (lane == 0) {  // producer
@@ -302,9 +305,10 @@ int launch(cudaStream_t st, int dev, int m, int n, int k, float alpha, const flo
   CUtensorMap ta, tb;
   if (!make_map(&ta, A, k, m, lda, kBM) || !make_map(&tb, B, k, n, ldb, BN)) return 1;
   dim3 grid((unsigned)((m + kBM - 1) / kBM), (unsigned)((n + BN - 1) / BN));
-  k_gemm_tf32<BN, STAGES><<<grid, kThreads, T::kSmemBytes, st>>>(ta, tb, C, ldc, m, n, k, alpha, beta,
-                                                                   c_rowmajor ? 1 : 0, err);
-  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+  return pdl_launch(k_gemm_tf32<BN, STAGES>, grid, dim3(kThreads), T::kSmemBytes, st, ta, tb, C, ldc, m, n, k, alpha,
+                    beta, c_rowmajor ? 1 : 0, err) == cudaSuccess
+             ? 0
+             : 1;
 }
 
 }  // namespace

@@ -49,6 +49,7 @@
 
 #include "gemm_tf32.h"
 #include "lu_mixed.h"
+#include "pdl.cuh"
 
 namespace {
 
@@ -140,6 +141,8 @@ __global__ void __launch_bounds__(kLuThreads) k_diag_lu(const float2* __restrict
   auto minus = [](float2 a, float2 l, float ux, float uy) {  // a - l u
     return make_float2(fmaf(-l.x, ux, fmaf(l.y, uy, a.x)), fmaf(-l.x, uy, fmaf(-l.y, ux, a.y)));
   };
+  pdl_wait();
+  pdl_next();
   if (warp < kLuRowWarps) {
     const int row = warp * 16 + (lane >> 1), h = lane & 1;  // places 4q + 2h, 4q + 2h + 1 of this row
     float2 a[16][2];
@@ -287,6 +290,8 @@ __global__ void __launch_bounds__(256) k_expand_rm(const float2* __restrict__ A,
                                                    int kc, float* __restrict__ E, int lde) {
   __shared__ float2 tile[32][33];
   const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  pdl_wait();
+  pdl_next();
   for (int c = ty; c < 32; c += 8)
     if (i0 + tx < w && k0 + c < kc) tile[c][tx] = A[(size_t)(c0 + k0 + c) * lda + r0 + i0 + tx];
   __syncthreads();
@@ -301,6 +306,8 @@ __global__ void __launch_bounds__(256) k_extract_l(const float* __restrict__ Lha
                                                    float2* __restrict__ A, int lda, int k1, int k0) {
   __shared__ float2 tile[32][33];
   const int i0 = blockIdx.x * 32, c0 = blockIdx.y * 32, tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  pdl_wait();
+  pdl_next();
   for (int r = ty; r < 32; r += 8)
     if (i0 + r < wr && c0 + tx < nbk)
       tile[r][tx] = make_float2(Lhat[(size_t)(2 * (i0 + r)) * ldl + 2 * (c0 + tx)],
@@ -323,6 +330,8 @@ __global__ void __launch_bounds__(256) k_perm_expand(float2* A, int lda, int n, 
                                                      float* __restrict__ E, int lde) {
   __shared__ float2 tile[kNB][33];
   const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;  // 8 x 32
+  pdl_wait();
+  pdl_next();
   if ((int)blockIdx.x < pblocks) {
     const int c = blockIdx.x * 32 + tx;
     const bool live = c < n && (c < k0 || c >= k0 + nbk);
@@ -405,6 +414,8 @@ __global__ void __launch_bounds__(256, 1) k_panel_inverse(const float2* __restri
   const int p0 = p * kPW, pw = min(kPW, n - p0), nbk = (pw + kNB - 1) / kNB;
   const float2* invc = lower ? invLc : invUc;
   float* out = (lower ? invLp : invUp) + (size_t)p * kPLd * kPLd;
+  pdl_wait();
+  pdl_next();
   for (int e = tid; e < kPLd * kPLd / 4; e += 256) reinterpret_cast<float4*>(out)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   auto width = [&](int b) { return min(kNB, pw - b * kNB); };
   auto write_block = [&](const float2* zb, int bi, int bj) {
@@ -457,6 +468,8 @@ __global__ void __launch_bounds__(256, 1) k_panel_inverse(const float2* __restri
 __global__ void k_gather_rows(const float2* __restrict__ B, int n, int nrhs, const int* __restrict__ perm,
                               float2* __restrict__ Y, int ldy) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  pdl_wait();
+  pdl_next();
   if (r >= ldy || q >= nrhs) return;
   Y[(size_t)q * ldy + r] = r < n ? B[(size_t)q * n + (perm ? perm[r] : r)] : make_float2(0.0f, 0.0f);
 }
@@ -464,6 +477,8 @@ __global__ void k_gather_rows(const float2* __restrict__ B, int n, int nrhs, con
 // X (n x nrhs, ld n) <- the first n rows of Y (ld ldy).
 __global__ void k_copy_rows(const float2* __restrict__ Y, int ldy, int n, int nrhs, float2* __restrict__ X) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+  pdl_wait();
+  pdl_next();
   if (r >= n || q >= nrhs) return;
   X[(size_t)q * n + r] = Y[(size_t)q * ldy + r];
 }
@@ -574,7 +589,7 @@ int mixed_lu_factor(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasC
   const int ldr = 2 * lda;
   auto expand = [&](int r0, int c0, int w, int kc, float* E, int lde) {
     dim3 grid((unsigned)((w + 31) / 32), (unsigned)((kc + 31) / 32));
-    k_expand_rm<<<grid, 256, 0, st>>>(A, lda, r0, c0, w, kc, E, lde);
+    pdl_launch(k_expand_rm, grid, dim3(256), 0, st, A, lda, r0, c0, w, kc, E, lde);
     *launches += 1;
     return cudaGetLastError() == cudaSuccess;
   };
@@ -588,11 +603,11 @@ int mixed_lu_factor(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasC
                 k2 = 2 * nbk;
       float* iL = invL + (size_t)s * K2 * K2;
       float* iU = invU + (size_t)s * K2 * K2;
-      k_diag_lu<<<1, kLuThreads, kDiagSmem, st>>>(A, lda, k0, nbk, perm, iL, iU, invLc + (size_t)b * kNB * kNB,
-                                      invUc + (size_t)b * kNB * kNB, dinfo);
+      pdl_launch(k_diag_lu, dim3(1), dim3(kLuThreads), kDiagSmem, st, A, lda, k0, nbk, perm, iL, iU,
+                 invLc + (size_t)b * kNB * kNB, invUc + (size_t)b * kNB * kNB, dinfo);
       {  // the block's permutation and the expansion of its column below, one launch
         const int pb = (n + 31) / 32, nex = wr > 0 ? ((wr + 31) / 32) * ((nbk + 31) / 32) : 0;
-        k_perm_expand<<<pb + nex, 256, 0, st>>>(A, lda, n, k0, nbk, perm, pb, wr, Ehat, K2);
+        pdl_launch(k_perm_expand, dim3(pb + nex), dim3(256), 0, st, A, lda, n, k0, nbk, perm, pb, wr, Ehat, K2);
       }
       *launches += 2;
       if (cudaGetLastError() != cudaSuccess) return 1;
@@ -608,7 +623,7 @@ int mixed_lu_factor(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasC
       }
       {  // L_ik into A
         dim3 grid((unsigned)((wr + 31) / 32), (unsigned)((nbk + 31) / 32));
-        k_extract_l<<<grid, 256, 0, st>>>(Lhat, K2, wr, nbk, A, lda, k1, k0);
+        pdl_launch(k_extract_l, grid, dim3(256), 0, st, Lhat, K2, wr, nbk, A, lda, k1, k0);
         *launches += 1;
         if (cudaGetLastError() != cudaSuccess) return 1;
       }
@@ -639,7 +654,8 @@ int mixed_lu_factor(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasC
   if (cudaFuncSetAttribute(k_panel_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, kInvSmem) != cudaSuccess)
     return 1;
   const int np = (n + kPW - 1) / kPW;
-  k_panel_inverse<<<dim3((unsigned)np, 2), 256, kInvSmem, st>>>(A, lda, n, invLc, invUc, ws + L.invLp, ws + L.invUp);
+  pdl_launch(k_panel_inverse, dim3((unsigned)np, 2), dim3(256), kInvSmem, st, A, lda, n, invLc, invUc, ws + L.invLp,
+             ws + L.invUp);
   *launches += 1;
   if (cudaGetLastError() != cudaSuccess) return 1;
   return 0;
@@ -678,12 +694,12 @@ int mixed_lu_solve(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasCo
   Gemm g{own_gemm, blas, ct, st, dflag, launches, lib_calls};
   auto expand = [&](int r0, int c0, int w, int kc, int lde) {
     dim3 grid((unsigned)((w + 31) / 32), (unsigned)((kc + 31) / 32));
-    k_expand_rm<<<grid, 256, 0, st>>>(A, lda, r0, c0, w, kc, Ebig, lde);
+    pdl_launch(k_expand_rm, grid, dim3(256), 0, st, A, lda, r0, c0, w, kc, Ebig, lde);
     *launches += 1;
     return cudaGetLastError() == cudaSuccess;
   };
   const dim3 rows((unsigned)((nl + 255) / 256), (unsigned)nrhs);
-  k_gather_rows<<<rows, 256, 0, st>>>(X, n, nrhs, perm, Y, nl);  // Y = P X
+  pdl_launch(k_gather_rows, rows, dim3(256), 0, st, X, n, nrhs, perm, Y, nl);  // Y = P X
   *launches += 1;
   if (cudaGetLastError() != cudaSuccess) return 1;
   int rc;
@@ -712,7 +728,7 @@ int mixed_lu_solve(cudaStream_t st, cublasHandle_t blas, bool own_gemm, cublasCo
         return 10 + rc;
     }
   }
-  k_copy_rows<<<dim3((unsigned)((n + 255) / 256), (unsigned)nrhs), 256, 0, st>>>(Y, nl, n, nrhs, X);
+  pdl_launch(k_copy_rows, dim3((unsigned)((n + 255) / 256), (unsigned)nrhs), dim3(256), 0, st, Y, nl, n, nrhs, X);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
