@@ -166,13 +166,27 @@ __device__ __noinline__ double pidcock_image(int table, double r, double zf, dou
 // read and written per entry) measured the same within 3 %, one loop body for
 // all columns (less code, idle rows computed) 6-20 % slower.
 constexpr int kSerThreads = 96;
-template <int BR>
+// What a launch evaluates: panel pairs, combined into A and S, or the points
+// of hams_eval_green (a chunk of its list, point t of the chunk being source t
+// and field point t of g), whose G and gradient go to out.
+struct PairIO {
+  static constexpr bool kPoints = false;
+  const uint32_t* __restrict__ pairs;
+  const double* __restrict__ rs;
+  const double* __restrict__ rd;
+  double2* __restrict__ A;
+  double2* __restrict__ S;
+};
+struct PointIO {
+  static constexpr bool kPoints = true;
+  const uint32_t* __restrict__ list;
+  const int* __restrict__ flag;
+  double2* __restrict__ out;
+  size_t npts;
+};
+template <int BR, class IO>
 __global__ void __launch_bounds__(kSerThreads, 5) k_green_series(DevGeom g, WaveDev w, const double* __restrict__ wvn,
-                                                                 hams::ModeTab mt, RadTab rt,
-                                                                 const uint32_t* __restrict__ pairs, long long count,
-                                                                 const double* __restrict__ rs,
-                                                                 const double* __restrict__ rd,
-                                                                 double2* __restrict__ A, double2* __restrict__ S,
+                                                                 hams::ModeTab mt, RadTab rt, IO io, long long count,
                                                                  int* ovf, int rows) {
   extern __shared__ double sm[];
   __shared__ double2 dz[32];
@@ -181,15 +195,27 @@ __global__ void __launch_bounds__(kSerThreads, 5) k_green_series(DevGeom g, Wave
   const long long t0 = ((long long)gridDim.x - 1 - blockIdx.x) * 32 + lane;
   const bool live = t0 < count;
   const long long t = live ? t0 : count - 1;
-  const uint32_t p = pairs[t], tn = (uint32_t)g.tn;
-  const int j = (int)(p / tn), i = (int)(p - (uint32_t)j * tn);
-  const int flag = near_flag(g, i, j);
+  uint32_t p;
+  int i, j, flag;
+  if constexpr (IO::kPoints) {
+    p = io.list[t];
+    i = j = (int)t;
+    flag = io.flag[p];
+  } else {
+    const uint32_t tn = (uint32_t)g.tn;
+    p = io.pairs[t];
+    j = (int)(p / tn);
+    i = (int)(p - (uint32_t)j * tn);
+    flag = near_flag(g, i, j);
+  }
   const double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], zp = g.fxyz[i + 2 * g.tn];
   const double xq = g.xq[j], yq = g.xq[j + g.n], zq = g.xq[j + 2 * g.n];
-  if (w.limit) {
-    if (table == 0 && live)
-      store_pair(g, p, i, j, hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag), rs, rd, A, S);
-    return;
+  if constexpr (!IO::kPoints) {
+    if (w.limit) {
+      if (table == 0 && live)
+        store_pair(g, p, i, j, hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag), io.rs, io.rd, io.A, io.S);
+      return;
+    }
   }
   const double xpq = xq - xp, ypq = yq - yp, zpq = zq + zp, h = w.h;
   const double rr = sqrt(xpq * xpq + ypq * ypq);
@@ -274,13 +300,21 @@ __global__ void __launch_bounds__(kSerThreads, 5) k_green_series(DevGeom g, Wave
     v.re -= (ir + ir1);
     v.re += flag == 1 ? ir1 : ir1 + ir;
     if (live) {
-      const double ds = g.ds[j];
-      S[p] = make_double2(rs[p] + v.re * ds, v.im * ds);
+      if constexpr (IO::kPoints) {
+        io.out[p] = make_double2(v.re, v.im);
+      } else {
+        const double ds = g.ds[j];
+        io.S[p] = make_double2(io.rs[p] + v.re * ds, v.im * ds);
+      }
     }
   } else if (table == 2) {
     v.re += ((zq - zp) / r / (r * r) + zpq / r1 / (r1 * r1));
     v.re -= flag == 1 ? zpq * ir13 : zpq * ir13 + (zq - zp) * ir3;
-    dz[lane] = make_double2(v.re, v.im);
+    if constexpr (IO::kPoints) {
+      if (live) io.out[p + 3 * io.npts] = make_double2(v.re, v.im);
+    } else {
+      dz[lane] = make_double2(v.re, v.im);
+    }
   }
   __syncthreads();
   if (table == 1 && live) {
@@ -292,12 +326,19 @@ __global__ void __launch_bounds__(kSerThreads, 5) k_green_series(DevGeom g, Wave
     }
     gx.re -= flag == 1 ? xpq * ir13 : xpq * ir13 + xpq * ir3;
     gy.re -= flag == 1 ? ypq * ir13 : ypq * ir13 + ypq * ir3;
+    if constexpr (IO::kPoints) {
+      io.out[p + io.npts] = make_double2(gx.re, gx.im);
+      io.out[p + 2 * io.npts] = make_double2(gy.re, gy.im);
+      return;
+    }
     const double2 gz = dz[lane];
     const double ds = g.ds[j], n1 = g.nrm[j], n2 = g.nrm[j + g.n], n3 = g.nrm[j + 2 * g.n];
-    double are = rd[p] + ds * (gx.re * n1 + gy.re * n2 + gz.x * n3);
-    const double aim = ds * (gx.im * n1 + gy.im * n2 + gz.y * n3);
-    if (i == j) are += 2.0 * 3.141592653589793;
-    A[p] = make_double2(are, aim);
+    if constexpr (!IO::kPoints) {
+      double are = io.rd[p] + ds * (gx.re * n1 + gy.re * n2 + gz.x * n3);
+      const double aim = ds * (gx.im * n1 + gy.im * n2 + gz.y * n3);
+      if (i == j) are += 2.0 * 3.141592653589793;
+      io.A[p] = make_double2(are, aim);
+    }
   }
 }
 
@@ -307,23 +348,30 @@ static size_t series_smem(int rows) {
 }
 
 int series_kernels_init() {
-  return cudaFuncSetAttribute(k_green_series<hams::kPidcock>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)series_smem(hams::kPidcockMax)) != cudaSuccess ||
-         cudaFuncSetAttribute(k_green_series<hams::kEigenE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)series_smem(hams::kEigenEMax)) != cudaSuccess;
+  auto opt = [](const void* f, int rows) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)series_smem(rows)) != cudaSuccess;
+  };
+  return opt((const void*)k_green_series<hams::kPidcock, PairIO>, hams::kPidcockMax) ||
+         opt((const void*)k_green_series<hams::kEigenE, PairIO>, hams::kEigenEMax) ||
+         opt((const void*)k_green_series<hams::kPidcock, PointIO>, hams::kPidcockMax) ||
+         opt((const void*)k_green_series<hams::kEigenE, PointIO>, hams::kEigenEMax);
+}
+
+template <class IO>
+static void launch_series(int br, int ntmax, cudaStream_t st, const DevGeom& g, const WaveDev& w, const double* wvn,
+                          const hams::ModeTab& mt, const RadTab& rt, const IO& io, long long count, int* ovf) {
+  const unsigned blocks = (unsigned)((count + 31) / 32);
+  const size_t sh = series_smem(ntmax);
+  if (br == hams::kPidcock)
+    k_green_series<hams::kPidcock, IO><<<blocks, kSerThreads, sh, st>>>(g, w, wvn, mt, rt, io, count, ovf, ntmax);
+  else
+    k_green_series<hams::kEigenE, IO><<<blocks, kSerThreads, sh, st>>>(g, w, wvn, mt, rt, io, count, ovf, ntmax);
 }
 
 void launch_green_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,
                          const hams::ModeTab& mt, RadTab rt, const uint32_t* pairs, long long count, const double* rs,
                          const double* rd, double2* A, double2* S, int* ovf) {
-  const unsigned blocks = (unsigned)((count + 31) / 32);
-  const size_t sh = series_smem(ntmax);
-  if (br == hams::kPidcock)
-    k_green_series<hams::kPidcock>
-        <<<blocks, kSerThreads, sh, st>>>(g, w, wvn, mt, rt, pairs, count, rs, rd, A, S, ovf, ntmax);
-  else
-    k_green_series<hams::kEigenE>
-        <<<blocks, kSerThreads, sh, st>>>(g, w, wvn, mt, rt, pairs, count, rs, rd, A, S, ovf, ntmax);
+  launch_series(br, ntmax, st, g, w, wvn, mt, rt, PairIO{pairs, rs, rd, A, S}, count, ovf);
 }
 
 // Per-frequency mode tables (ModeTab) for modes 2..nmode-1: one thread per
@@ -377,11 +425,14 @@ void launch_mode_tables(cudaStream_t st, DevGeom g, WaveDev w, const double* wvn
   k_mode_tables<<<grid, 128, 0, st>>>(g, w, wvn, nmode, pm, ac, src, srct, fld, fldt);
 }
 
-// Batch Green evaluation of hams_eval_green: any branch, one pair per thread.
+// Batch Green evaluation: any branch, one pair per thread; list (count
+// entries): the points to evaluate, or null for all.
 __global__ void k_eval_green(int npts, const double* __restrict__ pts, const int* __restrict__ flag, WaveDev w,
-                             const double* __restrict__ wvn, double2* __restrict__ out, int* ovf) {
+                             const double* __restrict__ wvn, double2* __restrict__ out, int* ovf,
+                             const uint32_t* __restrict__ list, int count) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npts) return;
+  if (t >= count) return;
+  if (list) t = (int)list[t];
   double xq = pts[t], yq = pts[t + npts], zq = pts[t + 2 * (size_t)npts];
   double xp = pts[t + 3 * (size_t)npts], yp = pts[t + 4 * (size_t)npts], zp = pts[t + 5 * (size_t)npts];
   grn4 G;
@@ -411,6 +462,97 @@ __global__ void k_eval_green(int npts, const double* __restrict__ pts, const int
   for (int k = 0; k < 4; ++k) out[t + (size_t)k * npts] = make_double2(G.g[k].re, G.g[k].im);
 }
 
+// The points of hams_eval_green, sorted by branch and series length
+// (kPointBins keys): a histogram, the offsets formed by the host, and the
+// points filed into their bins (the order inside a bin is free: every point is
+// computed by itself).
+__global__ void __launch_bounds__(256) k_point_bins(int npts, const double* __restrict__ pts, double h,
+                                                    unsigned short* __restrict__ key, uint32_t* __restrict__ hist) {
+  __shared__ uint32_t sh[kPointBins];
+  for (int b = threadIdx.x; b < kPointBins; b += blockDim.x) sh[b] = 0;
+  __syncthreads();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < npts) {
+    const double dx = pts[t] - pts[t + 3 * (size_t)npts], dy = pts[t + npts] - pts[t + 4 * (size_t)npts];
+    const double rr = sqrt(dx * dx + dy * dy);
+    const int k = hams::fin_branch(rr, h) * kPointTerms + min(max(hams::fin_terms(rr, h), 0), kPointTerms - 1);
+    key[t] = (unsigned short)k;
+    atomicAdd(&sh[k], 1u);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < kPointBins; b += blockDim.x)
+    if (sh[b]) atomicAdd(&hist[b], sh[b]);
+}
+__global__ void k_point_file(int npts, const unsigned short* __restrict__ key, uint32_t* __restrict__ next,
+                             uint32_t* __restrict__ list) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < npts) list[atomicAdd(&next[key[t]], 1u)] = (uint32_t)t;
+}
+// A chunk of the list as sources xq and field points fx (m x 3 each) with
+// their distances r.
+__global__ void k_point_gather(int npts, const double* __restrict__ pts, const uint32_t* __restrict__ list, int m,
+                               double* __restrict__ xq, double* __restrict__ fx, double* __restrict__ r) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= m) return;
+  const size_t p = list[t];
+  double q[6];
+  for (int k = 0; k < 6; ++k) q[k] = pts[p + k * (size_t)npts];
+  for (int k = 0; k < 3; ++k) {
+    xq[t + k * m] = q[k];
+    fx[t + k * m] = q[3 + k];
+  }
+  const double xpq = q[0] - q[3], ypq = q[1] - q[4];
+  r[t] = sqrt(xpq * xpq + ypq * ypq);
+}
+// LINTON points, a warp each (hams::WarpQuad); lane 0 stores.
+constexpr int kPointWarps = 4;
+__global__ void __launch_bounds__(32 * kPointWarps) k_point_linton(int npts, const double* __restrict__ pts,
+                                                                   const int* __restrict__ flag, WaveDev w,
+                                                                   const double* __restrict__ wvn,
+                                                                   const uint32_t* __restrict__ list, int count,
+                                                                   double2* __restrict__ out, int* ovf) {
+  __shared__ double stack[kPointWarps][2][hams::kQuadStack];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5, k = blockIdx.x * kPointWarps + wl;
+  if (k >= count) return;  // the whole warp
+  const size_t t = list[k], n = npts;
+  int o = 0;
+  const hams::WarpQuad quad{stack[wl][0], stack[wl][1], lane};
+  const grn4 G = hams::fingreen3d_linton(pts[t], pts[t + 3 * n], pts[t + n], pts[t + 4 * n], pts[t + 2 * n],
+                                         pts[t + 5 * n], w.v, wvn, w.h, flag[t], &o, quad);
+  if (lane != 0) return;
+  if (o) atomicOr(ovf, 1);
+  for (int q = 0; q < 4; ++q) out[t + q * n] = make_double2(G.g[q].re, G.g[q].im);
+}
+
+void launch_point_bins(cudaStream_t st, int npts, const double* pts, double h, unsigned short* key, uint32_t* hist) {
+  k_point_bins<<<(npts + 255) / 256, 256, 0, st>>>(npts, pts, h, key, hist);
+}
+void launch_point_file(cudaStream_t st, int npts, const unsigned short* key, uint32_t* next, uint32_t* list) {
+  k_point_file<<<(npts + 255) / 256, 256, 0, st>>>(npts, key, next, list);
+}
+void launch_point_linton(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
+                         const uint32_t* list, int count, double2* out, int* ovf) {
+  k_point_linton<<<(count + kPointWarps - 1) / kPointWarps, 32 * kPointWarps, 0, st>>>(npts, pts, flag, w, wvn, list,
+                                                                                       count, out, ovf);
+}
+void launch_point_eigen(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
+                        const uint32_t* list, int count, double2* out, int* ovf) {
+  k_eval_green<<<(count + 127) / 128, 128, 0, st>>>(npts, pts, flag, w, wvn, out, ovf, list, count);
+}
+void launch_point_series(int br, int ntmax, cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w,
+                         const double* wvn, const uint32_t* list, int m, const PointWork& pw, double2* out, int* ovf) {
+  k_point_gather<<<(m + 127) / 128, 128, 0, st>>>(npts, pts, list, m, pw.xq, pw.fx, pw.r);
+  DevGeom g{};
+  g.n = g.tn = m;
+  g.xq = pw.xq;
+  g.fxyz = pw.fx;
+  const int nmode = ntmax + 1;
+  launch_mode_tables(st, g, w, wvn, nmode, pw.pm, pw.ac, pw.src, pw.srct, pw.fld, pw.fldt);
+  const hams::ModeTab mt{m, m, nmode, pw.pm, pw.ac, pw.src, pw.srct, pw.fld, pw.fldt};
+  launch_rad_series(br, st, g, w, wvn, pw.r, nullptr, m, pw.kt, pw.jy);
+  launch_series(br, ntmax, st, g, w, wvn, mt, RadTab{nullptr, 0, pw.kt, pw.jy}, PointIO{list, flag, out, (size_t)npts},
+                m, ovf);
+}
 
 // Source (S) and normal-dipole (D) influence of every hull panel J at field
 // point f, the terms CalPotentialMulti sums (PressureElevationMulti.f90:81-137):
@@ -482,5 +624,5 @@ void launch_field_pairs(cudaStream_t st, DevGeom g, WaveDev w, const double* wvn
 
 void launch_eval_green(unsigned blocks, cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w,
                        const double* wvn, double2* out, int* ovf) {
-  k_eval_green<<<blocks, 128, 0, st>>>(npts, pts, flag, w, wvn, out, ovf);
+  k_eval_green<<<blocks, 128, 0, st>>>(npts, pts, flag, w, wvn, out, ovf, nullptr, npts);
 }

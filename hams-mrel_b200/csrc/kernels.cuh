@@ -90,6 +90,24 @@ void launch_mode_tables(cudaStream_t st, DevGeom g, WaveDev w, const double* wvn
                         double2* src, double2* srct, double* fld, double* fldt);
 void launch_eval_green(unsigned blocks, cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w,
                        const double* wvn, double2* out, int* ovf);
+// The points of hams_eval_green by branch (kPointTerms keys each) and series
+// length: key and histogram, the lists, and each branch's points from its list
+// (the series a chunk of at most kPointChunk points at a time, whose mode and
+// radial tables pw holds).
+constexpr int kPointTerms = 128, kPointBins = 4 * kPointTerms, kPointChunk = 8192;
+struct PointWork {
+  double *xq, *fx, *r, *pm, *ac, *fld, *fldt, *kt;
+  double2 *src, *srct;
+  double4* jy;
+};
+void launch_point_bins(cudaStream_t st, int npts, const double* pts, double h, unsigned short* key, uint32_t* hist);
+void launch_point_file(cudaStream_t st, int npts, const unsigned short* key, uint32_t* next, uint32_t* list);
+void launch_point_linton(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
+                         const uint32_t* list, int count, double2* out, int* ovf);
+void launch_point_eigen(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
+                        const uint32_t* list, int count, double2* out, int* ovf);
+void launch_point_series(int br, int ntmax, cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w,
+                         const double* wvn, const uint32_t* list, int m, const PointWork& pw, double2* out, int* ovf);
 // Influence of every hull panel at nfp field points xfp (nfp,3): Sf, Df (nfp x n).
 void launch_field_pairs(cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, int nfp, const double* xfp,
                         double2* Sf, double2* Df, int* ovf);

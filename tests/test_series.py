@@ -138,3 +138,29 @@ def test_assembly_over_distance_patterns(mesh):
         for got, ref in ((a[::stride], oa[:, :, 0]), (b[::stride], ob[:, :, 0]), (d[::stride], od[:, 0, :])):
             assert np.linalg.norm(got - ref) < 1e-10 * np.linalg.norm(ref)
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 97, 4096])
+@pytest.mark.parametrize("lo,hi", [(1e-4, 2.0), (0.0005, 0.05), (0.05, 0.5)])
+def test_points_by_branch_equal_points_one_by_one(n, lo, hi):
+    """hams_eval_green files its points by branch and series length; hams_eval_green_static takes them
+    a thread each, as they come.  The EIGENE and PIDCOCK sums have the same bits either way, and so has
+    LINTON's quadrature by lanes: the results are equal."""
+    lib = hams_b200.load_library()
+    lib.hams_eval_green_static.argtypes = lib.hams_eval_green.argtypes
+    xyz, ncn, ncon, cnt = meshgen.combine([meshgen.cylinder(4.0, 4.0, 8, 2, 2)])
+    ctx = hams_b200.Context(hams_b200.prepare_geometry(xyz, ncn, ncon, cnt, np.zeros((1, 3))), 31.0, g=9.81)
+    rng = np.random.default_rng(n)
+    r, th = 31.0 * np.exp(rng.uniform(np.log(lo), np.log(hi), n)), rng.uniform(0.0, 6.28, n)
+    pts = np.zeros((n, 6), order="F")
+    pts[:, 3], pts[:, 4] = r * np.cos(th), r * np.sin(th)
+    pts[:, 2], pts[:, 5] = rng.uniform(-12.0, -0.3, n), rng.uniform(-12.0, -0.3, n)
+    flag = (rng.uniform(size=n) < 0.5).astype(np.int32)
+    wave = ctx.wave(1.3)
+    got, ref = ctx.eval_green(wave, pts, flag), np.zeros((n, 4), dtype=np.complex128, order="F")
+    assert lib.hams_eval_green_static(ctx._h, ctypes.byref(wave), n, pts.ctypes.data_as(hams_b200.P_dbl),
+                                      flag.ctypes.data_as(hams_b200.P_int),
+                                      ref.ctypes.data_as(hams_b200.P_dbl)) == 0
+    assert np.array_equal(got, ref)
+    ctx.close()
