@@ -500,6 +500,10 @@ struct ThreadQuad {
   }
 };
 
+template <class F>
+struct LaneShared {
+  static constexpr bool value = false;
+};
 struct WarpQuad {
   double* sa;  // kQuadStack interval bounds each, this warp's shared memory
   double* sb;
@@ -517,11 +521,13 @@ struct WarpQuad {
       --sp;
       const double x0 = sa[sp], x1 = sb[sp], hw = (x1 - x0) / 2.0;
       double fv = 0.0;
-      if (lane < 15) {  // Kronrod node lane + 1; the even ones are the Gauss nodes
-        const int kk = lane + 1;
-        const double c = (kk % 2 == 0) ? c_xgq[kk / 2 - 1] : c_xkq[kk - 1];
-        fv = f(0.5 * (x1 + x0 + (x1 - x0) * c));
-      }
+      // Kronrod node lane + 1; the even ones are the Gauss nodes.  An integrand
+      // that takes the lane shares a node between lanes k and k + 16.
+      const int kk = (lane & 15) < 15 ? (lane & 15) + 1 : 15;
+      const double c = (kk % 2 == 0) ? c_xgq[kk / 2 - 1] : c_xkq[kk - 1];
+      const double x = 0.5 * (x1 + x0 + (x1 - x0) * c);
+      if constexpr (LaneShared<F>::value) fv = f(x, lane);
+      else if (lane < 15) fv = f(x);
       double v[15];
 #pragma unroll
       for (int k = 0; k < 15; ++k) v[k] = __shfl_sync(0xffffffffu, fv, k);
@@ -553,6 +559,34 @@ struct WarpQuad {
     }
     return sum;
   }
+};
+
+// G1/G2/G3 with a node's four terms shared by lanes k (the first two) and
+// k + 16; lane k has the value.
+struct LinGLanes {
+  int tag;
+  double v, r, zf, zp, h;
+  __device__ __forceinline__ double operator()(double t, int lane) const {
+    const double val[4] = {-zp - zf, 2.0 * h - zp + zf, 2.0 * h + zp - zf, 4.0 * h + zp + zf};
+    double s[2] = {0.0, 0.0};
+    const bool zero = fabs(t) < 1.0e-8;
+    if (!zero) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const double vi = lane < 16 ? val[q] : val[2 + q], dval = q ? 1.0 : -1.0;
+        const double ev = exp(-v * vi), arg = vi / 2.0 / t - v * t;
+        s[q] = tag == 3 ? -v * dval * ev * erfc_zj(arg) + ev * derfc_zj(arg) * dval / 2.0 / t : ev * erfc_zj(arg);
+      }
+    }
+    const double s2 = __shfl_down_sync(0xffffffffu, s[0], 16), s3 = __shfl_down_sync(0xffffffffu, s[1], 16);
+    if (zero) return 0.0;
+    const double sum = s[0] + s[1] + s2 + s3, e = exp(v * v * (t * t) - (r * r) / 4.0 / (t * t));
+    return tag == 2 ? r / 2.0 / (t * t * t) * e * sum : e * sum / t;
+  }
+};
+template <>
+struct LaneShared<LinGLanes> {
+  static constexpr bool value = true;
 };
 
 // SA0/DSA0/SAM/DSAM series (FinGreen3D.f90:1389-1740)
@@ -652,17 +686,22 @@ __device__ __forceinline__ cplx nm_mode(double h, cplx k) {  // NM, FinGreen3D.f
   return cmk(h / 2.0 * (1.0 + q.re), h / 2.0 * q.im);
 }
 
-template <class Q = ThreadQuad>
-__device__ inline void linton(double r, double zf, double zp, double v, double wk, const double* __restrict__ wvn,
-                              double h, cplx g[3], int* overflow, const Q& quad = Q{}) {
-  const double pi = 3.141592653589793, eps = HAMS_F4(1.E-6);
+// The splitting parameter A of LINTON (FinGreen3D.f90:735-745)
+__device__ inline double linton_split(double v, double wk, double h) {
   double a;
   if (v < 0.02) a = 3324.2 * (v * v * v) - 258.89 * (v * v) + 8.3958 * v + 1.3208;
   else if (v < 0.1) a = -30.303 * (v * v * v) - 2.8138 * (v * v) + 2.7740 * v + 0.05052;
   else if (v < 1.0) a = 1.5699 * (v * v * v) - 2.5075 * (v * v) + 1.8316 * v + 0.1077;
   else a = -0.000069641 * (v * v * v) - 0.0017082 * (v * v) + 0.45566 * v + 0.80551;
-  a = fabs(a) / (wk * h);
-  double pa = a * h;
+  return fabs(a) / (wk * h);
+}
+
+// Its mode sum (g) and image sums (es), FinGreen3D.f90:746-832.
+template <class Q>
+__device__ inline void linton_sums(double r, double zf, double zp, double wk, double a, const double* __restrict__ wvn,
+                                   double h, cplx g[3], double es[3], int* overflow, const Q& quad) {
+  const double pi = 3.141592653589793, eps = HAMS_F4(1.E-6);
+  const double pa = a * h;
   double sr = sqrt(r * r + (zf - zp) * (zf - zp));
   double sr1 = sqrt(r * r + (2.0 * h + zf + zp) * (2.0 * h + zf + zp));
   double sr2 = sqrt(r * r + (zf + zp) * (zf + zp));
@@ -713,12 +752,18 @@ __device__ inline void linton(double r, double zf, double zp, double v, double w
     es2 = es2 - e1 / (4.0 * pi * (sr1 * sr1)) * dsr1z + d1 / (4.0 * pi * sr1 * pa) * dsr1z +
           dsr2z / (4.0 * pi * (sr2 * sr2));
   }
-  double q1 = quad([=](double t) { return lin_g(1, v, r, zf, zp, h, t); }, 0.0, pa / 2.0, eps, overflow);
-  double q2 = quad([=](double t) { return lin_g(2, v, r, zf, zp, h, t); }, 0.0, pa / 2.0, eps, overflow);
-  double q3 = quad([=](double t) { return lin_g(3, v, r, zf, zp, h, t); }, 0.0, pa / 2.0, eps, overflow);
-  g[0].re = g[0].re - es0 - v / 2.0 / pi * q1;
-  g[1].re = g[1].re - es1 + v / 2.0 / pi * q2;
-  g[2].re = g[2].re - es2 - v / 2.0 / pi * q3;
+  es[0] = es0;
+  es[1] = es1;
+  es[2] = es2;
+}
+
+// LINTON's result from its sums and the integrals q of G1..G3.
+__device__ inline void linton_finish(double r, double zf, double zp, double v, double wk, double h, const double es[3],
+                                     const double q[3], cplx g[3]) {
+  const double pi = 3.141592653589793;
+  g[0].re = g[0].re - es[0] - v / 2.0 / pi * q[0];
+  g[1].re = g[1].re - es[1] + v / 2.0 / pi * q[1];
+  g[2].re = g[2].re - es[2] - v / 2.0 / pi * q[2];
 
   // propagating mode written with J0 only (FinGreen3D.f90:845-852)
   double j0, j1, y0, y1;
@@ -732,6 +777,17 @@ __device__ inline void linton(double r, double zf, double zp, double v, double w
   g[0] = -4.0 * pi * g[0];
   g[1] = -4.0 * pi * g[1];
   g[2] = -4.0 * pi * g[2];
+}
+
+template <class Q = ThreadQuad>
+__device__ inline void linton(double r, double zf, double zp, double v, double wk, const double* __restrict__ wvn,
+                              double h, cplx g[3], int* overflow, const Q& quad = Q{}) {
+  const double eps = HAMS_F4(1.E-6), a = linton_split(v, wk, h);
+  double es[3], q[3];
+  linton_sums(r, zf, zp, wk, a, wvn, h, g, es, overflow, quad);
+  for (int k = 0; k < 3; ++k)
+    q[k] = quad([=](double t) { return lin_g(k + 1, v, r, zf, zp, h, t); }, 0.0, a * h / 2.0, eps, overflow);
+  linton_finish(r, zf, zp, v, wk, h, es, q, g);
 }
 
 // Branch of FINGREEN3D_R (FinGreen3D.f90:183-191)

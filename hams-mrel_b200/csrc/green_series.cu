@@ -7,6 +7,8 @@
 // and sum of those series is rounded exactly as in the CPU checker; the
 // transcendental functions inside them come from detmath.h.  The remaining
 // kernels (hams_gpu.cu) keep fused multiply-adds.
+#include <atomic>
+
 #include "kernels.cuh"
 #include "epsilon.h"
 #include "rankine.cuh"
@@ -347,14 +349,22 @@ static size_t series_smem(int rows) {
   return ((size_t)hams::eps_columns(rows) * 8 + (size_t)hams::eps_pairs(rows) * 4) * kSerThreads;
 }
 
+// The shared-memory sizes of the series kernels, once per device.
 int series_kernels_init() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+  if (dev < 64 && done[dev]) return 0;
   auto opt = [](const void* f, int rows) {
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)series_smem(rows)) != cudaSuccess;
   };
-  return opt((const void*)k_green_series<hams::kPidcock, PairIO>, hams::kPidcockMax) ||
-         opt((const void*)k_green_series<hams::kEigenE, PairIO>, hams::kEigenEMax) ||
-         opt((const void*)k_green_series<hams::kPidcock, PointIO>, hams::kPidcockMax) ||
-         opt((const void*)k_green_series<hams::kEigenE, PointIO>, hams::kEigenEMax);
+  if (opt((const void*)k_green_series<hams::kPidcock, PairIO>, hams::kPidcockMax) ||
+      opt((const void*)k_green_series<hams::kEigenE, PairIO>, hams::kEigenEMax) ||
+      opt((const void*)k_green_series<hams::kPidcock, PointIO>, hams::kPidcockMax) ||
+      opt((const void*)k_green_series<hams::kEigenE, PointIO>, hams::kEigenEMax))
+    return 1;
+  if (dev < 64) done[dev] = true;
+  return 0;
 }
 
 template <class IO>

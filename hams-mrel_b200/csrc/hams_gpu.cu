@@ -495,68 +495,146 @@ __global__ void __launch_bounds__(128, 8) k_green_eigen(DevGeom g, WaveDev w, co
   store_pair(g, p, i, j, G, rs, rd, A, S);
 }
 
-// LINTON pairs, a thread each.
-__global__ void __launch_bounds__(128) k_green_linton_threads(DevGeom g, WaveDev w, const double* __restrict__ wvn,
-                                                              hams::ModeTab mt, const uint32_t* __restrict__ pairs,
-                                                              long long count, const double* __restrict__ rs,
-                                                              const double* __restrict__ rd, double2* __restrict__ A,
-                                                              double2* __restrict__ S, int* ovf) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  size_t p = pairs[t];
-  int i = (int)(p % (size_t)g.tn), j = (int)(p / (size_t)g.tn);
-  int flag = near_flag(g, i, j);
-  double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], zp = g.fxyz[i + 2 * g.tn];
-  double xq = g.xq[j], yq = g.xq[j + g.n], zq = g.xq[j + 2 * g.n];
-  grn4 G;
-  if (w.limit) {
-    G = hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag);
-  } else {
-    int o = 0;
-    hams::TableModes md{mt, j, i};
-    G = hams::fingreen3d<hams::kLinton>(xq, xp, yq, yp, zq, zp, w.v, wvn, w.h, flag, (void*)nullptr, &o, md);
-    if (o) atomicOr(ovf, 1);
-  }
-  store_pair(g, p, i, j, G, rs, rd, A, S);
+// LINTON (R/h < 0.0005) depends on a pair's distance and depths only, and its
+// pairs lie in vertical columns of panels: a 5,400-panel array of cylinders has
+// 37,800 pairs of 101 different (R, z, zeta).  The different triples are found
+// once per geometry (build_linton_rows), evaluated here, a row (G and its R and
+// z derivatives) each, and the rows given to their pairs by k_linton_pairs.
+// A row is a long FP64 chain: adaptive Gauss-Kronrod integrals of three
+// integrands and a mode sum.  Few rows: a block of four warps each, a warp per
+// integral (its fifteen nodes, two lanes a node) and one for the sums; many: a
+// thread each.  5,400
+// panels, every pair: 2.05 -> 0.14 ms; one body of 234 panels 0.31 -> 0.12 ms
+// (a warp or a thread per pair before).
+struct LintonPair {
+  int i, j;
+  double xpq, ypq, zq, zp, rr;
+};
+__device__ __forceinline__ LintonPair linton_pair(const DevGeom& g, uint32_t p) {
+  const uint32_t tn = (uint32_t)g.tn;
+  LintonPair q;
+  q.j = (int)(p / tn);
+  q.i = (int)(p - (uint32_t)q.j * tn);
+  const double xp = g.fxyz[q.i], yp = g.fxyz[q.i + g.tn], xq = g.xq[q.j], yq = g.xq[q.j + g.n];
+  q.zp = g.fxyz[q.i + 2 * g.tn];
+  q.zq = g.xq[q.j + 2 * g.n];
+  q.xpq = xq - xp;
+  q.ypq = yq - yp;
+  q.rr = sqrt(q.xpq * q.xpq + q.ypq * q.ypq);
+  return q;
+}
+__device__ __forceinline__ void linton_store(double2* __restrict__ fg, long long row, const cplx (&f)[3]) {
+  for (int k = 0; k < 3; ++k) fg[3 * row + k] = make_double2(f[k].re, f[k].im);
 }
 
-// The LINTON branch with one warp per pair: the pair's adaptive
-// Gauss-Kronrod integrals spread their nodes over the warp's lanes
-// (hams::WarpQuad); lane 0 stores the pair.  The branch has few pairs (the
-// panels of one vertical column of a body), each a long chain of FP64
-// quadrature, so a thread per pair leaves most of the GPU idle.  128 threads
-// per CTA, 4 pairs.
-constexpr int kLintonWarps = 4;
-// Below this many LINTON pairs per SM the warp-per-pair kernel runs (on the
-// 5,400-panel 3 x 3 array: 4,200 pairs with body blocks 1.5 ms against 6.5 ms
-// for a thread per pair at 0.2 rad/s; all 37,800 pairs 9.2 ms against 3.7 ms,
-// mean over frequencies).
-constexpr int kLintonWarpPairsPerSm = 64;
-__global__ void __launch_bounds__(32 * kLintonWarps) k_green_linton(DevGeom g, WaveDev w, const double* __restrict__ wvn,
-                                                                  const uint32_t* __restrict__ pairs, long long count,
-                                                                  const double* __restrict__ rs,
-                                                                  const double* __restrict__ rd,
-                                                                  double2* __restrict__ A, double2* __restrict__ S,
-                                                                  int* ovf) {
-  __shared__ double stack[kLintonWarps][2][hams::kQuadStack];
+__global__ void __launch_bounds__(128) k_linton_rows_threads(DevGeom g, WaveDev w, const double* __restrict__ wvn,
+                                                             const uint32_t* __restrict__ pairs,
+                                                             const uint32_t* __restrict__ rep, long long rows,
+                                                             double2* __restrict__ fg, int* ovf) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= rows) return;
+  const LintonPair q = linton_pair(g, pairs[rep ? rep[t] : t]);
+  cplx f[3];
+  int o = 0;
+  hams::linton(q.rr, q.zq, q.zp, w.v, wvn[0], wvn, w.h, f, &o);
+  if (o) atomicOr(ovf, 1);
+  linton_store(fg, t, f);
+}
+
+// Below this many rows per SM a block per row; above a thread per row (the
+// blocks' lanes repeat the work outside the integrals).
+constexpr int kLintonRowsPerSm = 64;
+__global__ void __launch_bounds__(128) k_linton_rows(DevGeom g, WaveDev w, const double* __restrict__ wvn,
+                                                     const uint32_t* __restrict__ pairs,
+                                                     const uint32_t* __restrict__ rep, double2* __restrict__ fg,
+                                                     int* ovf) {
+  __shared__ double stack[4][2][hams::kQuadStack];
+  __shared__ double integral[3];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const long long t = (long long)blockIdx.x * kLintonWarps + wl;
-  if (t >= count) return;  // the whole warp
-  size_t p = pairs[t];
-  int i = (int)(p % (size_t)g.tn), j = (int)(p / (size_t)g.tn);
-  int flag = near_flag(g, i, j);
-  double xp = g.fxyz[i], yp = g.fxyz[i + g.tn], zp = g.fxyz[i + 2 * g.tn];
-  double xq = g.xq[j], yq = g.xq[j + g.n], zq = g.xq[j + 2 * g.n];
+  const long long row = blockIdx.x;
+  const LintonPair q = linton_pair(g, pairs[rep ? rep[row] : row]);
+  const hams::WarpQuad quad{stack[wl][0], stack[wl][1], lane};
+  const double wk = wvn[0], a = hams::linton_split(w.v, wk, w.h);
+  cplx f[3];
+  double es[3];
+  int o = 0;
+  if (wl < 3) {
+    const double v = quad(hams::LinGLanes{wl + 1, w.v, q.rr, q.zq, q.zp, w.h}, 0.0, a * w.h / 2.0, HAMS_F4(1.E-6), &o);
+    if (lane == 0) integral[wl] = v;
+  } else {
+    hams::linton_sums(q.rr, q.zq, q.zp, wk, a, wvn, w.h, f, es, &o, quad);
+  }
+  if (o && lane == 0) atomicOr(ovf, 1);
+  __syncthreads();
+  if (wl < 3) return;
+  const double qs[3] = {integral[0], integral[1], integral[2]};
+  hams::linton_finish(q.rr, q.zq, q.zp, w.v, wk, w.h, es, qs, f);
+  if (lane == 0) linton_store(fg, row, f);
+}
+
+// A and S of the LINTON pairs from their rows.
+__global__ void __launch_bounds__(128) k_linton_pairs(DevGeom g, WaveDev w, const uint32_t* __restrict__ pairs,
+                                                      const uint32_t* __restrict__ lrow, long long count,
+                                                      const double2* __restrict__ fg, const double* __restrict__ rs,
+                                                      const double* __restrict__ rd, double2* __restrict__ A,
+                                                      double2* __restrict__ S) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t p = pairs[t];
+  const LintonPair q = linton_pair(g, p);
+  const int flag = near_flag(g, q.i, q.j);
   grn4 G;
   if (w.limit) {
-    G = hams::green_limit(w.limit == 2, xq, xp, yq, yp, zq, zp, flag);
+    G = hams::green_limit(w.limit == 2, g.xq[q.j], g.fxyz[q.i], g.xq[q.j + g.n], g.fxyz[q.i + g.tn], q.zq, q.zp, flag);
   } else {
-    int o = 0;
-    const hams::WarpQuad quad{stack[wl][0], stack[wl][1], lane};
-    G = hams::fingreen3d_linton(xq, xp, yq, yp, zq, zp, w.v, wvn, w.h, flag, &o, quad);
-    if (o && lane == 0) atomicOr(ovf, 1);
+    const long long row = lrow ? lrow[t] : t;
+    cplx f[3];
+    for (int k = 0; k < 3; ++k) f[k] = hams::cmk(fg[3 * row + k].x, fg[3 * row + k].y);
+    const double zpq = q.zq + q.zp;
+    const double r = sqrt(q.rr * q.rr + (q.zp - q.zq) * (q.zp - q.zq)), r1 = sqrt(q.rr * q.rr + zpq * zpq);
+    G = hams::finish_green(f, q.xpq, q.ypq, q.zq, q.zp, q.rr, r, r1, flag);
   }
-  if (lane == 0) store_pair(g, p, i, j, G, rs, rd, A, S);
+  store_pair(g, p, q.i, q.j, G, rs, rd, A, S);
+}
+
+// A 64-bit hash of a LINTON pair's (R, z, zeta); equal triples are neighbours
+// once sorted by it.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
+  x ^= x >> 30;
+  x *= 0xbf58476d1ce4e5b9ull;
+  x ^= x >> 27;
+  x *= 0x94d049bb133111ebull;
+  return x ^ (x >> 31);
+}
+__global__ void k_linton_keys(DevGeom g, const uint32_t* __restrict__ pairs, long long count,
+                              unsigned long long* __restrict__ key, uint32_t* __restrict__ idx) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const LintonPair q = linton_pair(g, pairs[t]);
+  unsigned long long k = mix64((unsigned long long)__double_as_longlong(q.rr) + 0x9e3779b97f4a7c15ull);
+  k = mix64(k ^ (unsigned long long)__double_as_longlong(q.zq));
+  key[t] = mix64(k + 3 * (unsigned long long)__double_as_longlong(q.zp));
+  idx[t] = (uint32_t)t;
+}
+// 1 at the first of equal triples, decided by the triples themselves
+__global__ void k_linton_heads(DevGeom g, const uint32_t* __restrict__ pairs, const uint32_t* __restrict__ idx,
+                               long long count, uint32_t* __restrict__ head) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  bool h = t == 0;
+  if (!h) {
+    const LintonPair a = linton_pair(g, pairs[idx[t]]), b = linton_pair(g, pairs[idx[t - 1]]);
+    h = a.rr != b.rr || a.zq != b.zq || a.zp != b.zp;
+  }
+  head[t] = h;
+}
+__global__ void k_linton_file(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ rank, long long count,
+                              uint32_t* __restrict__ lrow, uint32_t* __restrict__ rep) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t k = rank[t] - 1;
+  lrow[idx[t]] = k;
+  if (t == 0 || rank[t - 1] != rank[t]) rep[k] = idx[t];
 }
 
 __global__ void __launch_bounds__(128) k_green_inf(DevGeom g, WaveDev w, const unsigned char* __restrict__ copied,
@@ -1129,6 +1207,11 @@ struct hams_ctx {
   DBuf<int> ipiv, info, ovf;
   DBuf<char> work;
   DBuf<char> work32;
+  // LINTON rows: the row of every pair of bin 0 and a pair of each row (none:
+  // a row per pair), this frequency's rows
+  DBuf<uint32_t> lrow, lrep;
+  long long lin_rows = 0;
+  DBuf<double2> lin_fg;
   // timing: ev[0..5] stage marks, evb[0..4] branch marks, evf after the factorisation
   cudaEvent_t ev[6] = {};
   cudaEvent_t evb[6] = {};
@@ -1359,6 +1442,47 @@ static int build_pairs(hams_ctx* c) {
   CU(cudaMemcpyAsync(dvals.p, vals.data(), vals.size() * 4, cudaMemcpyHostToDevice, c->st));
   k_bin_offsets<<<1, 32, 0, c->st>>>(keys2.p, (long long)np, dvals.p, (int)vals.size(), offs.p);
   TRY(launch_check(c));
+// The different (R, z, zeta) of the LINTON pairs (k_linton_rows).
+static int build_linton_rows(hams_ctx* c) {
+  const long long n = c->bin_off[1];
+  c->lrow.release(true);
+  c->lrep.release(true);
+  c->lin_rows = n;
+  if (n <= 0) return 0;
+  DBuf<unsigned long long> key, key2;
+  DBuf<uint32_t> idx, idx2, rank;
+  DBuf<char> tbuf;
+  size_t t1 = 0, t2 = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, t1, key.p, key2.p, idx.p, idx2.p, (size_t)n, 0, 64, c->st);
+  cub::DeviceScan::InclusiveSum(nullptr, t2, rank.p, rank.p, (size_t)n, c->st);
+  // without the memory for the sort, every pair is its own row
+  if (key.alloc(n) || key2.alloc(n) || idx.alloc(n) || idx2.alloc(n) || rank.alloc(n) ||
+      tbuf.alloc(std::max(t1, t2)) || c->lrow.alloc(n)) {
+    g_err.clear();
+    c->lrow.release();
+    return 0;
+  }
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  k_linton_keys<<<nb, 256, 0, c->st>>>(c->g, c->pairs.p, n, key.p, idx.p);
+  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, t1, key.p, key2.p, idx.p, idx2.p, (size_t)n, 0, 64, c->st));
+  k_linton_heads<<<nb, 256, 0, c->st>>>(c->g, c->pairs.p, idx2.p, n, rank.p);
+  CU(cub::DeviceScan::InclusiveSum(tbuf.p, t2, rank.p, rank.p, (size_t)n, c->st));
+  c->lib_calls += 2;
+  uint32_t rows = 0;
+  CU(cudaMemcpyAsync(&rows, rank.p + n - 1, 4, cudaMemcpyDeviceToHost, c->st));
+  CU(cudaStreamSynchronize(c->st));
+  TRY(c->lrep.alloc(rows));
+  k_linton_file<<<nb, 256, 0, c->st>>>(idx2.p, rank.p, n, c->lrow.p, c->lrep.p);
+  TRY(launch_check(c, 3));
+  CU(cudaStreamSynchronize(c->st));
+  key.release(true);
+  key2.release(true);
+  for (DBuf<uint32_t>* d : {&idx, &idx2, &rank}) d->release(true);
+  tbuf.release(true);
+  c->lin_rows = rows;
+  return 0;
+}
+
   CU(cudaMemcpyAsync(got.data(), offs.p, got.size() * sizeof(long long), cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
   for (int b = 0; b <= kBins; ++b) c->bin_off[b] = got[b];
@@ -1402,6 +1526,7 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
   bst[nb] = off;
   if (off != n) return fail(HAMS_ERR_ARG, "body_nelem sums to %d, nelem is %d", off, n);
   TRY(c->xq.alloc(3 * (size_t)n)); TRY(c->fxyz.alloc(3 * (size_t)tn)); TRY(c->ds.alloc(n)); TRY(c->pnsz.alloc(n));
+  TRY(build_linton_rows(c));
   TRY(c->nrm.alloc(6 * (size_t)n)); TRY(c->vtx.alloc(12 * (size_t)n)); TRY(c->ncn.alloc(n)); TRY(c->body.alloc(n));
   TRY(c->bstart.alloc(nb + 1));
   c->vtx_h = vtx;
@@ -1515,6 +1640,7 @@ static int ctx_frequency_buffers(hams_ctx* c) {
 }
 
 // Streams, library handles and events of destroyed contexts and lanes, per
+  if (c->bin_off[1] > 0) TRY(c->lin_fg.alloc(3 * (size_t)c->lin_rows));
 // device, for the next ones (cuBLAS and cuSOLVER handles are slow to create;
 // the library leaves their settings at the defaults except the stream, which
 // stays bound to the handle's own stream).
@@ -1588,7 +1714,8 @@ static void release_handle_pool() {
 // Stream, library handles and events of a context, on its device.
 static int ctx_handles(hams_ctx* c) {
   if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice(%d) failed", c->dev);
-  if (series_kernels_init()) return fail(HAMS_ERR_CUDA, "series kernels: shared memory size refused");
+  if (c->opts.depth >= 0.0 && series_kernels_init())
+    return fail(HAMS_ERR_CUDA, "series kernels: shared memory size refused");
   if (handles_from_pool(c)) {
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev);
     return 0;
@@ -1648,6 +1775,9 @@ static int make_lane(hams_ctx* c, hams_ctx** out) {
     view_pairs(l, c);
     l->sg_on = c->sg_on;
     l->sg_far = c->sg_far;
+  l->lrow.view(c->lrow);
+  l->lrep.view(c->lrep);
+  l->lin_rows = c->lin_rows;
     l->sg_kmin = c->sg_kmin;
     l->sg_kmax = c->sg_kmax;
     l->sgd = c->sgd;
@@ -1948,16 +2078,19 @@ static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_s
         TRY(series_bin(c, wd, br));
         continue;
       }
-      // few pairs (body blocks): a warp per pair for latency; many: a thread per pair, whose
-      // one wave over the GPU costs less than the warps' redundant lanes
-      const uint32_t* lst = c->pairs.p;
-      if (cnt < (long long)c->sms * kLintonWarpPairsPerSm)
-        k_green_linton<<<(unsigned)((cnt + kLintonWarps - 1) / kLintonWarps), 32 * kLintonWarps, 0, c->st>>>(
-            c->g, wd, c->wvn.p, lst, cnt, c->rs.p, c->rd.p, c->A.p, c->S.p, c->ovf.p);
-      else
-        k_green_linton_threads<<<(unsigned)((cnt + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->mt, lst, cnt,
-                                                                                 c->rs.p, c->rd.p, c->A.p, c->S.p,
-                                                                                 c->ovf.p);
+      const long long rows = c->lin_rows;
+      if (!wd.limit) {
+        if (rows < (long long)c->sms * kLintonRowsPerSm)
+          k_linton_rows<<<(unsigned)rows, 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p, c->lrep.p, c->lin_fg.p,
+                                                           c->ovf.p);
+        else
+          k_linton_rows_threads<<<(unsigned)((rows + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p,
+                                                                                   c->lrep.p, rows, c->lin_fg.p,
+                                                                                   c->ovf.p);
+        TRY(launch_check(c));
+      }
+      k_linton_pairs<<<(unsigned)((cnt + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->pairs.p, c->lrow.p, cnt,
+                                                                       c->lin_fg.p, c->rs.p, c->rd.p, c->A.p, c->S.p);
       TRY(launch_check(c));
     }
     CU(cudaEventRecord(c->evb[4], c->st));
