@@ -791,84 +791,116 @@ __global__ void k_dbc_weights(DevGeom g, WaveDev w, IncWave q, const double* __r
 // ---------------------------------------------------------------------------
 // right-hand sides: chunked reductions over source panels
 // ---------------------------------------------------------------------------
-constexpr int kChunk = 256;  // source panels per chunk (chunks never straddle bodies)
+constexpr int kChunk = 256, kChunkMin = 32;  // source panels per chunk (chunks never straddle bodies)
+constexpr int kHead = 8;                     // headings per pass over S
+// The chunk length: the longest that still gives every SM two blocks of 128
+// rows.  With 256 throughout, one body of 234 panels had two blocks in all
+// (195 us; 14 us now).
+static int chunk_length(int tn, int n, int sms) {
+  int len = kChunk;
+  while (len > kChunkMin && (long long)((tn + 127) / 128) * ((n + len - 1) / len) < 2LL * sms) len /= 2;
+  return len;
+}
 
-// part(c, I, k): k < 6 radiation mode k of the chunk's body, k >= 6 heading k-6.
+// part(c, k, I): k < 6 radiation mode k of the chunk's body, k >= 6 heading k-6.
 // With PROBE the entries of S are replaced by their error probe (the scale
 // of their cell, map and k_probe_scales, times Re S): the right-hand sides of
-// the probe.
+// the probe.  Bound by the read of S and the FP64 pipe: the chunk's normals and diffraction
+// weights are in shared memory, and a thread (a row) has four entries of S in
+// flight (5,400 panels, 4 headings: 220 us against 416 us with the weights read
+// from memory for every entry).
+constexpr int kRhsBatch = 4;
+// Dynamic shared memory of k_rhs_partial for chunks of at most len panels.
+static size_t rhs_smem(int len, int nbeta) { return (size_t)len * (6 * 8 + std::min(nbeta, kHead) * 16); }
 template <bool PROBE>
 __global__ void __launch_bounds__(128) k_rhs_partial(DevGeom g, const double2* __restrict__ S,
                                                      const int2* __restrict__ chunks, const double2* __restrict__ wd,
                                                      int nbeta, double2* __restrict__ part,
                                                      const unsigned char* __restrict__ map = nullptr,
                                                      const double* __restrict__ scale = nullptr) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int c = blockIdx.y;
-  if (i >= g.tn) return;
-  int j0 = chunks[c].x, j1 = chunks[c].y;
-  int nk = 6 + nbeta;
-  double2* out = part + ((size_t)c * g.tn + i) * nk;
+  extern __shared__ __align__(16) double sn[];  // (len, 6), then sw (len, hs): rhs_smem
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+  const int j0 = chunks[c].x, len = chunks[c].y - j0, nk = 6 + nbeta, hs = min(nbeta, kHead);
+  double2* sw = reinterpret_cast<double2*>(sn + 6 * len);
+  const bool live = i < g.tn;
+  double2* out = part + (size_t)c * nk * g.tn + i;
+  const double2* row = S + (size_t)j0 * g.tn + (live ? i : 0);
+  const unsigned char* mrow = PROBE ? map + (size_t)j0 * g.tn + (live ? i : 0) : nullptr;
+  for (int e = threadIdx.x; e < 6 * len; e += blockDim.x)
+    sn[(e % len) * 6 + e / len] = g.nrm[j0 + e % len + (size_t)(e / len) * g.n];
   // one pass over the chunk's entries of S for the radiation sums and the
-  // first 8 headings (each sum in the order of j, as before), one more per
-  // further 8 headings
+  // first 8 headings (each sum in the order of j), one more per further 8
+  // headings
   double rr[6] = {0, 0, 0, 0, 0, 0}, ri[6] = {0, 0, 0, 0, 0, 0};
-  for (int b0 = 0; b0 == 0 || b0 < nbeta; b0 += 8) {
-    double dr[8] = {0, 0, 0, 0, 0, 0, 0, 0}, di[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const int nbb = max(0, min(8, nbeta - b0));
-    for (int j = j0; j < j1; ++j) {
-      double2 s = S[(size_t)i + (size_t)j * g.tn];
-      if (PROBE) {
-        const unsigned char cell = map[(size_t)i + (size_t)j * g.tn];
-        s = make_double2(cell != kNoCell ? scale[2 * cell + 1] * s.x : 0.0, 0.0);
-      }
-      if (b0 == 0) {
+  for (int b0 = 0; b0 == 0 || b0 < nbeta; b0 += kHead) {
+    double dr[kHead] = {0, 0, 0, 0, 0, 0, 0, 0}, di[kHead] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const int nbb = max(0, min(kHead, nbeta - b0));
+    __syncthreads();  // the previous pass has read sw
+    for (int e = threadIdx.x; e < nbb * len; e += blockDim.x)
+      sw[(e % len) * hs + e / len] = wd[j0 + e % len + (size_t)(b0 + e / len) * g.n];
+    __syncthreads();
+    if (live) {
+      for (int q = 0; q < len; q += kRhsBatch) {
+        double2 v[kRhsBatch];
 #pragma unroll
-        for (int m = 0; m < 6; ++m) {
-          double nm = g.nrm[j + (size_t)m * g.n];
-          rr[m] += s.x * nm;
-          ri[m] += s.y * nm;
+        for (int u = 0; u < kRhsBatch; ++u) {
+          const size_t at = (size_t)min(q + u, len - 1) * g.tn;
+          v[u] = row[at];
+          if (PROBE) {
+            const unsigned char cell = mrow[at];
+            v[u] = make_double2(cell != kNoCell ? scale[2 * cell + 1] * v[u].x : 0.0, 0.0);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kRhsBatch; ++u) {
+          if (q + u >= len) break;
+          const double2 s = v[u];
+          if (b0 == 0) {
+            const double2* n2 = reinterpret_cast<const double2*>(sn + (q + u) * 6);
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+              const double2 nm = n2[m];
+              rr[2 * m] += s.x * nm.x;
+              ri[2 * m] += s.y * nm.x;
+              rr[2 * m + 1] += s.x * nm.y;
+              ri[2 * m + 1] += s.y * nm.y;
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < kHead; ++b)
+            if (b < nbb) {
+              const double2 wv = sw[(q + u) * hs + b];
+              dr[b] -= s.x * wv.x - s.y * wv.y;  // (as one chain of two FMAs: 327 us)
+              di[b] -= s.x * wv.y + s.y * wv.x;
+            }
         }
       }
-#pragma unroll
-      for (int b = 0; b < 8; ++b)
-        if (b < nbb) {
-          double2 wv = wd[j + (size_t)(b0 + b) * g.n];
-          dr[b] -= s.x * wv.x - s.y * wv.y;
-          di[b] -= s.x * wv.y + s.y * wv.x;
-        }
+      if (b0 == 0)
+        for (int m = 0; m < 6; ++m) out[(size_t)m * g.tn] = make_double2(rr[m], ri[m]);
+      for (int b = 0; b < nbb; ++b) out[(size_t)(6 + b0 + b) * g.tn] = make_double2(dr[b], di[b]);
     }
-    if (b0 == 0)
-      for (int m = 0; m < 6; ++m) out[m] = make_double2(rr[m], ri[m]);
-    for (int b = 0; b < nbb; ++b) out[6 + b0 + b] = make_double2(dr[b], di[b]);
   }
 }
 
-// B (tn, 6nb + nbeta): radiation columns of body b, then diffraction columns.
-__global__ void k_rhs_final(int tn, int nb, int nchunks, const int* __restrict__ chunk_body,
-                            const double2* __restrict__ part, int nbeta, double2* __restrict__ B) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+// B (tn, 6nb + nbeta): radiation columns of body b (the sums of its chunks
+// bchunk[b] .. bchunk[b+1] - 1), then diffraction columns (all chunks); one
+// column per blockIdx.y.
+__global__ void __launch_bounds__(128) k_rhs_final(int tn, int nb, int nchunks, const int* __restrict__ bchunk,
+                                                   const double2* __restrict__ part, int nbeta,
+                                                   double2* __restrict__ B) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, col = blockIdx.y, nk = 6 + nbeta;
   if (i >= tn) return;
-  int nk = 6 + nbeta, ldb = tn;
-  for (int b = 0; b < nb; ++b)
-    for (int m = 0; m < 6; ++m) B[i + (size_t)(6 * b + m) * ldb] = make_double2(0.0, 0.0);
-  for (int c = 0; c < nchunks; ++c) {
-    const double2* p = part + ((size_t)c * tn + i) * nk;
-    int b = chunk_body[c];
-    for (int m = 0; m < 6; ++m) {
-      double2 v = B[i + (size_t)(6 * b + m) * ldb];
-      B[i + (size_t)(6 * b + m) * ldb] = make_double2(v.x + p[m].x, v.y + p[m].y);
-    }
+  const bool rad = col < 6 * nb;
+  const int b = col / 6, k = rad ? col - 6 * b : col - 6 * nb + 6;
+  const int c0 = rad ? bchunk[b] : 0, c1 = rad ? bchunk[b + 1] : nchunks;
+  double sr = 0.0, si = 0.0;
+#pragma unroll 4
+  for (int c = c0; c < c1; ++c) {
+    const double2 p = part[((size_t)c * nk + k) * tn + i];
+    sr += p.x;
+    si += p.y;
   }
-  for (int k = 0; k < nbeta; ++k) {
-    double sr = 0.0, si = 0.0;
-    for (int c = 0; c < nchunks; ++c) {
-      const double2* p = part + ((size_t)c * tn + i) * nk;
-      sr += p[6 + k].x;
-      si += p[6 + k].y;
-    }
-    B[i + (size_t)(6 * nb + k) * ldb] = make_double2(sr, si);
-  }
+  B[i + (size_t)col * tn] = make_double2(sr, si);
 }
 
 // ---------------------------------------------------------------------------
@@ -1175,6 +1207,11 @@ struct hams_ctx {
   DBuf<uint32_t> rid;
   DBuf<double> ur;
   uint32_t rad_base[4] = {}, rad_n[4] = {};
+  // LINTON rows: the row of every pair of bin 0 and a pair of each row (none:
+  // a row per pair), this frequency's rows
+  DBuf<uint32_t> lrow, lrep;
+  long long lin_rows = 0;
+  DBuf<double2> lin_fg;
   // positions where the series of bins 1, 2 and 4 get longer than the two
   // lengths of kNtCut (launch_series)
   long long nt_cut[kBins][2] = {};
@@ -1186,8 +1223,9 @@ struct hams_ctx {
   long long blk_pairs = 0;
   // chunks of source panels for the RHS reduction
   std::vector<int2> chunks_h;
+  int chunk_len = 0;  // of the longest chunk
   DBuf<int2> chunks;
-  DBuf<int> chunk_body;
+  DBuf<int> bchunk;  // each body's first chunk, and the end
   // per-frequency buffers
   DBuf<double2> A, S, B, part, wd, C, D, X, R;
   DBuf<float2> Af, Xf, luw;
@@ -1207,11 +1245,6 @@ struct hams_ctx {
   DBuf<int> ipiv, info, ovf;
   DBuf<char> work;
   DBuf<char> work32;
-  // LINTON rows: the row of every pair of bin 0 and a pair of each row (none:
-  // a row per pair), this frequency's rows
-  DBuf<uint32_t> lrow, lrep;
-  long long lin_rows = 0;
-  DBuf<double2> lin_fg;
   // timing: ev[0..5] stage marks, evb[0..4] branch marks, evf after the factorisation
   cudaEvent_t ev[6] = {};
   cudaEvent_t evb[6] = {};
@@ -1307,7 +1340,7 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
   auto rel = [](auto&... b) { (b.release(true), ...); };
   rel(c->fp_x, c->fp_sld, c->fp_S, c->fp_D, c->fp_bc, c->fp_pot, c->fp_out, c->hxp, c->hyp, c->hw);
   rel(c->xq, c->fxyz, c->ds, c->pnsz, c->nrm, c->vtx, c->ncn, c->body, c->bstart, c->rs, c->rd, c->pairs);
-  rel(c->blk_copied, c->blk_list, c->chunks, c->chunk_body, c->A, c->S, c->B, c->part, c->wd, c->C, c->D, c->X, c->R);
+  rel(c->blk_copied, c->blk_list, c->chunks, c->bchunk, c->A, c->S, c->B, c->part, c->wd, c->C, c->D, c->X, c->R);
   rel(c->Af, c->Xf, c->luw, c->gv, c->gw, c->gz, c->gy, c->gpre, c->gnrm, c->gpiv, c->perm);
   rel(c->wvn, c->beta, c->outbuf, c->colratio, c->mt_pm, c->mt_ac, c->mt_fld, c->mt_fldt, c->mt_src, c->mt_srct);
   rel(c->ipiv, c->info, c->ovf, c->work, c->work32, c->sg_wh, c->sg_w0, c->sg_bias, c->sg_samp, c->sg_g1, c->sg_g2);
@@ -1409,39 +1442,6 @@ static int build_distances(hams_ctx* c) {
   return 0;
 }
 
-// Sorted pair list and bin offsets (finite depth); rebuilt when the surrogate
-// is switched on or off.
-static int build_pairs(hams_ctx* c) {
-  const int n = c->n, tn = c->tn;
-  size_t np = (size_t)tn * n;
-  if (np > 0xffffffffull) return fail(HAMS_ERR_UNSUPPORTED, "%zu pairs exceed the 32-bit pair index", np);
-  DBuf<uint32_t> keys, keys2, idx;
-  TRY(keys.alloc(np)); TRY(keys2.alloc(np)); TRY(idx.alloc(np)); TRY(c->pairs.alloc(np));
-  dim3 grid2((tn + 127) / 128, n);
-  k_pair_keys<<<grid2, 128, 0, c->st>>>(c->g, c->opts.depth, c->sg_on, c->sg_far, c->nblk ? c->blk_copied.p : nullptr,
-                                         keys.p, idx.p);
-  TRY(launch_check(c));
-  size_t tmp = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, tmp, keys.p, keys2.p, idx.p, c->pairs.p, np, 0, 11, c->st);
-  DBuf<char> tbuf;
-  TRY(tbuf.alloc(tmp));
-  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, tmp, keys.p, keys2.p, idx.p, c->pairs.p, np, 0, 11, c->st));
-  c->lib_calls += 1;
-  // bin boundaries, and where the series of bins 1, 2 and 4 pass kNtCut:
-  // first index of each key in the sorted keys, found on the device (a binary
-  // search each) so that only these numbers come back
-  std::vector<uint32_t> vals;
-  for (int b = 0; b <= kBins; ++b) vals.push_back((uint32_t)b << 8);
-  for (int b : {1, 2, 4})
-    for (int q = 0; q < 2; ++q) vals.push_back(((uint32_t)b << 8) + kNtCut[b == 1][q] + 1);
-  DBuf<long long> offs;
-  DBuf<uint32_t> dvals;
-  TRY(offs.alloc(vals.size()));
-  TRY(dvals.alloc(vals.size()));
-  std::vector<long long> got(vals.size());
-  CU(cudaMemcpyAsync(dvals.p, vals.data(), vals.size() * 4, cudaMemcpyHostToDevice, c->st));
-  k_bin_offsets<<<1, 32, 0, c->st>>>(keys2.p, (long long)np, dvals.p, (int)vals.size(), offs.p);
-  TRY(launch_check(c));
 // The different (R, z, zeta) of the LINTON pairs (k_linton_rows).
 static int build_linton_rows(hams_ctx* c) {
   const long long n = c->bin_off[1];
@@ -1483,6 +1483,39 @@ static int build_linton_rows(hams_ctx* c) {
   return 0;
 }
 
+// Sorted pair list and bin offsets (finite depth); rebuilt when the surrogate
+// is switched on or off.
+static int build_pairs(hams_ctx* c) {
+  const int n = c->n, tn = c->tn;
+  size_t np = (size_t)tn * n;
+  if (np > 0xffffffffull) return fail(HAMS_ERR_UNSUPPORTED, "%zu pairs exceed the 32-bit pair index", np);
+  DBuf<uint32_t> keys, keys2, idx;
+  TRY(keys.alloc(np)); TRY(keys2.alloc(np)); TRY(idx.alloc(np)); TRY(c->pairs.alloc(np));
+  dim3 grid2((tn + 127) / 128, n);
+  k_pair_keys<<<grid2, 128, 0, c->st>>>(c->g, c->opts.depth, c->sg_on, c->sg_far, c->nblk ? c->blk_copied.p : nullptr,
+                                         keys.p, idx.p);
+  TRY(launch_check(c));
+  size_t tmp = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tmp, keys.p, keys2.p, idx.p, c->pairs.p, np, 0, 11, c->st);
+  DBuf<char> tbuf;
+  TRY(tbuf.alloc(tmp));
+  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, tmp, keys.p, keys2.p, idx.p, c->pairs.p, np, 0, 11, c->st));
+  c->lib_calls += 1;
+  // bin boundaries, and where the series of bins 1, 2 and 4 pass kNtCut:
+  // first index of each key in the sorted keys, found on the device (a binary
+  // search each) so that only these numbers come back
+  std::vector<uint32_t> vals;
+  for (int b = 0; b <= kBins; ++b) vals.push_back((uint32_t)b << 8);
+  for (int b : {1, 2, 4})
+    for (int q = 0; q < 2; ++q) vals.push_back(((uint32_t)b << 8) + kNtCut[b == 1][q] + 1);
+  DBuf<long long> offs;
+  DBuf<uint32_t> dvals;
+  TRY(offs.alloc(vals.size()));
+  TRY(dvals.alloc(vals.size()));
+  std::vector<long long> got(vals.size());
+  CU(cudaMemcpyAsync(dvals.p, vals.data(), vals.size() * 4, cudaMemcpyHostToDevice, c->st));
+  k_bin_offsets<<<1, 32, 0, c->st>>>(keys2.p, (long long)np, dvals.p, (int)vals.size(), offs.p);
+  TRY(launch_check(c));
   CU(cudaMemcpyAsync(got.data(), offs.p, got.size() * sizeof(long long), cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
   for (int b = 0; b <= kBins; ++b) c->bin_off[b] = got[b];
@@ -1493,6 +1526,7 @@ static int build_linton_rows(hams_ctx* c) {
   keys2.release(true);
   idx.release(true);
   tbuf.release(true);
+  TRY(build_linton_rows(c));
   return build_distances(c);
 }
 
@@ -1526,7 +1560,6 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
   bst[nb] = off;
   if (off != n) return fail(HAMS_ERR_ARG, "body_nelem sums to %d, nelem is %d", off, n);
   TRY(c->xq.alloc(3 * (size_t)n)); TRY(c->fxyz.alloc(3 * (size_t)tn)); TRY(c->ds.alloc(n)); TRY(c->pnsz.alloc(n));
-  TRY(build_linton_rows(c));
   TRY(c->nrm.alloc(6 * (size_t)n)); TRY(c->vtx.alloc(12 * (size_t)n)); TRY(c->ncn.alloc(n)); TRY(c->body.alloc(n));
   TRY(c->bstart.alloc(nb + 1));
   c->vtx_h = vtx;
@@ -1589,16 +1622,17 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
 
   // chunks of source panels for the RHS reduction
   c->chunks_h.clear();
-  std::vector<int> cb;
-  for (int b = 0; b < nb; ++b)
-    for (int j = bst[b]; j < bst[b + 1]; j += kChunk) {
-      c->chunks_h.push_back(make_int2(j, std::min(j + kChunk, bst[b + 1])));
-      cb.push_back(b);
-    }
+  std::vector<int> cb;  // each body's first chunk
+  const int clen = c->chunk_len = chunk_length(tn, n, c->sms);
+  for (int b = 0; b < nb; ++b) {
+    cb.push_back((int)c->chunks_h.size());
+    for (int j = bst[b]; j < bst[b + 1]; j += clen) c->chunks_h.push_back(make_int2(j, std::min(j + clen, bst[b + 1])));
+  }
+  cb.push_back((int)c->chunks_h.size());
   TRY(c->chunks.alloc(c->chunks_h.size()));
-  TRY(c->chunk_body.alloc(cb.size()));
+  TRY(c->bchunk.alloc(cb.size()));
   CU(cudaMemcpyAsync(c->chunks.p, c->chunks_h.data(), c->chunks_h.size() * sizeof(int2), cudaMemcpyHostToDevice, c->st));
-  CU(cudaMemcpyAsync(c->chunk_body.p, cb.data(), cb.size() * sizeof(int), cudaMemcpyHostToDevice, c->st));
+  CU(cudaMemcpyAsync(c->bchunk.p, cb.data(), cb.size() * sizeof(int), cudaMemcpyHostToDevice, c->st));
 
   TRY(ctx_frequency_buffers(c));
   CU(cudaStreamSynchronize(c->st));
@@ -1606,6 +1640,7 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
 }
 
 static int rad_buffers(hams_ctx* c) {
+  if (c->bin_off[1] > 0) TRY(c->lin_fg.alloc(3 * (size_t)c->lin_rows));
   for (int br = 1; br < 4; ++br)
     if (c->rad_n[br]) {
       TRY(c->rad_k[br].alloc((size_t)c->rad_n[br] * rad_stride(br)));
@@ -1640,7 +1675,6 @@ static int ctx_frequency_buffers(hams_ctx* c) {
 }
 
 // Streams, library handles and events of destroyed contexts and lanes, per
-  if (c->bin_off[1] > 0) TRY(c->lin_fg.alloc(3 * (size_t)c->lin_rows));
 // device, for the next ones (cuBLAS and cuSOLVER handles are slow to create;
 // the library leaves their settings at the defaults except the stream, which
 // stays bound to the handle's own stream).
@@ -1741,6 +1775,9 @@ static void view_pairs(hams_ctx* l, hams_ctx* c) {
   l->pairs.view(c->pairs);
   l->rid.view(c->rid);
   l->ur.view(c->ur);
+  l->lrow.view(c->lrow);
+  l->lrep.view(c->lrep);
+  l->lin_rows = c->lin_rows;
   for (int br = 0; br < 4; ++br) l->rad_base[br] = c->rad_base[br], l->rad_n[br] = c->rad_n[br];
   for (int b = 0; b < kBins; ++b) l->nt_cut[b][0] = c->nt_cut[b][0], l->nt_cut[b][1] = c->nt_cut[b][1];
 }
@@ -1768,16 +1805,13 @@ static int make_lane(hams_ctx* c, hams_ctx** out) {
     l->xq.view(c->xq); l->fxyz.view(c->fxyz); l->ds.view(c->ds); l->pnsz.view(c->pnsz); l->nrm.view(c->nrm);
     l->vtx.view(c->vtx); l->ncn.view(c->ncn); l->body.view(c->body); l->bstart.view(c->bstart);
     l->rs.view(c->rs); l->rd.view(c->rd); l->chunks.view(c->chunks);
-    l->chunk_body.view(c->chunk_body);
+    l->bchunk.view(c->bchunk);
     l->blk_copied.view(c->blk_copied); l->blk_list.view(c->blk_list);
     l->nblk = c->nblk; l->blk_rows = c->blk_rows; l->blk_cols = c->blk_cols; l->blk_pairs = c->blk_pairs;
     l->g = c->g;
     view_pairs(l, c);
     l->sg_on = c->sg_on;
     l->sg_far = c->sg_far;
-  l->lrow.view(c->lrow);
-  l->lrep.view(c->lrep);
-  l->lin_rows = c->lin_rows;
     l->sg_kmin = c->sg_kmin;
     l->sg_kmax = c->sg_kmax;
     l->sgd = c->sgd;
@@ -1788,6 +1822,7 @@ static int make_lane(hams_ctx* c, hams_ctx** out) {
     l->sg_ns5 = c->sg_ns5;
     l->sms = c->sms;
     l->chunks_h = c->chunks_h;
+    l->chunk_len = c->chunk_len;
     rc = ctx_frequency_buffers(l);
   }
   if (rc < 0) {
@@ -2044,8 +2079,10 @@ static int copy_blocks_and_rhs(hams_ctx* c, int nbeta) {
     TRY(launch_check(c));
   }
   const int nch = (int)c->chunks_h.size();
-  k_rhs_partial<false><<<dim3((tn + 127) / 128, nch), 128, 0, c->st>>>(c->g, c->S.p, c->chunks.p, c->wd.p, nbeta, c->part.p);
-  k_rhs_final<<<(tn + 127) / 128, 128, 0, c->st>>>(tn, nb, nch, c->chunk_body.p, c->part.p, nbeta, c->B.p);
+  k_rhs_partial<false><<<dim3((tn + 127) / 128, nch), 128, rhs_smem(c->chunk_len, nbeta), c->st>>>(
+      c->g, c->S.p, c->chunks.p, c->wd.p, nbeta, c->part.p);
+  k_rhs_final<<<dim3((tn + 127) / 128, 6 * nb + nbeta), 128, 0, c->st>>>(
+      tn, nb, nch, c->bchunk.p, c->part.p, nbeta, c->B.p);
   return launch_check(c, 2);
 }
 
@@ -2147,9 +2184,11 @@ static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_s
     k_dbc_weights<<<dim3((n + 127) / 128, nbeta), 128, 0, c->st>>>(c->g, wd, q, c->beta.p, nbeta, c->wd.p);
     TRY(launch_check(c));
   }
-  k_rhs_partial<false><<<dim3((tn + 127) / 128, nch), 128, 0, c->st>>>(c->g, c->S.p, c->chunks.p, c->wd.p, nbeta, c->part.p);
+  k_rhs_partial<false><<<dim3((tn + 127) / 128, nch), 128, rhs_smem(c->chunk_len, nbeta), c->st>>>(
+      c->g, c->S.p, c->chunks.p, c->wd.p, nbeta, c->part.p);
   TRY(launch_check(c));
-  k_rhs_final<<<(tn + 127) / 128, 128, 0, c->st>>>(tn, nb, nch, c->chunk_body.p, c->part.p, nbeta, c->B.p);
+  k_rhs_final<<<dim3((tn + 127) / 128, 6 * nb + nbeta), 128, 0, c->st>>>(
+      tn, nb, nch, c->bchunk.p, c->part.p, nbeta, c->B.p);
   TRY(launch_check(c));
   CU(cudaEventRecord(c->ev[2], c->st));
   return 0;
@@ -2728,9 +2767,11 @@ static int judge_rhs(hams_ctx* c, int nbeta, const double2* X, double2* out, flo
   k_probe_scales<<<1, 256, 0, c->st>>>(c->sg_cells.p, c->sg_scale.p);
   // dB: the right-hand sides of the probe of S (this frequency's diffraction weights are still in wd)
   const int nch = (int)c->chunks_h.size();
-  k_rhs_partial<true><<<dim3((tn + 127) / 128, nch), 128, 0, c->st>>>(c->g, c->S.p, c->chunks.p, c->wd.p, nbeta,
+  k_rhs_partial<true><<<dim3((tn + 127) / 128, nch), 128, rhs_smem(c->chunk_len, nbeta), c->st>>>(
+      c->g, c->S.p, c->chunks.p, c->wd.p, nbeta,
                                                                       c->part.p, c->sg_map.p, c->sg_scale.p);
-  k_rhs_final<<<(tn + 127) / 128, 128, 0, c->st>>>(tn, nb, nch, c->chunk_body.p, c->part.p, nbeta, out);
+  k_rhs_final<<<dim3((tn + 127) / 128, 6 * nb + nbeta), 128, 0, c->st>>>(
+      tn, nb, nch, c->bchunk.p, c->part.p, nbeta, out);
   // out = dB - dA X, X rounded to complex64 in xs
   const size_t nx = (size_t)n * nrhs;
   k_z2c<<<592, 256, 0, c->st>>>(X, xs, nx);
