@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kSerThreads, 5) k_green_series(DevGeom g, Wave
     if constexpr (!IO::kPoints) {
       double are = io.rd[p] + ds * (gx.re * n1 + gy.re * n2 + gz.x * n3);
       const double aim = ds * (gx.im * n1 + gy.im * n2 + gz.y * n3);
-      if (i == j) are += 2.0 * 3.141592653589793;
+      if (g.diag && i == j) are += 2.0 * 3.141592653589793;
       io.A[p] = make_double2(are, aim);
     }
   }
@@ -431,7 +431,7 @@ __global__ void k_mode_tables(DevGeom g, WaveDev w, const double* __restrict__ w
 
 void launch_mode_tables(cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, int nmode, double* pm, double* ac,
                         double2* src, double2* srct, double* fld, double* fldt) {
-  dim3 grid((g.tn + 127) / 128, nmode - 1);
+  dim3 grid((max(g.n, g.tn) + 127) / 128, nmode - 1);
   k_mode_tables<<<grid, 128, 0, st>>>(g, w, wvn, nmode, pm, ac, src, srct, fld, fldt);
 }
 
@@ -565,7 +565,8 @@ void launch_point_series(int br, int ntmax, cudaStream_t st, int npts, const dou
 }
 
 // Source (S) and normal-dipole (D) influence of every hull panel J at field
-// point f, the terms CalPotentialMulti sums (PressureElevationMulti.f90:81-137):
+// point f without pair lists (sets of more than 2^32 - 1 pairs, or no memory
+// for the lists), the terms CalPotentialMulti sums (PressureElevationMulti.f90:81-137):
 // S = FLAG*SIJ + G ds, D = (FLAG*DIJ + grad G ds) . n_J, with the Rankine
 // integrals at the field point (SGLINTBD_MULTI_QUAD2/TRI2,
 // SingularIntgrMulti.f90:454-776) and FLAG = (distance <= 50 PNSZ_J).

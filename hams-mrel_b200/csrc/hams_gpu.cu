@@ -597,8 +597,9 @@ __global__ void __launch_bounds__(128) k_linton_pairs(DevGeom g, WaveDev w, cons
   store_pair(g, p, q.i, q.j, G, rs, rd, A, S);
 }
 
-// A 64-bit hash of a LINTON pair's (R, z, zeta); equal triples are neighbours
-// once sorted by it.
+// A hash of a LINTON pair's (R, z, zeta); equal triples are neighbours once
+// sorted by its lower half (unless others share it: then a triple may get
+// more than one row).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
   x ^= x >> 30;
   x *= 0xbf58476d1ce4e5b9ull;
@@ -1184,6 +1185,9 @@ struct hams_ctx {
   int nfp = 0;
   DBuf<double> fp_x, fp_sld;
   DBuf<double2> fp_S, fp_D, fp_bc, fp_pot, fp_out;
+  // the points' pair set: a context whose field points are fp_x, with this
+  // one's sources and stream (field_context); A and S hold the influences
+  hams_ctx* field = nullptr;
   std::vector<double> fp_last;
   std::vector<std::vector<double>> fp_batch;
   bool hm_ready = false;      // GMRES: cluster tree uploaded to hm
@@ -1308,6 +1312,7 @@ extern "C" const char* hams_last_error(void) { return g_err.c_str(); }
 // error reporting for the other translation units of the library
 int hams_set_error(int code, const char* msg) { return fail(code, "%s", msg); }
 
+static void field_free(hams_ctx* f);
 static bool handles_to_pool(hams_ctx* c);
 static void release_handle_pool();
 
@@ -1339,7 +1344,10 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
   // the context's stream is idle: its buffers go back to the cache without a device-wide wait
   auto rel = [](auto&... b) { (b.release(true), ...); };
   rel(c->fp_x, c->fp_sld, c->fp_S, c->fp_D, c->fp_bc, c->fp_pot, c->fp_out, c->hxp, c->hyp, c->hw);
+  field_free(c->field);
   rel(c->xq, c->fxyz, c->ds, c->pnsz, c->nrm, c->vtx, c->ncn, c->body, c->bstart, c->rs, c->rd, c->pairs);
+  rel(c->rid, c->ur, c->lrow, c->lrep, c->lin_fg);
+  for (int br = 0; br < 4; ++br) rel(c->rad_k[br], c->rad_j[br]);
   rel(c->blk_copied, c->blk_list, c->chunks, c->bchunk, c->A, c->S, c->B, c->part, c->wd, c->C, c->D, c->X, c->R);
   rel(c->Af, c->Xf, c->luw, c->gv, c->gw, c->gz, c->gy, c->gpre, c->gnrm, c->gpiv, c->perm);
   rel(c->wvn, c->beta, c->outbuf, c->colratio, c->mt_pm, c->mt_ac, c->mt_fld, c->mt_fldt, c->mt_src, c->mt_srct);
@@ -1363,6 +1371,7 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
 }
 
 static int ctx_frequency_buffers(hams_ctx* c);
+static int field_context(hams_ctx* c, hams_ctx* of);
 
 // Series lengths (EIGENE, then PIDCOCK) at which a bin's launch is split, so
 // that its shared memory fits the lengths it holds (launch_series).
@@ -1453,7 +1462,7 @@ static int build_linton_rows(hams_ctx* c) {
   DBuf<uint32_t> idx, idx2, rank;
   DBuf<char> tbuf;
   size_t t1 = 0, t2 = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, t1, key.p, key2.p, idx.p, idx2.p, (size_t)n, 0, 64, c->st);
+  cub::DeviceRadixSort::SortPairs(nullptr, t1, key.p, key2.p, idx.p, idx2.p, (size_t)n, 0, 32, c->st);
   cub::DeviceScan::InclusiveSum(nullptr, t2, rank.p, rank.p, (size_t)n, c->st);
   // without the memory for the sort, every pair is its own row
   if (key.alloc(n) || key2.alloc(n) || idx.alloc(n) || idx2.alloc(n) || rank.alloc(n) ||
@@ -1464,7 +1473,7 @@ static int build_linton_rows(hams_ctx* c) {
   }
   const unsigned nb = (unsigned)((n + 255) / 256);
   k_linton_keys<<<nb, 256, 0, c->st>>>(c->g, c->pairs.p, n, key.p, idx.p);
-  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, t1, key.p, key2.p, idx.p, idx2.p, (size_t)n, 0, 64, c->st));
+  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, t1, key.p, key2.p, idx.p, idx2.p, (size_t)n, 0, 32, c->st));
   k_linton_heads<<<nb, 256, 0, c->st>>>(c->g, c->pairs.p, idx2.p, n, rank.p);
   CU(cub::DeviceScan::InclusiveSum(tbuf.p, t2, rank.p, rank.p, (size_t)n, c->st));
   c->lib_calls += 2;
@@ -1575,7 +1584,8 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
   CU(cudaMemcpyAsync(c->ncn.p, geo->ncn, (size_t)n * 4, cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync(c->body.p, body.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync(c->bstart.p, bst.data(), (size_t)(nb + 1) * 4, cudaMemcpyHostToDevice, c->st));
-  c->g = DevGeom{n, tn, nb, c->xq.p, c->fxyz.p, c->ds.p, c->pnsz.p, c->nrm.p, c->vtx.p, c->ncn.p, c->body.p, c->bstart.p};
+  c->g = DevGeom{n, tn, nb, c->xq.p, c->fxyz.p, c->ds.p, c->pnsz.p, c->nrm.p, c->vtx.p, c->ncn.p, c->body.p,
+                 c->bstart.p, 1};
 
   // Rankine tables
   size_t np = (size_t)tn * n;
@@ -1649,22 +1659,27 @@ static int rad_buffers(hams_ctx* c) {
   return 0;
 }
 
+// Mode and radial tables and LINTON rows of one frequency in flight.
+static int mode_buffers(hams_ctx* c) {
+  const int n = c->n, tn = c->tn;
+  const size_t km = hams::kModeMax;
+  TRY(c->mt_pm.alloc(km)); TRY(c->mt_ac.alloc(km));
+  TRY(c->mt_src.alloc(km * n)); TRY(c->mt_srct.alloc(km * n));
+  TRY(c->mt_fld.alloc(km * tn)); TRY(c->mt_fldt.alloc(km * tn));
+  // modes needed by the longest series present: PIDCOCK 99, EIGENE 50, EIGEN 10
+  int nmode = 11;
+  if (c->bin_off[3] > c->bin_off[2] || c->bin_off[5] > c->bin_off[4]) nmode = hams::kEigenEMax + 1;
+  if (c->bin_off[2] > c->bin_off[1]) nmode = hams::kPidcockMax + 1;
+  TRY(rad_buffers(c));
+  c->mt = hams::ModeTab{n, tn, nmode, c->mt_pm.p, c->mt_ac.p, c->mt_src.p, c->mt_srct.p, c->mt_fld.p, c->mt_fldt.p};
+  return 0;
+}
+
 // Buffers of one frequency in flight: mode tables, A and S, roots, flags.
 static int ctx_frequency_buffers(hams_ctx* c) {
   const int n = c->n, tn = c->tn;
   size_t np = (size_t)tn * n;
-  if (c->opts.depth >= 0.0) {
-    const size_t km = hams::kModeMax;
-    TRY(c->mt_pm.alloc(km)); TRY(c->mt_ac.alloc(km));
-    TRY(c->mt_src.alloc(km * n)); TRY(c->mt_srct.alloc(km * n));
-    TRY(c->mt_fld.alloc(km * tn)); TRY(c->mt_fldt.alloc(km * tn));
-    // modes needed by the longest series present: PIDCOCK 99, EIGENE 50, EIGEN 10
-    int nmode = 11;
-    if (c->bin_off[3] > c->bin_off[2] || c->bin_off[5] > c->bin_off[4]) nmode = hams::kEigenEMax + 1;
-    if (c->bin_off[2] > c->bin_off[1]) nmode = hams::kPidcockMax + 1;
-    TRY(rad_buffers(c));
-    c->mt = hams::ModeTab{n, tn, nmode, c->mt_pm.p, c->mt_ac.p, c->mt_src.p, c->mt_srct.p, c->mt_fld.p, c->mt_fldt.p};
-  }
+  if (c->opts.depth >= 0.0) TRY(mode_buffers(c));
   TRY(c->A.alloc(np));
   TRY(c->S.alloc(np));
   TRY(c->wvn.alloc(HAMS_NK));
@@ -1824,6 +1839,7 @@ static int make_lane(hams_ctx* c, hams_ctx** out) {
     l->chunks_h = c->chunks_h;
     l->chunk_len = c->chunk_len;
     rc = ctx_frequency_buffers(l);
+    if (!rc && c->field) rc = field_context(l, c->field);
   }
   if (rc < 0) {
     std::string keep = g_err;
@@ -2061,6 +2077,26 @@ static int series_bin(hams_ctx* c, const WaveDev& wd, int b) {
                       b);
 }
 
+// The LINTON pairs (bin 0): their rows, then A and S.
+static int linton_bin(hams_ctx* c, const WaveDev& wd) {
+  const long long cnt = c->bin_off[1];
+  if (cnt <= 0) return 0;
+  const long long rows = c->lin_rows;
+  if (!wd.limit) {
+    if (rows < (long long)c->sms * kLintonRowsPerSm)
+      k_linton_rows<<<(unsigned)rows, 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p, c->lrep.p, c->lin_fg.p,
+                                                       c->ovf.p);
+    else
+      k_linton_rows_threads<<<(unsigned)((rows + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p,
+                                                                               c->lrep.p, rows, c->lin_fg.p,
+                                                                               c->ovf.p);
+    TRY(launch_check(c));
+  }
+  k_linton_pairs<<<(unsigned)((cnt + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->pairs.p, c->lrow.p, cnt,
+                                                                   c->lin_fg.p, c->rs.p, c->rd.p, c->A.p, c->S.p);
+  return launch_check(c);
+}
+
 // The far pairs (bins 4 and 5 of k_pair_keys) from the series: EIGENE and
 // EIGEN, as their own bins would (FinGreen3D.f90:413-660).
 static int far_series(hams_ctx* c, const WaveDev& wd) {
@@ -2111,24 +2147,7 @@ static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_s
       long long cnt = c->bin_off[br + 1] - c->bin_off[br];
       CU(cudaEventRecord(c->evb[br], c->st));
       if (cnt <= 0) continue;
-      if (br > 0) {
-        TRY(series_bin(c, wd, br));
-        continue;
-      }
-      const long long rows = c->lin_rows;
-      if (!wd.limit) {
-        if (rows < (long long)c->sms * kLintonRowsPerSm)
-          k_linton_rows<<<(unsigned)rows, 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p, c->lrep.p, c->lin_fg.p,
-                                                           c->ovf.p);
-        else
-          k_linton_rows_threads<<<(unsigned)((rows + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p,
-                                                                                   c->lrep.p, rows, c->lin_fg.p,
-                                                                                   c->ovf.p);
-        TRY(launch_check(c));
-      }
-      k_linton_pairs<<<(unsigned)((cnt + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->pairs.p, c->lrow.p, cnt,
-                                                                       c->lin_fg.p, c->rs.p, c->rd.p, c->A.p, c->S.p);
-      TRY(launch_check(c));
+      TRY(br > 0 ? series_bin(c, wd, br) : linton_bin(c, wd));
     }
     CU(cudaEventRecord(c->evb[4], c->st));
     // far pairs: the surrogate, or the series when this frequency is outside its domain
@@ -2707,9 +2726,94 @@ static int forces_dev(hams_ctx* c, const hams_wave* w, int nbeta) {
   return launch_check(c);
 }
 
+// The pair set of field points: the influence of every hull panel at the nfp
+// points fp_x takes the same branches, tables and kernels as the panel pairs
+// (100 points of a 2,340-panel array, two frequencies in flight: 1.1 ms with
+// the potentials' products, against 8.1 ms with k_field_pairs, a thread per
+// pair whatever its branch).  of: another context's pair set to share (a batch
+// lane's), or null to build it.
+static void field_free(hams_ctx* f) {
+  if (!f) return;
+  auto rel = [](auto&... b) { (b.release(true), ...); };
+  rel(f->rs, f->rd, f->pairs, f->rid, f->ur, f->lrow, f->lrep, f->lin_fg, f->A, f->S, f->wvn, f->ovf);
+  rel(f->mt_pm, f->mt_ac, f->mt_fld, f->mt_fldt, f->mt_src, f->mt_srct);
+  for (int br = 0; br < 4; ++br) rel(f->rad_k[br], f->rad_j[br]);
+  delete f;
+}
+static int field_setup(hams_ctx* f, hams_ctx* of) {
+  const size_t np = (size_t)f->tn * f->n;
+  if (of) {
+    f->rs.view(of->rs);
+    f->rd.view(of->rd);
+    view_pairs(f, of);
+  } else {
+    TRY(f->rs.alloc(np));
+    TRY(f->rd.alloc(np));
+    k_rankine<<<dim3((f->tn + 127) / 128, f->n), 128, 0, f->st>>>(f->g, f->rs.p, f->rd.p);
+    TRY(launch_check(f));
+    if (f->opts.depth >= 0.0) TRY(build_pairs(f));
+  }
+  if (f->opts.depth >= 0.0) TRY(mode_buffers(f));
+  TRY(f->A.alloc(np));
+  return f->S.alloc(np);
+}
+// c's pair set for its field points; the caller's stream c->st is idle.  Left
+// out (k_field_pairs takes over) where the pairs exceed the 32-bit index or
+// memory runs out.
+static int field_context(hams_ctx* c, hams_ctx* of) {
+  field_free(c->field);
+  c->field = nullptr;
+  if (c->nfp <= 0 || (size_t)c->nfp * c->n > 0xffffffffull) return 0;
+  hams_ctx* f = new hams_ctx();
+  f->is_lane = true;
+  f->opts = c->opts;
+  f->dev = c->dev;
+  f->st = c->st;
+  f->sms = c->sms;
+  f->n = c->n;
+  f->tn = c->nfp;
+  f->nb = c->nb;
+  f->g = c->g;
+  f->g.tn = c->nfp;
+  f->g.fxyz = c->fp_x.p;
+  f->g.diag = 0;
+  f->wvn.view(c->wvn);
+  f->ovf.view(c->ovf);
+  const int rc = field_setup(f, of);
+  c->launches += f->launches.load();
+  c->lib_calls += f->lib_calls.load();
+  if (rc < 0) {
+    field_free(f);
+    if (rc != HAMS_ERR_NOMEM) return rc;
+    g_err.clear();
+    return 0;
+  }
+  c->field = f;
+  return 0;
+}
+// This frequency's influences at the field points into f's A and S.
+static int field_green(hams_ctx* c, hams_ctx* f, const WaveDev& wd) {
+  const long long before = f->launches;
+  if (f->opts.depth < 0.0) {
+    k_green_inf<<<dim3((f->tn + 127) / 128, f->n), 128, 0, f->st>>>(f->g, wd, nullptr, f->rs.p, f->rd.p, f->A.p, f->S.p);
+    TRY(launch_check(f));
+  } else {
+    if (!wd.limit) {
+      launch_mode_tables(f->st, f->g, wd, f->wvn.p, f->mt.nmode, f->mt_pm.p, f->mt_ac.p, f->mt_src.p, f->mt_srct.p,
+                         f->mt_fld.p, f->mt_fldt.p);
+      TRY(launch_check(f));
+    }
+    for (bool& r : f->rad_ready) r = false;
+    TRY(linton_bin(f, wd));
+    for (int b = 1; b < 4; ++b) TRY(series_bin(f, wd, b));
+  }
+  c->launches += f->launches - before;
+  return 0;
+}
+
 // Potentials at the field points from the solved panel potentials X
 // (CalPotentialMulti, PressureElevationMulti.f90:55-272): the influence of
-// every panel at every point (k_field_pairs), then
+// every panel at every point (field_green), then
 // POT = (S_f BC - D_f X) / (2 pi or 4 pi) as two complex GEMMs, the incident
 // potential added for the total-potential solution; copied to fp_last.
 static int field_dev(hams_ctx* c, const hams_wave* w, int nbeta) {
@@ -2717,17 +2821,27 @@ static int field_dev(hams_ctx* c, const hams_wave* w, int nbeta) {
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0), zero = make_cuDoubleComplex(0.0, 0.0),
                         mone = make_cuDoubleComplex(-1.0, 0.0);
   WaveDev wd = wave_dev(c, w);
-  TRY(c->fp_S.alloc((size_t)nfp * n));
-  TRY(c->fp_D.alloc((size_t)nfp * n));
   TRY(c->fp_bc.alloc((size_t)n * ncol));
   TRY(c->fp_pot.alloc((size_t)nfp * ncol));
   TRY(c->fp_out.alloc((size_t)nfp * (ncol + nbeta)));
-  launch_field_pairs(c->st, c->g, wd, c->wvn.p, nfp, c->fp_x.p, c->fp_S.p, c->fp_D.p, c->ovf.p);
+  double2 *fS, *fD;
+  if (c->field) {
+    TRY(field_green(c, c->field, wd));
+    fS = c->field->S.p;
+    fD = c->field->A.p;
+  } else {
+    TRY(c->fp_S.alloc((size_t)nfp * n));
+    TRY(c->fp_D.alloc((size_t)nfp * n));
+    fS = c->fp_S.p;
+    fD = c->fp_D.p;
+    launch_field_pairs(c->st, c->g, wd, c->wvn.p, nfp, c->fp_x.p, fS, fD, c->ovf.p);
+    TRY(launch_check(c));
+  }
   k_field_bc<<<dim3((n + 127) / 128, ncol), 128, 0, c->st>>>(c->g, nbeta, c->wd.p, c->fp_bc.p);
-  TRY(launch_check(c, 2));
-  CUB_(cublasZgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, nfp, ncol, n, &one, (cuDoubleComplex*)c->fp_S.p, nfp,
+  TRY(launch_check(c));
+  CUB_(cublasZgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, nfp, ncol, n, &one, (cuDoubleComplex*)fS, nfp,
                    (cuDoubleComplex*)c->fp_bc.p, n, &zero, (cuDoubleComplex*)c->fp_pot.p, nfp));
-  CUB_(cublasZgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, nfp, ncol, n, &mone, (cuDoubleComplex*)c->fp_D.p, nfp,
+  CUB_(cublasZgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, nfp, ncol, n, &mone, (cuDoubleComplex*)fD, nfp,
                    (cuDoubleComplex*)c->X.p, n, &one, (cuDoubleComplex*)c->fp_pot.p, nfp));
   c->lib_calls += 2;
   IncWave q = inc_params(wd, c->opts.amp, c->opts.g, c->opts.xw[0], c->opts.xw[1]);
@@ -3392,6 +3506,11 @@ extern "C" int hams_ctx_set_field_points(hams_ctx* c, int32_t nfp, const double*
     CU(cudaMemcpy(c->fp_x.p, xfp, 3 * (size_t)nfp * 8, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(c->fp_sld.p, sld.data(), (size_t)nfp * 8, cudaMemcpyHostToDevice));
   }
+  for (hams_ctx* l : c->lanes) {  // they share c's pair set
+    field_free(l->field);
+    l->field = nullptr;
+  }
+  TRY(field_context(c, nullptr));
   for (hams_ctx* l : c->lanes) {
     l->nfp = nfp;
     l->fp_last.clear();
@@ -3399,7 +3518,9 @@ extern "C" int hams_ctx_set_field_points(hams_ctx* c, int32_t nfp, const double*
       l->fp_x.view(c->fp_x);
       l->fp_sld.view(c->fp_sld);
     }
+    if (c->field) TRY(field_context(l, c->field));
   }
+  CU(cudaStreamSynchronize(c->st));
   return 0;
 }
 

@@ -21,6 +21,7 @@ struct DevGeom {
   const int* ncn;      // (n)
   const int* body;     // (n) body of each source panel
   const int* bstart;   // (nb+1)
+  int diag;            // field point i is source panel i (the 2 pi of the hull diagonal)
 };
 
 struct WaveDev {
@@ -51,7 +52,7 @@ __device__ __forceinline__ void store_pair_v(size_t p, int i, int j, const grn4&
 __device__ __forceinline__ void store_pair(const DevGeom& g, size_t p, int i, int j, const grn4& G,
                                            const double* __restrict__ rs, const double* __restrict__ rd,
                                            double2* __restrict__ A, double2* __restrict__ S) {
-  store_pair_v(p, i, j, G, g.ds[j], g.nrm[j], g.nrm[j + g.n], g.nrm[j + 2 * g.n], rs[p], rd[p], A, S);
+  store_pair_v(p, i, g.diag ? j : -1, G, g.ds[j], g.nrm[j], g.nrm[j + g.n], g.nrm[j + 2 * g.n], rs[p], rd[p], A, S);
 }
 
 
