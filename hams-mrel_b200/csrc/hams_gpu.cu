@@ -85,6 +85,7 @@ static int fail(int code, const char* fmt, ...) {
   } while (0)
 
 #include "kernels.cuh"
+#include "lu_fp64.h"
 #include "lu_mixed.h"
 #include "gemm_tf32.h"
 #include "green_sg.h"
@@ -1237,6 +1238,8 @@ struct hams_ctx {
   DBuf<double> gnrm;
   DBuf<int> gpiv;
   DBuf<int> perm;
+  int zlu = -1;  // fp64: the own LU runs at this order (-1: not asked yet)
+  DBuf<int> zwork;
   int lu_used = -1;  // mixed form: factorisation used by the last solve (HAMS_LU_*)
   DBuf<double> wvn, beta, outbuf, colratio;
   DBuf<double> mt_pm, mt_ac, mt_fld, mt_fldt;  // per-frequency mode tables (finite depth)
@@ -1349,7 +1352,8 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
   rel(c->rid, c->ur, c->lrow, c->lrep, c->lin_fg);
   for (int br = 0; br < 4; ++br) rel(c->rad_k[br], c->rad_j[br]);
   rel(c->blk_copied, c->blk_list, c->chunks, c->bchunk, c->A, c->S, c->B, c->part, c->wd, c->C, c->D, c->X, c->R);
-  rel(c->Af, c->Xf, c->luw, c->gv, c->gw, c->gz, c->gy, c->gpre, c->gnrm, c->gpiv, c->perm);
+  rel(c->Af, c->Xf, c->luw, c->gv, c->gw, c->gz, c->gy, c->gpre, c->gnrm, c->gpiv, c->perm,
+      c->zwork);
   rel(c->wvn, c->beta, c->outbuf, c->colratio, c->mt_pm, c->mt_ac, c->mt_fld, c->mt_fldt, c->mt_src, c->mt_srct);
   rel(c->ipiv, c->info, c->ovf, c->work, c->work32, c->sg_wh, c->sg_w0, c->sg_bias, c->sg_samp, c->sg_g1, c->sg_g2);
   rel(c->sg_map, c->sg_scale, c->jB, c->jdX, c->sg_red, c->sg_cells, c->outbuf2);
@@ -2677,6 +2681,17 @@ static int solve_dev(hams_ctx* c, int nrhs, int* info_host) {
   // (AssbMatx_irr.f90:494-498)
   if (c->opts.solver == HAMS_SOLVER_GMRES) return gmres_solve(c, M, rhs, nrhs);
   if (c->opts.precision == HAMS_PREC_FP64) {
+    if (c->zlu < 0) c->zlu = zlu_supported(n) == 0;
+    if (c->zlu) {  // M is overwritten by its factors
+      TRY(c->zwork.alloc(zlu_work_ints()));
+      long long la = 0, lb = 0;
+      const int rc = zlu_solve(c->st, c->blas, n, nrhs, M, c->X.p, c->info.p, c->zwork.p, c->evf, &la, &lb);
+      c->launches += la;
+      c->lib_calls += lb;
+      if (rc) return fail(HAMS_ERR_CUDA, "LU: %s", rc >= 10 ? "a cuBLAS product failed" : cudaGetErrorString(cudaGetLastError()));
+      CU(cudaMemcpyAsync(info_host, c->info.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+      return 0;
+    }
     int lw = 0;
     CUS(cusolverDnZgetrf_bufferSize(c->solver, n, n, (cuDoubleComplex*)M, n, &lw));
     TRY(c->work.alloc((size_t)lw * sizeof(cuDoubleComplex)));
