@@ -38,6 +38,13 @@ constexpr int kZThreads = 512;      // rows per block of the panel's cluster
 constexpr int kZMoves = 2 * kZW;    // row moves of a panel at most
 constexpr int kZList = 2 * kZMoves;  // workspace per panel of a block: (destination or -1, source) pairs
 
+// Systems of one order factored together (blockIdx.z, or .y of the panels'
+// clusters, the system): strides of A and X, the workspace after one another.
+struct ZBatch {
+  size_t a, x;
+  __device__ __forceinline__ int* list(int* work, int sys) const { return work + (size_t)sys * kZP * kZList; }
+};
+
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
   return make_double2(fma(-a.y, b.y, a.x * b.x), fma(a.y, b.x, a.x * b.y));
 }
@@ -69,7 +76,7 @@ __device__ __forceinline__ double2 zrcp(double2 d) {
 // order.  At the end the pivot rows are stored in their order,
 // the rows they displace in the places they leave; moves lists both.
 __global__ void __launch_bounds__(kZThreads, 1) k_zpanel(double2* __restrict__ A, int lda, int n, int c0, int w,
-                                                        int* __restrict__ moves, int* info) {
+                                                        ZBatch zb, int* __restrict__ work, int panel, int* info) {
   __shared__ __align__(16) double2 offer[2][16][kZW];  // [column & 1][block]: each block's best row
   __shared__ uint32_t okey[2][16];
   __shared__ int orow[2][16];
@@ -83,6 +90,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zpanel(double2* __restrict__ A
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(nct));
   const int r = c0 + (int)rank * kZThreads + tid;
   const bool live = r < n;
+  A += blockIdx.y * zb.a;
+  int* moves = zb.list(work, blockIdx.y) + panel * kZList;
   pdl_wait();
   pdl_next();
   double2 a[kZW];
@@ -239,12 +248,14 @@ __device__ __forceinline__ void load_diag(double2* T, const double2* __restrict_
 // takes 8 columns: 16 threads each, one per panel row.
 constexpr int kZApplyCols = 8;
 __global__ void __launch_bounds__(128) k_zapply(double2* __restrict__ A, int lda, int k0, int k1, int c0, int w,
-                                                const int* __restrict__ moves) {
+                                                ZBatch zb, int* work, int panel) {
   __shared__ double2 buf[kZMoves * kZApplyCols];
   __shared__ double2 L[kZW][kZW + 1];
   // the block's columns without the panel's
   const int left = c0 - k0, total = left + (k1 - c0 - w), q0 = blockIdx.x * kZApplyCols;
   const int cols = min(kZApplyCols, total - q0);
+  A += blockIdx.z * zb.a;
+  const int* moves = zb.list(work, blockIdx.z) + panel * kZList;
   pdl_wait();
   pdl_next();
   auto col = [&](int q) { return A + (size_t)(q0 + q < left ? k0 + q0 + q : c0 + w + (q0 + q - left)) * lda; };
@@ -264,8 +275,10 @@ __global__ void __launch_bounds__(128) k_zapply(double2* __restrict__ A, int lda
 // block's columns r0 .. k1-1, the panel's w columns k.  A block of 128 threads
 // takes 128 rows and 8 columns, a row per thread.
 constexpr int kZUpCols = 8;
-__global__ void __launch_bounds__(128) k_zupdate(double2* __restrict__ A, int lda, int n, int k1, int c0, int w) {
+__global__ void __launch_bounds__(128) k_zupdate(double2* __restrict__ A, int lda, int n, int k1, int c0, int w,
+                                                 ZBatch zb) {
   __shared__ double2 U[kZW][kZUpCols];
+  A += blockIdx.z * zb.a;
   pdl_wait();
   pdl_next();
   const int r0 = c0 + w, r = r0 + blockIdx.x * 128 + threadIdx.x, q0 = r0 + blockIdx.y * kZUpCols;
@@ -300,13 +313,16 @@ __global__ void __launch_bounds__(128) k_zupdate(double2* __restrict__ A, int ld
 constexpr int kZRightCols = 16;
 constexpr int kZRightSmem = (kZB * (kZB + 1) + kZB * (kZRightCols + 1)) * (int)sizeof(double2);
 __global__ void __launch_bounds__(256) k_zright(double2* __restrict__ A, int lda, int n, int k0, int kb,
-                                                double2* __restrict__ X, int nrhs, const int* __restrict__ moves) {
+                                                double2* __restrict__ X, int nrhs, ZBatch zb, int* work) {
   extern __shared__ __align__(16) double2 zs[];
   double2* L = zs;                       // [column k][row i], ld kZB + 1
   double2* Y = zs + kZB * (kZB + 1);     // [row i][column q], ld kZRightCols + 1; the moves' buffer before
   constexpr int kLl = kZB + 1, kYl = kZRightCols + 1;
   const int right = n - k0 - kb, total = k0 + right + nrhs, q0 = blockIdx.x * kZRightCols;
   const int cols = min(kZRightCols, total - q0);
+  A += blockIdx.z * zb.a;
+  X += blockIdx.z * zb.x;
+  const int* moves = zb.list(work, blockIdx.z);
   auto col = [&](int q) {
     const int c = q0 + q;
     return c < k0 ? A + (size_t)c * lda
@@ -353,13 +369,15 @@ __global__ void __launch_bounds__(256) k_zright(double2* __restrict__ A, int lda
 constexpr int kZBackCols = 8;
 constexpr int kZBackSmem = (kZB * (kZB + 1) + kZB * (kZBackCols + 1) + kZB) * (int)sizeof(double2);
 __global__ void __launch_bounds__(128) k_zback(const double2* __restrict__ A, int lda, int n, int k0, int kb,
-                                               double2* __restrict__ X, int nrhs) {
+                                               double2* __restrict__ X, int nrhs, ZBatch zb) {
   extern __shared__ __align__(16) double2 zs[];
   double2* U = zs;
   double2* Y = zs + kZB * (kZB + 1);
   double2* R = Y + kZB * (kZBackCols + 1);  // reciprocals of the diagonal
   constexpr int kUl = kZB + 1, kYl = kZBackCols + 1;
   const int q0 = blockIdx.x * kZBackCols, cols = min(kZBackCols, nrhs - q0);
+  A += blockIdx.z * zb.a;
+  X += blockIdx.z * zb.x;
   pdl_wait();
   pdl_next();
   load_diag<128>(U, A, lda, k0, kb);
@@ -405,10 +423,11 @@ int cluster_of(int rows) {
   return c;
 }
 
-cudaError_t launch_panel(cudaStream_t st, double2* A, int n, int c0, int w, int* moves, int* info) {
+cudaError_t launch_panel(cudaStream_t st, int batch, double2* A, int n, int c0, int w, ZBatch zb, int* work, int panel,
+                         int* info) {
   const int cs = cluster_of(n - c0);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs);
+  cfg.gridDim = dim3(cs, batch);
   cfg.blockDim = dim3(kZThreads);
   cfg.stream = st;
   cudaLaunchAttribute at[2];
@@ -419,12 +438,12 @@ cudaError_t launch_panel(cudaStream_t st, double2* A, int n, int c0, int w, int*
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, k_zpanel, A, n, n, c0, w, moves, info);
+  return cudaLaunchKernelEx(&cfg, k_zpanel, A, n, n, c0, w, zb, work, panel, info);
 }
 
 }  // namespace
 
-size_t zlu_work_ints() { return (size_t)kZP * kZList; }
+size_t zlu_work_ints(int batch) { return (size_t)batch * kZP * kZList; }
 
 int zlu_supported(int n) {
   if (n < 1 || n > kZluMaxRows) return 1;
@@ -452,55 +471,63 @@ int zlu_supported(int n) {
   return 0;
 }
 
-int zlu_solve(cudaStream_t st, cublasHandle_t blas, int n, int nrhs, double2* A, double2* X, int* info, int* work,
-              cudaEvent_t evf, long long* launches, long long* lib_calls) {
+int zlu_solve(cudaStream_t st, cublasHandle_t blas, int batch, int n, int nrhs, double2* A, size_t sa, double2* X,
+              size_t sx, int* info, int* work, cudaEvent_t evf, long long* launches, long long* lib_calls) {
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0), mone = make_cuDoubleComplex(-1.0, 0.0);
   if (cudaMemsetAsync(info, 0, sizeof(int), st) != cudaSuccess) return 1;
-  auto gemm = [&](int m, int nn, int k, const double2* a, const double2* b, int ldb, double2* c, int ldc) {
+  const ZBatch zb{sa, sx};
+  // c -= a b, a and c with their stride, b with sb
+  auto gemm = [&](int m, int nn, int k, const double2* a, const double2* b, size_t sb, double2* c, size_t sc) {
     if (m <= 0 || nn <= 0) return 0;
     *lib_calls += 1;
-    const cublasStatus_t s = cublasZgemm(blas, CUBLAS_OP_N, CUBLAS_OP_N, m, nn, k, &mone, (const cuDoubleComplex*)a, n,
-                                         (const cuDoubleComplex*)b, ldb, &one, (cuDoubleComplex*)c, ldc);
+    const cuDoubleComplex *pa = (const cuDoubleComplex*)a, *pb = (const cuDoubleComplex*)b;
+    cuDoubleComplex* pc = (cuDoubleComplex*)c;
+    const cublasStatus_t s =
+        batch == 1 ? cublasZgemm(blas, CUBLAS_OP_N, CUBLAS_OP_N, m, nn, k, &mone, pa, n, pb, n, &one, pc, n)
+                   : cublasZgemmStridedBatched(blas, CUBLAS_OP_N, CUBLAS_OP_N, m, nn, k, &mone, pa, n, (long long)sa, pb,
+                                               n, (long long)sb, &one, pc, n, (long long)sc, batch);
     return s == CUBLAS_STATUS_SUCCESS ? 0 : 10 + (int)s;
   };
+  auto blocks = [&](int count, int per) { return (unsigned)((count + per - 1) / per); };
   for (int k0 = 0; k0 < n; k0 += kZB) {
     const int k1 = k0 + kZB < n ? k0 + kZB : n, kb = k1 - k0, right = n - k1;
     for (int p = 0, c0 = k0; c0 < k1; ++p, c0 += kZW) {
       const int w = k1 - c0 < kZW ? k1 - c0 : kZW, others = kb - w;
-      int* moves = work + p * kZList;
-      if (launch_panel(st, A, n, c0, w, moves, info) != cudaSuccess) return 1;
+      if (launch_panel(st, batch, A, n, c0, w, zb, work, p, info) != cudaSuccess) return 1;
       *launches += 1;
       if (others > 0) {
-        pdl_launch(k_zapply, dim3((others + kZApplyCols - 1) / kZApplyCols), dim3(128), 0, st, A, n, k0, k1, c0, w,
-                   moves);
+        pdl_launch(k_zapply, dim3(blocks(others, kZApplyCols), 1, batch), dim3(128), 0, st, A, n, k0, k1, c0, w, zb,
+                   work, p);
         *launches += 1;
       }
       const int rest = k1 - c0 - w, below = n - c0 - w;
       if (rest > 0) {
-        pdl_launch(k_zupdate, dim3((below + 127) / 128, (rest + kZUpCols - 1) / kZUpCols), dim3(128), 0, st, A, n, n,
-                   k1, c0, w);
+        pdl_launch(k_zupdate, dim3(blocks(below, 128), blocks(rest, kZUpCols), batch), dim3(128), 0, st, A, n, n, k1,
+                   c0, w, zb);
         *launches += 1;
       }
     }
     const int total = k0 + right + nrhs;
     if (total > 0) {
-      pdl_launch(k_zright, dim3((total + kZRightCols - 1) / kZRightCols), dim3(256), kZRightSmem, st, A, n, n, k0, kb,
-                 X, nrhs, work);
+      pdl_launch(k_zright, dim3(blocks(total, kZRightCols), 1, batch), dim3(256), kZRightSmem, st, A, n, n, k0, kb, X,
+                 nrhs, zb, work);
       *launches += 1;
     }
     if (cudaGetLastError() != cudaSuccess) return 1;
-    int rc = gemm(right, right, kb, A + (size_t)k0 * n + k1, A + (size_t)k1 * n + k0, n, A + (size_t)k1 * n + k1, n);
-    if (!rc) rc = gemm(right, nrhs, kb, A + (size_t)k0 * n + k1, X + k0, n, X + k1, n);
+    double2* Lk = A + (size_t)k0 * n + k1;
+    int rc = gemm(right, right, kb, Lk, A + (size_t)k1 * n + k0, sa, A + (size_t)k1 * n + k1, sa);
+    if (!rc) rc = gemm(right, nrhs, kb, Lk, X + k0, sx, X + k1, sx);
     if (rc) return rc;
   }
   if (evf && cudaEventRecord(evf, st) != cudaSuccess) return 1;
   if (nrhs <= 0) return 0;
   for (int k0 = (n - 1) / kZB * kZB; k0 >= 0; k0 -= kZB) {
     const int kb = k0 + kZB < n ? kZB : n - k0;
-    pdl_launch(k_zback, dim3((nrhs + kZBackCols - 1) / kZBackCols), dim3(128), kZBackSmem, st, A, n, n, k0, kb, X, nrhs);
+    pdl_launch(k_zback, dim3(blocks(nrhs, kZBackCols), 1, batch), dim3(128), kZBackSmem, st, A, n, n, k0, kb, X, nrhs,
+               zb);
     *launches += 1;
     if (cudaGetLastError() != cudaSuccess) return 1;
-    const int rc = gemm(k0, nrhs, kb, A + (size_t)k0 * n, X + k0, n, X, n);
+    const int rc = gemm(k0, nrhs, kb, A + (size_t)k0 * n, X + k0, sx, X, sx);
     if (rc) return rc;
   }
   return 0;
