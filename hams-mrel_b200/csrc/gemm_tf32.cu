@@ -1,7 +1,8 @@
 // gemm_tf32.cu -- C = alpha A B + beta C on the fifth-generation tensor cores.
 //
-// One CTA computes a 128 x 128 tile of C.  Warp 0 streams the K panels of A
-// and B into a three-stage shared-memory ring with the tensor memory
+// One CTA computes a 128 x 128 (or 128 x 64) tile of C; wide products take a
+// persistent kernel of 128 x 256 tiles (k_gemm_tf32_wide).  Warp 0 streams the K
+// panels of A and B into a three-stage shared-memory ring with the tensor memory
 // accelerator (cp.async.bulk.tensor, 128-byte swizzle, no multicast: every
 // operand is this GPU's own memory); warp 1 owns the tile's 128 tensor-memory
 // columns and issues tcgen05.mma kind::tf32 (M = 128, N = 128, K = 8) from
@@ -40,7 +41,8 @@ constexpr long long kSpin = 1ll << 22;
 
 // Tile shape of one variant: BN columns of C per CTA (the MMA's N and the
 // tensor-memory columns), STAGES K panels in flight.  64 x 4 stages: 96 KB,
-// two CTAs per SM; 128 x 3: 97 KB, two CTAs; 256 x 3: 145 KB, one CTA.
+// two CTAs per SM; 128 x 3: 97 KB, two CTAs.  The 256-column variant is
+// k_gemm_tf32_wide below.
 template <int BN, int STAGES>
 struct Tile {
   static constexpr int kBBytes = BN * kBK * 4;
@@ -48,11 +50,13 @@ struct Tile {
   static constexpr int kOffBar = kOffB + STAGES * kBBytes;  // full[STAGES], empty[STAGES], acc
   static constexpr int kOffMisc = kOffBar + 8 * (2 * STAGES + 1);
   static constexpr int kSmemBytes = kOffMisc + 16 + 1024;  // + alignment slack of the dynamic window
-  // instruction descriptor, kind::tf32: D f32 (bit 4), A and B tf32 (format 2
-  // at bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-  static constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                     ((uint32_t)(kBM >> 4) << 24);
 };
+
+// instruction descriptor, kind::tf32: D f32 (bit 4), A and B tf32 (format 2
+// at bits 7 and 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+constexpr uint32_t idesc(int bn) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -98,14 +102,38 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "r"(taddr));
 }
 
+__device__ __forceinline__ void tma_panel(const CUtensorMap* tm, uint32_t dst, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+
+// the four K = 8 steps of one K panel (8 tf32 = 32 bytes along the swizzled
+// row each); the first overwrites the accumulator when first is set
+__device__ __forceinline__ void mma_panel(uint32_t tacc, uint64_t da, uint64_t db, uint32_t idesc, bool first) {
+#pragma unroll
+  for (int kk = 0; kk < kBK / 8; ++kk) {
+    const uint32_t acc = !(first && kk == 0);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tacc),
+        "l"(da + (uint64_t)(2 * kk)), "l"(db + (uint64_t)(2 * kk)), "r"(idesc), "r"(acc));
+  }
+}
+
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(kThreads, BN <= 128 ? 2 : 1)
+__global__ void __launch_bounds__(kThreads, 2)
     k_gemm_tf32(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, float* __restrict__ C,
                 int ldc, int M, int N, int K, float alpha, float beta, int c_rowmajor, int* err) {
   using T = Tile<BN, STAGES>;
   constexpr int kBN = BN, kStages = STAGES, kBBytes = T::kBBytes, kOffB = T::kOffB, kOffBar = T::kOffBar,
                 kOffMisc = T::kOffMisc;
-  constexpr uint32_t kIdesc = T::kIdesc;
+  constexpr uint32_t kIdesc = idesc(BN);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);  // 1024-aligned window
   const uint32_t sbase = smem_u32(smem);
@@ -150,16 +178,8 @@ __global__ void __launch_bounds__(kThreads, BN <= 128 ? 2 : 1)
         const uint32_t fb = bar_full + 8 * s;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(kABytes + kBBytes)
                      : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-                "r"(sbase + s * kABytes),
-            "l"(reinterpret_cast<uint64_t>(&tmA)), "r"(kb * kBK), "r"(m0), "r"(fb)
-            : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-                "r"(sbase + kOffB + s * kBBytes),
-            "l"(reinterpret_cast<uint64_t>(&tmB)), "r"(kb * kBK), "r"(n0), "r"(fb)
-            : "memory");
+        tma_panel(&tmA, sbase + s * kABytes, kb * kBK, m0, fb);
+        tma_panel(&tmB, sbase + kOffB + s * kBBytes, kb * kBK, n0, fb);
         issued = kb + 1;
       }
       // the copies in flight land before the CTA leaves (bounded)
@@ -179,22 +199,11 @@ __global__ void __launch_bounds__(kThreads, BN <= 128 ? 2 : 1)
           break;
         }
         tc_fence_after();
-        const uint64_t da = sdesc_sw128(sbase + s * kABytes), db = sdesc_sw128(sbase + kOffB + s * kBBytes);
-#pragma unroll
-        for (int kk = 0; kk < kBK / 8; ++kk) {  // K = 8 tf32 = 32 bytes along the swizzled row
-          const uint32_t acc = (kb | kk) != 0;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tbase),
-              "l"(da + (uint64_t)(2 * kk)), "l"(db + (uint64_t)(2 * kk)), "r"(kIdesc), "r"(acc));
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         bar_empty + 8 * s)
-                     : "memory");
+        mma_panel(tbase, sdesc_sw128(sbase + s * kABytes), sdesc_sw128(sbase + kOffB + s * kBBytes), kIdesc, kb == 0);
+        tc_commit(bar_empty + 8 * s);
       }
       // completion of every MMA issued (also on abort, so that tensor memory is idle before it is freed)
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_acc)
-                   : "memory");
+      tc_commit(bar_acc);
       for (long long it = 0; it < kSpin && !mbar_try(bar_acc, 0); ++it) {
       }
     }
@@ -255,6 +264,190 @@ __global__ void __launch_bounds__(kThreads, BN <= 128 ? 2 : 1)
   }
 }
 
+// The wide variant: 128 x 256 tiles, a CTA per SM that takes tile after tile.
+// Two accumulators of 256 tensor-memory columns let the main loop of a tile run
+// under the epilogue of the one before, which the single-tile kernel gets from a
+// second CTA per SM that 256 columns have no shared memory for; eight epilogue
+// warps (two per tensor-memory quarter, 128 columns each) keep twice the reads
+// of C in flight.  The wide tile reads its operands from L2 1.28 times less
+// often than 128 x 128 ones, which bound the trailing updates.  Rank-512 updates
+// against the fastest of the single-tile variants (128 x 256 tiles in single-tile
+// form were slower than both, 4,329 us in the last case): 20.8 -> 16.8 us at
+// 2,600 x 1,300, 194 -> 139 us (392 TFLOP/s) at 10,344 x 5,172, 3,166 -> 1,916 us
+// (424 TFLOP/s) at 39,808 x 19,904, where C's read and write take 970 us at the
+// copy bandwidth and the operands' 19 GB from L2 bound the rest.
+constexpr int kWBN = 256, kWStages = 4, kWThreads = 320, kWEpi = 8;
+struct Wide {
+  static constexpr int kBBytes = kWBN * kBK * 4;
+  static constexpr int kOffB = kWStages * kABytes;
+  static constexpr int kOffBar = kOffB + kWStages * kBBytes;  // full, empty [stages], acc full, acc empty [2], done
+  static constexpr int kBars = 2 * kWStages + 5;
+  static constexpr int kOffMisc = kOffBar + 8 * kBars;
+  static constexpr int kSmemBytes = kOffMisc + 16 + 1024;
+};
+
+__global__ void __launch_bounds__(kWThreads, 1)
+    k_gemm_tf32_wide(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     float* __restrict__ C, int ldc, int M, int N, int K, float alpha, float beta, int c_rowmajor,
+                     int* err) {
+  constexpr uint32_t kIdesc = idesc(kWBN);
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+  const uint32_t sbase = smem_u32(smem);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Wide::kOffBar);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Wide::kOffMisc);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + Wide::kOffMisc + 4);
+  const uint32_t bar_full = smem_u32(&bars[0]), bar_empty = smem_u32(&bars[kWStages]),
+                 bar_acc = smem_u32(&bars[2 * kWStages]), bar_free = smem_u32(&bars[2 * kWStages + 2]),
+                 bar_done = smem_u32(&bars[2 * kWStages + 4]);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nk = (K + kBK - 1) / kBK, mt = (M + kBM - 1) / kBM;
+  const int tiles = mt * ((N + kWBN - 1) / kWBN);
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < Wide::kBars; ++s) {
+      const int count = s == 2 * kWStages + 2 || s == 2 * kWStages + 3 ? kWEpi : 1;
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bars[s])), "r"(count));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                 "r"(2 * kWBN));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tbase = *reinterpret_cast<volatile uint32_t*>(tslot);
+  pdl_wait();  // the operands and C are the predecessors' results
+  pdl_next();
+  auto give_up = [&] {
+    atomicOr(err, 1);
+    *abort_flag = 1;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {  // producer: the K panels of all tiles, one after another
+      int p = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x)
+        for (int kb = 0; kb < nk; ++kb, ++p) {
+          const int s = p % kWStages;
+          if (p >= kWStages && !mbar_wait(bar_empty + 8 * s, (uint32_t)((p / kWStages - 1) & 1), abort_flag)) {
+            give_up();
+            ok = false;
+            break;
+          }
+          const uint32_t fb = bar_full + 8 * s;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(kABytes + Wide::kBBytes)
+                       : "memory");
+          tma_panel(&tmA, sbase + s * kABytes, kb * kBK, t % mt * kBM, fb);
+          tma_panel(&tmB, sbase + Wide::kOffB + s * Wide::kBBytes, kb * kBK, t / mt * kWBN, fb);
+        }
+      // the copies in flight land before the CTA leaves (bounded)
+      for (int i = p > kWStages ? p - kWStages : 0; i < p; ++i) {
+        const int s = i % kWStages;
+        for (long long it = 0; it < kSpin && !mbar_try(bar_full + 8 * s, (uint32_t)((i / kWStages) & 1)); ++it) {
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // MMA issue
+      int p = 0, u = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++u) {
+        const int b = u & 1;
+        if (u >= 2) {  // the epilogue has read this accumulator's last tile
+          if (!mbar_wait(bar_free + 8 * b, (uint32_t)((u / 2 - 1) & 1), abort_flag)) {
+            give_up();
+            break;
+          }
+          tc_fence_after();
+        }
+        for (int kb = 0; kb < nk; ++kb, ++p) {
+          const int s = p % kWStages;
+          if (!mbar_wait(bar_full + 8 * s, (uint32_t)((p / kWStages) & 1), abort_flag)) {
+            give_up();
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          mma_panel(tbase + (uint32_t)(b * kWBN), sdesc_sw128(sbase + s * kABytes),
+                    sdesc_sw128(sbase + Wide::kOffB + s * Wide::kBBytes), kIdesc, kb == 0);
+          tc_commit(bar_empty + 8 * s);
+        }
+        if (ok) tc_commit(bar_acc + 8 * b);
+      }
+      // completion of every MMA issued (also on abort, so that tensor memory is idle before it is freed)
+      tc_commit(bar_done);
+      for (long long it = 0; it < kSpin && !mbar_try(bar_done, 0); ++it) {
+      }
+    }
+  } else {  // epilogue: warp w reads tensor-memory lanes 32 (w % 4) ..., columns 128 of one half
+    const int q = warp & 3, half = (warp - 2) / 4 * (kWBN / 2);
+    constexpr int kCh = 32;
+    int u = 0;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++u) {
+      const int b = u & 1, row = t % mt * kBM + 32 * q + lane, n0 = t / mt * kWBN + half;
+      const bool live = row < M;
+      auto load_chunk = [&](int c0, float (&cv)[kCh]) {
+#pragma unroll
+        for (int j = 0; j < kCh; ++j) {
+          const int col = n0 + c0 + j;
+          cv[j] = (beta != 0.0f && live && col < N)
+                      ? (c_rowmajor ? C[(size_t)row * ldc + col] : C[(size_t)col * ldc + row])
+                      : 0.0f;
+        }
+      };
+      float cn[kCh];
+      load_chunk(0, cn);
+      bool ok = mbar_wait(bar_acc + 8 * b, (uint32_t)((u / 2) & 1), abort_flag);
+      if (!ok) give_up();
+      ok = __all_sync(0xffffffffu, ok && !*abort_flag);  // the tensor-memory loads below are warp-wide
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t trow = tbase + (uint32_t)(b * kWBN + half) + ((uint32_t)(32 * q) << 16);
+#pragma unroll 1
+      for (int c0 = 0; c0 < kWBN / 2; c0 += kCh) {
+        float cc[kCh];
+#pragma unroll
+        for (int j = 0; j < kCh; ++j) cc[j] = cn[j];
+        if (c0 + kCh < kWBN / 2) load_chunk(c0 + kCh, cn);  // in flight while this chunk is written
+        uint32_t v[32];
+        tmem_ld32(trow + (uint32_t)c0, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (c0 + kCh == kWBN / 2) {  // the accumulator is free for the tile after next
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_free + 8 * b) : "memory");
+        }
+        if (live) {
+#pragma unroll
+          for (int j = 0; j < kCh; ++j) {
+            const int col = n0 + c0 + j;
+            if (col < N) {
+              float* dst = c_rowmajor ? C + (size_t)row * ldc + col : C + (size_t)col * ldc + row;
+              *dst = fmaf(alpha, __uint_as_float(v[j]), beta * cc[j]);
+            }
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(2 * kWBN));
+  }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
@@ -311,6 +504,34 @@ int launch(cudaStream_t st, int dev, int m, int n, int k, float alpha, const flo
              : 1;
 }
 
+int launch_wide(cudaStream_t st, int dev, int m, int n, int k, float alpha, const float* A, int lda, const float* B,
+                int ldb, float beta, float* C, int ldc, bool c_rowmajor, int* err) {
+  // the shared-memory opt-in and the number of SMs, once per device
+  static std::mutex mu;
+  static int sms[64] = {};
+  int ctas;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!sms[dev]) {
+      int count = 0;
+      if (cudaFuncSetAttribute(k_gemm_tf32_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, Wide::kSmemBytes) !=
+              cudaSuccess ||
+          cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+      sms[dev] = count;
+    }
+    ctas = sms[dev];
+  }
+  CUtensorMap ta, tb;
+  if (!make_map(&ta, A, k, m, lda, kBM) || !make_map(&tb, B, k, n, ldb, kWBN)) return 1;
+  const long long tiles = (long long)((m + kBM - 1) / kBM) * ((n + kWBN - 1) / kWBN);
+  if (tiles > 0x3fffffff) return 1;
+  return pdl_launch(k_gemm_tf32_wide, dim3((unsigned)std::min<long long>(tiles, ctas)), dim3(kWThreads),
+                    Wide::kSmemBytes, st, ta, tb, C, ldc, m, n, k, alpha, beta, c_rowmajor ? 1 : 0, err) == cudaSuccess
+             ? 0
+             : 1;
+}
+
 }  // namespace
 
 int gemm_tf32_variant(cudaStream_t st, int variant, int m, int n, int k, float alpha, const float* A, int lda,
@@ -324,7 +545,7 @@ int gemm_tf32_variant(cudaStream_t st, int variant, int m, int n, int k, float a
   switch (variant) {
     case 0: return launch<64, 4>(st, dev, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, c_rowmajor, err);
     case 1: return launch<128, 3>(st, dev, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, c_rowmajor, err);
-    case 2: return launch<256, 3>(st, dev, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, c_rowmajor, err);
+    case 2: return launch_wide(st, dev, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, c_rowmajor, err);
     default: return 1;
   }
 }
