@@ -61,13 +61,13 @@ WORKLOAD = "3x3 cylinder array R=4 T=8 spacing 20 m, 5400 quad panels, depth 50 
            "headings 0/30/60/90 deg (54 rad + 4 dif RHS)"
 
 # FP64 operations per EIGENE panel pair of the series Green kernel, from the
-# executed-instruction counters of one ncu capture of that kernel on the
+# executed-instruction counters of one ncu capture of that kernel's three launches on the
 # 3,240-panel profiling case (`--profile-case --form fp64`): dadd + dmul +
 # 2 dfma (smsp__sass_thread_inst_executed_op_d*), and its DRAM bytes per pair
-# (dram__bytes_read.sum + dram__bytes_write.sum over the launch's 4,093,706
+# (dram__bytes_read.sum + dram__bytes_write.sum over the launches' 4,093,706
 # pairs), scaled to a full launch by its pair count.
-EIGENE_FP64_FLOPS_PER_PAIR = 44_410
-EIGENE_DRAM_BYTES_PER_PAIR = 2_381
+EIGENE_FP64_FLOPS_PER_PAIR = 14_317
+EIGENE_DRAM_BYTES_PER_PAIR = 98
 # DRAM bytes per pair of the surrogate kernel: ncu's dram__bytes_read.sum +
 # dram__bytes_write.sum on the 3,240-panel profiling case with identical body
 # blocks (125.5 MB for 3,210,660 pairs), scaled to a full launch by its pair

@@ -21,7 +21,8 @@
 // large triangular solves.  Factorisation and solve (58 right-hand sides at
 // 5,400 panels) against it: 43.5 -> 31.0 ms at 5,400 panels, 14.9 -> 9.0 ms at
 // 2,340 (two in flight), 4.9 -> 2.4 ms at 800 (eight in flight), 0.68 -> 0.66 ms
-// at 234.  What bounds it: the panels' chains (1.9 us per column, 10.6 ms at 5,400
+// at 234.  GMRES inverts its body blocks with it (identity right-hand sides,
+// bodies of one size as one batch).  What bounds it: the panels' chains (1.9 us per column, 10.6 ms at 5,400
 // panels), then ZGEMM (16 ms, 70 % of the FP64 tensor rate).
 #include "lu_fp64.h"
 
