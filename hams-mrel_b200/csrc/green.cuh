@@ -12,7 +12,7 @@
 //
 // The eigenfunction-series terms of EIGEN/EIGENE/PIDCOCK use the
 // bit-reproducible sin/cos/exp/log of detmath.h in the operation order of the
-// CPU checker: the epsilon extrapolation amplifies last-bit differences of a
+// CPU oracle: the epsilon extrapolation amplifies last-bit differences of a
 // math library to up to 1e-3 in single values.
 //
 // Every routine returns the wave part of G with 1/r and 1/r1 removed, plus

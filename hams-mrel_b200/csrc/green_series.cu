@@ -4,7 +4,7 @@
 // terms and extrapolate them with the Wynn epsilon algorithm (Limes), which
 // divides by differences of nearly equal partial sums and stops on exact
 // equalities.  This file is compiled with --fmad=false so that every product
-// and sum of those series is rounded exactly as in the CPU checker; the
+// and sum of those series is rounded exactly as in the CPU oracle; the
 // transcendental functions inside them come from detmath.h.  The remaining
 // kernels (hams_gpu.cu) keep fused multiply-adds.
 #include <atomic>

@@ -77,7 +77,7 @@ __host__ __device__ constexpr int rad_stride(int br) {
 // Launchers of the kernels compiled without implicit fused multiply-adds
 // (green_series.cu): the EIGENE (br = 2) and PIDCOCK (br = 1) branches, whose
 // epsilon-extrapolated series must see the same operation sequence as the
-// CPU checker, their radial tables (from the distances ur, or from the pairs
+// CPU oracle, their radial tables (from the distances ur, or from the pairs
 // of the list where ur is null), the distances themselves, the per-frequency
 // mode tables, and the batch evaluator.
 void launch_green_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,

@@ -139,7 +139,7 @@ static __constant__ SeriesConsts c_series = SeriesConsts();
 // K0(x), K1(x), IK01A (FinGrnExtSubs.f90:538-635).  K0/K1 feed the
 // epsilon-accelerated series, whose result moves with the last bit of its
 // inputs, so this routine uses the bit-reproducible exp/log of detmath.h and
-// the operation order of the CPU checker; the kernels that call it for the
+// the operation order of the CPU oracle; the kernels that call it for the
 // EIGENE/PIDCOCK series are compiled without implicit fused multiply-adds.
 // The reference compares the K0 series against a value it never initialised
 // on the first pass; zero is used, which cannot stop the series early.
