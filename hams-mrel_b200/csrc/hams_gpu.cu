@@ -2856,6 +2856,7 @@ static int field_context(hams_ctx* c, hams_ctx* of) {
   c->launches += f->launches.load();
   c->lib_calls += f->lib_calls.load();
   if (rc < 0) {
+    cudaStreamSynchronize(f->st);  // a kernel of the set may still write the buffers that go back
     field_free(f);
     if (rc != HAMS_ERR_NOMEM) return rc;
     g_err.clear();

@@ -1,0 +1,43 @@
+"""Calls that find too little device memory for what only saves time: they take the slower way, give the
+same results and leave no buffer to others while a kernel still writes it."""
+import pytest
+
+import short_memory
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def so(tmp_path_factory):
+    return short_memory.build(str(tmp_path_factory.mktemp("short")))
+
+
+def test_field_points_left_out_pair_set_is_idle_when_given_back(so):
+    """Infinite depth: the points' Rankine tables are being filled when the allocation of their influences
+    fails; the stream is waited for before the tables go back to the cache."""
+    got = short_memory.run(so, """
+geom = deck([meshgen.cylinder(5.0, 10.0, 18, 9, 4)])
+n, m, beta = 234, 20000, [0.3]
+rng = np.random.default_rng(1)
+p = np.column_stack([rng.uniform(8.0, 40.0, m), rng.uniform(-30.0, 30.0, m), -rng.uniform(0.5, 30.0, m)])
+want = None
+for short in (False, True):
+    ctx = hams_b200.Context(geom, -1.0, rho=1025.0, g=9.81)
+    w = ctx.wave(0.9)
+    mem.short_memory_reset()
+    if short:
+        hams_b200.release_cached()
+        mem.short_memory_limit(mem.short_memory_used() + (16 + 8) * n * m)
+    ctx.set_field_points(p)
+    calls, refused = log(), mem.short_memory_refused()
+    mem.short_memory_limit(0)
+    ctx.solve_frequency(w, beta)
+    pot = ctx.field_potentials(1)
+    if want is None: want = pot
+    ctx.close()
+answer(refused=refused, after=calls[calls.rindex("x") + 1:], err=rel(pot, want))
+""")
+    assert got["refused"] == 2  # the allocation and its repetition
+    after = got["after"]
+    assert "S" in after and (after.find("G") < 0 or after.find("S") < after.find("G")), after
+    assert got["err"] < 1e-12  # the same influences from k_field_pairs, their sums of 234 terms in another order
