@@ -2502,15 +2502,19 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
   TRY(c->gpiv.alloc(n));
   bool inv = nb > 1;
   for (int b = 0; b < nb && inv; ++b) inv = c->body_nelem[b] > 0 && zlu_supported(c->body_nelem[b]) == 0;
-  inv = inv && c->gblk.alloc(boff[nb]) == 0 && c->gtmp.alloc((size_t)n * nrhs) == 0;
+  TRY(c->gpre.alloc(nb > 1 ? boff[nb] : (size_t)n));  // either way needs it
+  if (inv && (c->gblk.alloc(boff[nb]) || c->gtmp.alloc((size_t)n * nrhs))) {
+    inv = false;
+    g_err.clear();
+    c->gblk.release();
+    c->gtmp.release();
+  }
   if (nb == 1) {
-    TRY(c->gpre.alloc(n));
     k_jacobi_setup<<<(n + 255) / 256, 256, 0, c->st>>>(M, n, c->gpre.p);
     TRY(launch_check(c));
   } else if (inv) {
     // runs of bodies of one size: identity right-hand sides in gpre, the blocks
     // and their factors in gblk
-    TRY(c->gpre.alloc(boff[nb]));
     TRY(c->zwork.alloc(zlu_work_ints(nb)));
     for (int b = 0, e = 0; b < nb; b = e) {
       const int nn = c->body_nelem[b];
@@ -2530,7 +2534,6 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
       TRY(launch_check(c));
     }
   } else {
-    TRY(c->gpre.alloc(boff[nb]));
     int lwmax = 0;
     for (int b = 0; b < nb; ++b) {
       const int nn = c->body_nelem[b];

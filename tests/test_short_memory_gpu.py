@@ -41,3 +41,39 @@ answer(refused=refused, after=calls[calls.rindex("x") + 1:], err=rel(pot, want))
     after = got["after"]
     assert "S" in after and (after.find("G") < 0 or after.find("S") < after.find("G")), after
     assert got["err"] < 1e-12  # the same influences from k_field_pairs, their sums of 234 terms in another order
+
+
+@pytest.mark.parametrize("without", ["second block", "copy of the right-hand sides"])
+def test_gmres_without_its_second_block(so, without):
+    """Memory for everything but the second set of body blocks, or but the copy of the right-hand sides
+    beside it: the library's factors, as where no inverse is formed.  Tolerance 1e-11 on the preconditioned
+    residual, systems of condition below 1e3: 1e-8."""
+    got = short_memory.run(so, f"without = {without!r}" + """
+geom = deck([meshgen.cylinder(5.0, 8.0, 24, 9, 4, 30.0 * k, 0.0) for k in range(3)])
+n, nn, nrhs = 936, 312, 19
+kw = dict(rho=1025.0, g=9.81, solver=hams_b200.SOLVER_GMRES, gmres_restart=40, gmres_maxit=400, gmres_tol=1e-11,
+          gmres_dense=1)
+w, beta = hams_b200.wave_properties(0.9, -1.0, 9.81), [0.3]
+ctx = hams_b200.Context(geom, -1.0, **kw)
+want = ctx.solve_frequency(w, beta)
+ctx.close()
+hams_b200.release_cached()
+mem.short_memory_reset()
+ctx = hams_b200.Context(geom, -1.0, **kw)
+ctx.solve_frequency(w, beta)
+peak = mem.short_memory_peak()
+ctx.close()
+hams_b200.release_cached()
+ctx = hams_b200.Context(geom, -1.0, **kw)
+block = (16 * 3 * nn * nn + (1 << 21) - 1 >> 21) << 21
+tmp = (16 * n * nrhs + 255) // 256 * 256
+mem.short_memory_reset()
+mem.short_memory_limit(peak - (block if without == "second block" else tmp))
+got = ctx.solve_frequency(w, beta)
+again = ctx.solve_frequency(w, beta)
+lib = hams_b200.load_library()
+lib.hams_last_error.restype = ctypes.c_char_p
+answer(refused=mem.short_memory_refused(), err=max(rel(a, b) for a, b in zip(got, want)), msg=lib.hams_last_error().decode(),
+       same=all(np.array_equal(a, b) for a, b in zip(got, again)))
+""")
+    assert got["refused"] > 0 and got["err"] < 1e-8 and got["same"] and got["msg"] == ""
