@@ -2425,6 +2425,13 @@ static int mixed_solve(hams_ctx* c, double2* M, const double2* rhs, int ldr, int
   return mixed_refine(c, M, rhs, ldr, nrhs);
 }
 
+// Most panels of a body whose block GMRES inverts.  An inverse takes four times
+// the operations of the factors and saves every step their triangular solves: two
+// bodies in infinite depth, five steps, factors against inverses 38.8 / 13.5 ms at
+// 1,600 panels each, 101.9 / 59.2 at 3,600, 146.8 / 114.2 at 4,800 (where two steps
+// make it even), 203.0 / 200.0 at 6,000, 308.9 / 411.3 at 7,920.
+constexpr int kInvRows = 5000;
+
 // GMRES (IterativeSolvers.f90:324-484, ZGMRES_SOLVE): X (n x nrhs) from the
 // FP64 matrix M and the right-hand sides rhs, every column from zero,
 // restarted every m steps, right-preconditioned by the LU factors of each
@@ -2487,12 +2494,11 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
   };
   // preconditioner: the inverse of each body's diagonal block by LU, packed one
   // after another (bodies of one size factored together), the library's LU
-  // factors where a body is too large for the own one or memory is short, or
+  // factors where a body has more than kInvRows panels or memory is short, or
   // the diagonal of M with one body.  A step is then one GEMM per run of
   // bodies, which reads the inverses once; the triangular solves with the
-  // factors were bound by their chains.  Four bodies of 600 panels: setting up
-  // 7.3 -> 2.3 ms, a step's products 3.3 -> 0.05 ms, the frequency 30.7 -> 11.3 ms.
-  // Two bodies of 4,100 panels: setting up 49 -> 67 ms, the whole solution 106 -> 76 ms.
+  // factors were bound by their chains.  Four bodies of 600 panels in 40 m: setting
+  // up 7.3 -> 2.3 ms, a step's products 3.3 -> 0.05 ms.
   std::vector<size_t> boff(nb + 1, 0);
   std::vector<int> bst(nb + 1, 0);
   for (int b = 0; b < nb; ++b) {
@@ -2501,7 +2507,8 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
   }
   TRY(c->gpiv.alloc(n));
   bool inv = nb > 1;
-  for (int b = 0; b < nb && inv; ++b) inv = c->body_nelem[b] > 0 && zlu_supported(c->body_nelem[b]) == 0;
+  for (int b = 0; b < nb && inv; ++b)
+    inv = c->body_nelem[b] > 0 && c->body_nelem[b] <= kInvRows && zlu_supported(c->body_nelem[b]) == 0;
   TRY(c->gpre.alloc(nb > 1 ? boff[nb] : (size_t)n));  // either way needs it
   if (inv && (c->gblk.alloc(boff[nb]) || c->gtmp.alloc((size_t)n * nrhs))) {
     inv = false;
