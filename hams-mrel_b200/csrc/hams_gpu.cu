@@ -1397,6 +1397,8 @@ constexpr int kNtCut[2][2] = {{26, 38}, {66, 82}};
 // of A), and the table bytes of a chunk of pairs where distances are not
 // numbered: small enough to stay in L2 between the two kernels.
 constexpr size_t kRadMin = (size_t)64 << 20;
+constexpr long long kRadLeast = 512;  // pairs of a chunk at least, where memory is short
+constexpr long long kLinChunk = 65536;  // LINTON pairs of a chunk without row numbers: 3 MB
 
 // The distinct distances of the series bins (RadTab): the pairs' distances
 // sorted, numbered where they change, the numbers scattered back to the
@@ -1445,7 +1447,11 @@ static int build_distances(hams_ctx* c) {
   CU(cudaMemcpyAsync(&nu, rank.p + ns - 1, 4, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
   c->ur.release(true);
-  TRY(c->ur.alloc(nu));
+  if (c->ur.alloc(nu)) {
+    g_err.clear();
+    c->rid.release(true);
+    return 0;
+  }
   for (int q = 0; q < 8; ++q) l[q] = q % 2 ? 0u : 0xffffffffu;
   CU(cudaMemcpyAsync(lim.p, l, sizeof l, cudaMemcpyHostToDevice, c->st));
   k_distance_rows<<<nb, 256, 0, c->st>>>(r2.p, idx2.p, rank.p, ns, c->bin_off[2] - o1, c->bin_off[3] - o1,
@@ -1458,12 +1464,18 @@ static int build_distances(hams_ctx* c) {
   r2.release(true);
   tbuf.release(true);
   const size_t cap = std::max(kRadMin, (size_t)c->tn * c->n * 8);
+  bool numbered = false;
   for (int br = 1; br < 4; ++br) {
     if (l[2 * br] > l[2 * br + 1]) continue;  // no pair
     const uint32_t n = l[2 * br + 1] - l[2 * br] + 1;
     if ((size_t)n * rad_stride(br) * 8 > cap) continue;
     c->rad_base[br] = l[2 * br];
     c->rad_n[br] = n;
+    numbered = true;
+  }
+  if (!numbered) {
+    c->rid.release(true);
+    c->ur.release(true);
   }
   return 0;
 }
@@ -1497,7 +1509,11 @@ static int build_linton_rows(hams_ctx* c) {
   uint32_t rows = 0;
   CU(cudaMemcpyAsync(&rows, rank.p + n - 1, 4, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
-  TRY(c->lrep.alloc(rows));
+  if (c->lrep.alloc(rows)) {
+    g_err.clear();
+    c->lrow.release();
+    return 0;
+  }
   k_linton_file<<<nb, 256, 0, c->st>>>(idx2.p, rank.p, n, c->lrow.p, c->lrep.p);
   TRY(launch_check(c, 3));
   CU(cudaStreamSynchronize(c->st));
@@ -1666,17 +1682,27 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
   return 0;
 }
 
-static int rad_buffers(hams_ctx* c) {
-  if (c->bin_off[1] > 0) TRY(c->lin_fg.alloc(3 * (size_t)c->lin_rows));
+// The tables of the numbered distances and LINTON rows.  A branch that they do
+// not fit for goes without numbers in this context: its pairs' own rows, a chunk
+// of pairs at a time (series_pairs, linton_bin).
+static void rad_buffers(hams_ctx* c) {
+  if (c->lrow.p && c->lin_fg.alloc(3 * (size_t)c->lin_rows)) {
+    c->lrow.release(true);
+    c->lrep.release(true);
+    c->lin_rows = c->bin_off[1];
+    g_err.clear();
+  }
   for (int br = 1; br < 4; ++br)
-    if (c->rad_n[br]) {
-      TRY(c->rad_k[br].alloc((size_t)c->rad_n[br] * rad_stride(br)));
-      TRY(c->rad_j[br].alloc(c->rad_n[br]));
+    if (c->rad_n[br] &&
+        (c->rad_k[br].alloc((size_t)c->rad_n[br] * rad_stride(br)) || c->rad_j[br].alloc(c->rad_n[br]))) {
+      c->rad_k[br].release(true);
+      c->rad_j[br].release(true);
+      c->rad_n[br] = 0;
+      g_err.clear();
     }
-  return 0;
 }
 
-// Mode and radial tables and LINTON rows of one frequency in flight.
+// Mode tables of one frequency in flight.
 static int mode_buffers(hams_ctx* c) {
   const int n = c->n, tn = c->tn;
   const size_t km = hams::kModeMax;
@@ -1687,7 +1713,6 @@ static int mode_buffers(hams_ctx* c) {
   int nmode = 11;
   if (c->bin_off[3] > c->bin_off[2] || c->bin_off[5] > c->bin_off[4]) nmode = hams::kEigenEMax + 1;
   if (c->bin_off[2] > c->bin_off[1]) nmode = hams::kPidcockMax + 1;
-  TRY(rad_buffers(c));
   c->mt = hams::ModeTab{n, tn, nmode, c->mt_pm.p, c->mt_ac.p, c->mt_src.p, c->mt_srct.p, c->mt_fld.p, c->mt_fldt.p};
   return 0;
 }
@@ -1703,6 +1728,7 @@ static int ctx_frequency_buffers(hams_ctx* c) {
   TRY(c->ovf.alloc(1));
   TRY(c->ipiv.alloc(n));
   TRY(c->info.alloc(2));  // the solver's info word and the tensor-core kernels' error word
+  if (c->opts.depth >= 0.0) rad_buffers(c);
   return 0;
 }
 
@@ -2076,9 +2102,12 @@ static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* 
   }
   // a row per pair, a chunk of pairs at a time; c->rad_k may hold the table
   // of the numbered distances, which is then filled again
-  const long long per = std::min<long long>(cnt, kRadMin / (rad_stride(br) * 8));
-  TRY(c->rad_k[br].alloc((size_t)per * rad_stride(br)));
-  TRY(c->rad_j[br].alloc(per));
+  long long per = std::min<long long>(cnt, kRadMin / (rad_stride(br) * 8));
+  while (c->rad_k[br].alloc((size_t)per * rad_stride(br)) || c->rad_j[br].alloc(per)) {
+    if (per <= kRadLeast) return HAMS_ERR_NOMEM;
+    per /= 2;
+    g_err.clear();
+  }
   c->rad_ready[br] = false;
   for (long long t = 0; t < cnt; t += per) {
     const long long n = std::min(per, cnt - t);
@@ -2094,24 +2123,34 @@ static int series_bin(hams_ctx* c, const WaveDev& wd, int b) {
                       b);
 }
 
-// The LINTON pairs (bin 0): their rows, then A and S.
+// The LINTON pairs (bin 0): their rows, then A and S; without row numbers a
+// chunk of pairs at a time, each pair its own row.
 static int linton_bin(hams_ctx* c, const WaveDev& wd) {
   const long long cnt = c->bin_off[1];
   if (cnt <= 0) return 0;
-  const long long rows = c->lin_rows;
-  if (!wd.limit) {
-    if (rows < (long long)c->sms * kLintonRowsPerSm)
-      k_linton_rows<<<(unsigned)rows, 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p, c->lrep.p, c->lin_fg.p,
-                                                       c->ovf.p);
-    else
-      k_linton_rows_threads<<<(unsigned)((rows + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, c->pairs.p,
-                                                                               c->lrep.p, rows, c->lin_fg.p,
-                                                                               c->ovf.p);
+  const bool numbered = c->lrow.p != nullptr;
+  long long per = numbered || wd.limit ? cnt : std::min(cnt, kLinChunk);
+  while (!numbered && !wd.limit && c->lin_fg.alloc(3 * (size_t)per)) {
+    if (per <= kRadLeast) return HAMS_ERR_NOMEM;
+    per /= 2;
+    g_err.clear();
+  }
+  for (long long t = 0; t < cnt; t += per) {
+    const long long n = std::min(per, cnt - t), rows = numbered ? c->lin_rows : n;
+    const uint32_t* lst = c->pairs.p + t;
+    if (!wd.limit) {
+      if (rows < (long long)c->sms * kLintonRowsPerSm)
+        k_linton_rows<<<(unsigned)rows, 128, 0, c->st>>>(c->g, wd, c->wvn.p, lst, c->lrep.p, c->lin_fg.p, c->ovf.p);
+      else
+        k_linton_rows_threads<<<(unsigned)((rows + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, lst, c->lrep.p,
+                                                                                 rows, c->lin_fg.p, c->ovf.p);
+      TRY(launch_check(c));
+    }
+    k_linton_pairs<<<(unsigned)((n + 127) / 128), 128, 0, c->st>>>(c->g, wd, lst, c->lrow.p, n, c->lin_fg.p, c->rs.p,
+                                                                   c->rd.p, c->A.p, c->S.p);
     TRY(launch_check(c));
   }
-  k_linton_pairs<<<(unsigned)((cnt + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->pairs.p, c->lrow.p, cnt,
-                                                                   c->lin_fg.p, c->rs.p, c->rd.p, c->A.p, c->S.p);
-  return launch_check(c);
+  return 0;
 }
 
 // The far pairs (bins 4 and 5 of k_pair_keys) from the series: EIGENE and
@@ -2838,7 +2877,9 @@ static int field_setup(hams_ctx* f, hams_ctx* of) {
   }
   if (f->opts.depth >= 0.0) TRY(mode_buffers(f));
   TRY(f->A.alloc(np));
-  return f->S.alloc(np);
+  TRY(f->S.alloc(np));
+  if (f->opts.depth >= 0.0) rad_buffers(f);
+  return 0;
 }
 // c's pair set for its field points; the caller's stream c->st is idle.  Left
 // out (k_field_pairs takes over) where the pairs exceed the 32-bit index or
@@ -3508,7 +3549,7 @@ extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t 
     c->sg_on = 0;
   }
   TRY(build_pairs(c));
-  TRY(rad_buffers(c));
+  rad_buffers(c);
   TRY(build_judge_samples(c));
   if (c->sg_on) {
     TRY(c->sg_map.alloc((size_t)c->tn * c->n));
@@ -3520,7 +3561,7 @@ extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t 
   c->mt.nmode = nmode;
   for (hams_ctx* l : c->lanes) {
     view_pairs(l, c);
-    TRY(rad_buffers(l));
+    rad_buffers(l);
     l->sg_on = c->sg_on;
     l->sg_far = c->sg_far;
     l->sg_kmin = c->sg_kmin;

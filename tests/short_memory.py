@@ -110,7 +110,7 @@ def build(folder):
 def run(so, script, timeout=300):
     """What `script` (after PRELUDE, in a process of its own with the stand-in) hands to answer()."""
     here = os.path.dirname(os.path.abspath(__file__))
-    path = [here, os.path.join(os.path.dirname(here), "hams-mrel_b200")]
+    path = [here] + [os.path.join(os.path.dirname(here), d) for d in ("hams-mrel_b200", "oracle")]
     p = subprocess.run([sys.executable, "-c", PRELUDE + script], capture_output=True, text=True, timeout=timeout,
                        env=dict(os.environ, LD_PRELOAD=so, SHORT_MEMORY_PATH=json.dumps(path)))
     lines = [x for x in p.stdout.splitlines() if x.startswith("ANSWER ")]

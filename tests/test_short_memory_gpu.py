@@ -77,3 +77,55 @@ answer(refused=mem.short_memory_refused(), err=max(rel(a, b) for a, b in zip(got
        same=all(np.array_equal(a, b) for a, b in zip(got, again)))
 """)
     assert got["refused"] > 0 and got["err"] < 1e-8 and got["same"] and got["msg"] == ""
+
+
+ROUGH = """
+import test_series
+geom = deck(test_series._rough([meshgen.cylinder(4.0, 6.0, 20, 5, 3)], 0.02, 1))
+beta, size = [0.3, 1.1], 1 << 20  # size: far below the tables of its 25,600 distances
+waves = [hams_b200.wave_properties(v, 45.0, 9.81) for v in (0.6, 1.3)]
+def live():
+    hams_b200.release_cached()
+    return mem.short_memory_used()
+"""
+
+
+def test_context_without_its_radial_tables(so):
+    """A table of the distinct distances that does not fit leaves its branch to the pairs' own rows: the
+    same numbers, the same operations, the same bits."""
+    got = short_memory.run(so, ROUGH + """
+def assembled(limit):
+    live()
+    mem.short_memory_limit(limit)
+    ctx = hams_b200.Context(geom, 45.0, rho=1025.0, g=9.81)
+    mem.short_memory_limit(0)
+    held = live()
+    out = [x.copy() for w in waves for x in ctx.assemble(w, beta)]
+    ctx.close()
+    return out, held
+want, held = assembled(0)
+got, less = assembled(held - size)
+answer(less=held - less, same=all(np.array_equal(a, b) for a, b in zip(got, want)))
+""")
+    assert got["less"] >= 1 << 20 and got["same"]
+
+
+def test_batch_lane_without_its_radial_tables(so):
+    """The lane of a batch's second frequency finds no room for the tables that its context has."""
+    got = short_memory.run(so, ROUGH + """
+def batch(limit):
+    live()
+    ctx = hams_b200.Context(geom, 45.0, rho=1025.0, g=9.81, batch_lanes=2)
+    ctx.solve_frequency(waves[0], beta)
+    live()
+    mem.short_memory_limit(limit)
+    out = ctx.solve_batch(waves, beta)
+    mem.short_memory_limit(0)
+    held = live()
+    ctx.close()
+    return out, held
+want, held = batch(0)
+got, less = batch(held - size)
+answer(less=held - less, same=all(np.array_equal(a, b) for a, b in zip(got, want)))
+""")
+    assert got["less"] >= 1 << 20 and got["same"]
