@@ -1080,6 +1080,19 @@ std::map<int, Dev> devs;
 
 inline size_t round_bytes(size_t b) { return b < (1u << 20) ? (b + 255) / 256 * 256 : (b + (2u << 20) - 1) / (2u << 20) * (2u << 20); }
 
+// The current device's cached blocks back to the driver; the bytes freed.
+size_t drop() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  Dev& d = devs[dev];
+  const size_t had = d.cached;
+  for (auto& f : d.free) cudaFree(f.second);
+  d.free.clear();
+  d.cached = 0;
+  return had;
+}
+
 void* take(size_t bytes) {
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1098,13 +1111,7 @@ void* take(size_t bytes) {
   void* p = nullptr;
   if (cudaMalloc(&p, want) == cudaSuccess) return p;
   cudaGetLastError();
-  {  // out of memory: give the cached blocks back and try once more
-    std::lock_guard<std::mutex> lock(mu);
-    Dev& d = devs[dev];
-    for (auto& f : d.free) cudaFree(f.second);
-    d.free.clear();
-    d.cached = 0;
-  }
+  drop();  // out of memory: give the cached blocks back and try once more
   p = nullptr;
   if (cudaMalloc(&p, want) == cudaSuccess) return p;
   cudaGetLastError();
@@ -1202,6 +1209,7 @@ struct hams_ctx {
   // the points' pair set: a context whose field points are fp_x, with this
   // one's sources and stream (field_context); A and S hold the influences
   hams_ctx* field = nullptr;
+  bool lean = false;  // memory ran short: none of what only saves time (shed)
   std::vector<double> fp_last;
   std::vector<std::vector<double>> fp_batch;
   bool hm_ready = false;      // GMRES: cluster tree uploaded to hm
@@ -1390,6 +1398,49 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
 static int ctx_frequency_buffers(hams_ctx* c);
 static int field_context(hams_ctx* c, hams_ctx* of);
 
+// A call that runs out of memory must not do so for what only saves time.  shed
+// gives that back, of c and of its lanes (none of them in use), with the cached
+// blocks: distance numbers and radial tables, LINTON rows, the field points' pair
+// set, GMRES's second blocks.  The context goes without them from then on; false
+// if there was nothing to give.
+static bool shed(hams_ctx* c) {
+  cudaGetLastError();  // of an allocation outside the cache
+  const bool first = !c->lean;
+  std::vector<hams_ctx*> all = c->lanes;  // the views before what they show
+  all.push_back(c);
+  for (hams_ctx* x : all)
+    if (x->st) cudaStreamSynchronize(x->st);
+  for (hams_ctx* x : all) {
+    x->lean = true;
+    field_free(x->field);
+    x->field = nullptr;
+    for (DBuf<uint32_t>* d : {&x->rid, &x->lrow, &x->lrep}) d->release(true);
+    x->ur.release(true);
+    x->lin_fg.release(true);
+    x->lin_rows = x->bin_off[1];
+    for (int br = 0; br < 4; ++br) {
+      x->rad_n[br] = 0;
+      x->rad_k[br].release(true);
+      x->rad_j[br].release(true);
+    }
+    x->gblk.release(true);
+    x->gtmp.release(true);
+  }
+  return devcache::drop() > 0 || first;
+}
+
+// f(), once more without what c can do without where it ran out of memory.
+template <class F>
+static int with_memory(hams_ctx* c, const F& f) {
+  int rc = f();
+  if (rc == HAMS_ERR_NOMEM && shed(c)) {
+    g_err.clear();
+    rc = f();
+    if (rc == HAMS_ERR_NOMEM) cudaGetLastError();
+  }
+  return rc;
+}
+
 // Series lengths (EIGENE, then PIDCOCK) at which a bin's launch is split, so
 // that its shared memory fits the lengths it holds (launch_series).
 constexpr int kNtCut[2][2] = {{26, 38}, {66, 82}};
@@ -1397,8 +1448,10 @@ constexpr int kNtCut[2][2] = {{26, 38}, {66, 82}};
 // of A), and the table bytes of a chunk of pairs where distances are not
 // numbered: small enough to stay in L2 between the two kernels.
 constexpr size_t kRadMin = (size_t)64 << 20;
-constexpr long long kRadLeast = 512;  // pairs of a chunk at least, where memory is short
 constexpr long long kLinChunk = 65536;  // LINTON pairs of a chunk without row numbers: 3 MB
+// Both where memory ran short (shed), and the fewest pairs of a chunk.
+constexpr size_t kRadLean = (size_t)2 << 20;
+constexpr long long kLinLean = 4096, kRadLeast = 512;
 
 // The distinct distances of the series bins (RadTab): the pairs' distances
 // sorted, numbered where they change, the numbers scattered back to the
@@ -1408,7 +1461,7 @@ static int build_distances(hams_ctx* c) {
   const long long o1 = c->bin_off[1], ns = c->bin_off[6] - o1;
   for (int br = 0; br < 4; ++br) c->rad_base[br] = c->rad_n[br] = 0;
   c->rid.release(true);
-  if (ns <= 0) return 0;
+  if (ns <= 0 || c->lean) return 0;
   DBuf<double> r, r2;
   DBuf<uint32_t> idx, idx2, rank, lim;
   // without the memory for the sort, every pair has its own row
@@ -1486,7 +1539,7 @@ static int build_linton_rows(hams_ctx* c) {
   c->lrow.release(true);
   c->lrep.release(true);
   c->lin_rows = n;
-  if (n <= 0) return 0;
+  if (n <= 0 || c->lean) return 0;
   DBuf<unsigned long long> key, key2;
   DBuf<uint32_t> idx, idx2, rank;
   DBuf<char> tbuf;
@@ -1677,7 +1730,7 @@ static int ctx_setup(hams_ctx* c, const hams_geom* geo) {
   CU(cudaMemcpyAsync(c->chunks.p, c->chunks_h.data(), c->chunks_h.size() * sizeof(int2), cudaMemcpyHostToDevice, c->st));
   CU(cudaMemcpyAsync(c->bchunk.p, cb.data(), cb.size() * sizeof(int), cudaMemcpyHostToDevice, c->st));
 
-  TRY(ctx_frequency_buffers(c));
+  TRY(with_memory(c, [&] { return ctx_frequency_buffers(c); }));
   CU(cudaStreamSynchronize(c->st));
   return 0;
 }
@@ -1836,6 +1889,7 @@ static void view_pairs(hams_ctx* l, hams_ctx* c) {
   l->lrow.view(c->lrow);
   l->lrep.view(c->lrep);
   l->lin_rows = c->lin_rows;
+  l->lean = c->lean;
   for (int br = 0; br < 4; ++br) l->rad_base[br] = c->rad_base[br], l->rad_n[br] = c->rad_n[br];
   for (int b = 0; b < kBins; ++b) l->nt_cut[b][0] = c->nt_cut[b][0], l->nt_cut[b][1] = c->nt_cut[b][1];
 }
@@ -2028,8 +2082,12 @@ extern "C" int hams_ctx_create(const hams_geom* geo, const hams_opts* opts, hams
     // once per device and process)
     std::vector<int> shapes;
     mixed_lu_gemm_shapes(c->n, shapes);
-    if (gemm_tf32_autotune(c->st, (int)shapes.size() / 3, shapes.data()))
-      rc = fail(HAMS_ERR_CUDA, "GEMM autotuner failed: %s", cudaGetErrorString(cudaGetLastError()));
+    rc = with_memory(c, [&] {
+      if (!gemm_tf32_autotune(c->st, (int)shapes.size() / 3, shapes.data())) return 0;
+      const cudaError_t e = cudaGetLastError();
+      return fail(e == cudaErrorMemoryAllocation ? HAMS_ERR_NOMEM : HAMS_ERR_CUDA, "GEMM autotuner failed: %s",
+                  cudaGetErrorString(e));
+    });
   }
   if (rc < 0) {
     std::string keep = g_err;
@@ -2102,7 +2160,7 @@ static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* 
   }
   // a row per pair, a chunk of pairs at a time; c->rad_k may hold the table
   // of the numbered distances, which is then filled again
-  long long per = std::min<long long>(cnt, kRadMin / (rad_stride(br) * 8));
+  long long per = std::min<long long>(cnt, (c->lean ? kRadLean : kRadMin) / (rad_stride(br) * 8));
   while (c->rad_k[br].alloc((size_t)per * rad_stride(br)) || c->rad_j[br].alloc(per)) {
     if (per <= kRadLeast) return HAMS_ERR_NOMEM;
     per /= 2;
@@ -2129,7 +2187,7 @@ static int linton_bin(hams_ctx* c, const WaveDev& wd) {
   const long long cnt = c->bin_off[1];
   if (cnt <= 0) return 0;
   const bool numbered = c->lrow.p != nullptr;
-  long long per = numbered || wd.limit ? cnt : std::min(cnt, kLinChunk);
+  long long per = numbered || wd.limit ? cnt : std::min(cnt, c->lean ? kLinLean : kLinChunk);
   while (!numbered && !wd.limit && c->lin_fg.alloc(3 * (size_t)per)) {
     if (per <= kRadLeast) return HAMS_ERR_NOMEM;
     per /= 2;
@@ -2545,7 +2603,7 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
     boff[b + 1] = boff[b] + (size_t)c->body_nelem[b] * c->body_nelem[b];
   }
   TRY(c->gpiv.alloc(n));
-  bool inv = nb > 1;
+  bool inv = nb > 1 && !c->lean;
   for (int b = 0; b < nb && inv; ++b)
     inv = c->body_nelem[b] > 0 && c->body_nelem[b] <= kInvRows && zlu_supported(c->body_nelem[b]) == 0;
   TRY(c->gpre.alloc(nb > 1 ? boff[nb] : (size_t)n));  // either way needs it
@@ -2887,7 +2945,7 @@ static int field_setup(hams_ctx* f, hams_ctx* of) {
 static int field_context(hams_ctx* c, hams_ctx* of) {
   field_free(c->field);
   c->field = nullptr;
-  if (c->nfp <= 0 || (size_t)c->nfp * c->n > 0xffffffffull) return 0;
+  if (c->nfp <= 0 || c->lean || (size_t)c->nfp * c->n > 0xffffffffull) return 0;
   hams_ctx* f = new hams_ctx();
   f->is_lane = true;
   f->opts = c->opts;
@@ -3180,7 +3238,7 @@ extern "C" int hams_solve_frequency(hams_ctx* c, const hams_wave* w, int32_t nbe
   g_err.clear();
   if (!c || !w || (nbeta > 0 && !beta)) return fail(HAMS_ERR_ARG, "null argument");
   if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
-  return solve_one(c, w, nbeta, beta, amas, bdmp, exfc);
+  return with_memory(c, [&] { return solve_one(c, w, nbeta, beta, amas, bdmp, exfc); });
 }
 
 // Frequencies in flight at once in hams_solve_batch when opts.batch_lanes is 0.
@@ -3197,7 +3255,7 @@ extern "C" int hams_solve_batch(hams_ctx* c, int32_t nfreq, const hams_wave* wav
   L = std::max(1, std::min(L, nfreq));
   while ((int)c->lanes.size() < L - 1) {
     hams_ctx* l = nullptr;
-    TRY(make_lane(c, &l));
+    TRY(with_memory(c, [&] { return make_lane(c, &l); }));
     c->lanes.push_back(l);
   }
   std::vector<hams_ctx*> lane{c};
@@ -3238,30 +3296,32 @@ extern "C" int hams_solve_batch(hams_ctx* c, int32_t nfreq, const hams_wave* wav
         }
     }
   };
-  std::vector<std::thread> th;
-  for (int t = 1; t < L; ++t) th.emplace_back(run, t);
-  run(0);
-  for (auto& x : th) x.join();
+  auto run_all = [&]() -> int {
+    next = 0;
+    lane_rc.assign(L, 0);
+    std::vector<std::thread> th;
+    for (int t = 1; t < L; ++t) th.emplace_back(run, t);
+    run(0);
+    for (auto& x : th) x.join();
+    for (int t = 0; t < L; ++t)
+      if (lane_rc[t] < 0) {
+        g_err = lane_err[t];
+        return lane_rc[t];
+      }
+    return 0;
+  };
+  const int rc = with_memory(c, run_all);
   c->note.clear();  // the batch's note: each frequency's own, in order
   for (int k = 0; k < nfreq; ++k)
     if (!note_of[k].empty()) c->note += (c->note.empty() ? "" : "; ") + ("frequency " + std::to_string(k) + ": ") + note_of[k];
-  for (int t = 0; t < L; ++t)
-    if (lane_rc[t] < 0) {
-      g_err = lane_err[t];
-      return lane_rc[t];
-    }
+  if (rc < 0) return rc;
   for (int k = 0; k < nfreq; ++k)
     if (rc_of[k] > 0) return rc_of[k];  // singular pivot of the first such frequency
   return 0;
 }
 
-extern "C" int hams_assemble(hams_ctx* c, const hams_wave* w, int32_t nbeta, const double* beta, double* amat,
-                             double* brmat, double* bdmat) {
-  g_err.clear();
-  if (!c || !w || (nbeta > 0 && !beta)) return fail(HAMS_ERR_ARG, "null argument");
-  if (c->unfolded)
-    return fail(HAMS_ERR_UNSUPPORTED, "hams_assemble: the context holds the unfolded mesh of a half-mesh deck");
-  if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
+static int assemble_one(hams_ctx* c, const hams_wave* w, int32_t nbeta, const double* beta, double* amat,
+                        double* brmat, double* bdmat) {
   const int n = c->n, tn = c->tn, ndof = 6 * c->nb, nrhs = ndof + nbeta;
   TRY(c->beta.alloc(std::max(nbeta, 1)));
   if (nbeta > 0) CU(cudaMemcpyAsync(c->beta.p, beta, (size_t)nbeta * 8, cudaMemcpyHostToDevice, c->st));
@@ -3288,6 +3348,16 @@ extern "C" int hams_assemble(hams_ctx* c, const hams_wave* w, int32_t nbeta, con
                          cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
   return 0;
+}
+
+extern "C" int hams_assemble(hams_ctx* c, const hams_wave* w, int32_t nbeta, const double* beta, double* amat,
+                             double* brmat, double* bdmat) {
+  g_err.clear();
+  if (!c || !w || (nbeta > 0 && !beta)) return fail(HAMS_ERR_ARG, "null argument");
+  if (c->unfolded)
+    return fail(HAMS_ERR_UNSUPPORTED, "hams_assemble: the context holds the unfolded mesh of a half-mesh deck");
+  if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
+  return with_memory(c, [&] { return assemble_one(c, w, nbeta, beta, amat, brmat, bdmat); });
 }
 
 // The points of hams_eval_green at a regular frequency in finite depth, branch
@@ -3395,7 +3465,7 @@ extern "C" int hams_eval_green(hams_ctx* c, const hams_wave* w, int32_t npts, co
     CU(cudaMemcpyAsync(&ovf, c->ovf.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
     return 0;
   };
-  TRY(done(run()));
+  TRY(with_memory(c, [&] { return done(run()); }));
   if (ovf) return fail(HAMS_ERR_NUMERIC, "adaptive quadrature stack overflow in the LINTON branch");
   return 0;
 }
@@ -3516,14 +3586,7 @@ static int build_judge_samples(hams_ctx* c) {
   return 0;
 }
 
-extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t nparams, double far_factor) {
-  g_err.clear();
-  if (!c || c->is_lane) return fail(HAMS_ERR_ARG, "null context");
-  if (params && nparams != sg::kParams)
-    return fail(HAMS_ERR_ARG, "surrogate parameter vector has %d floats, %d expected", nparams, sg::kParams);
-  if (params && !(far_factor > 0.0)) return fail(HAMS_ERR_ARG, "far_factor must be positive");
-  if (c->opts.depth < 0.0 && params) return fail(HAMS_ERR_UNSUPPORTED, "the surrogate covers finite depth only");
-  if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
+static int set_surrogate(hams_ctx* c, const float* params, double far_factor) {
   for (hams_ctx* l : c->lanes) CU(cudaStreamSynchronize(l->st));
   CU(cudaStreamSynchronize(c->st));
   if (params) {
@@ -3576,6 +3639,17 @@ extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t 
   return 0;
 }
 
+extern "C" int hams_ctx_set_surrogate(hams_ctx* c, const float* params, int32_t nparams, double far_factor) {
+  g_err.clear();
+  if (!c || c->is_lane) return fail(HAMS_ERR_ARG, "null context");
+  if (params && nparams != sg::kParams)
+    return fail(HAMS_ERR_ARG, "surrogate parameter vector has %d floats, %d expected", nparams, sg::kParams);
+  if (params && !(far_factor > 0.0)) return fail(HAMS_ERR_ARG, "far_factor must be positive");
+  if (c->opts.depth < 0.0 && params) return fail(HAMS_ERR_UNSUPPORTED, "the surrogate covers finite depth only");
+  if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
+  return with_memory(c, [&] { return set_surrogate(c, params, far_factor); });
+}
+
 extern "C" int hams_last_timings(hams_ctx* c, double* ms, int32_t n) {
   if (!c || !ms) return 0;
   int k = std::min<int>(n, hams_ctx::kTimings);
@@ -3585,11 +3659,7 @@ extern "C" int hams_last_timings(hams_ctx* c, double* ms, int32_t n) {
 
 extern "C" const char* hams_last_note(hams_ctx* c) { return c ? c->note.c_str() : ""; }
 
-extern "C" int hams_ctx_set_field_points(hams_ctx* c, int32_t nfp, const double* xfp) {
-  g_err.clear();
-  if (!c || c->is_lane) return fail(HAMS_ERR_ARG, "null context");
-  if (nfp < 0 || (nfp > 0 && !xfp)) return fail(HAMS_ERR_ARG, "bad field points");
-  if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
+static int set_field_points(hams_ctx* c, int32_t nfp, const double* xfp) {
   for (hams_ctx* l : c->lanes) CU(cudaStreamSynchronize(l->st));
   CU(cudaStreamSynchronize(c->st));
   c->nfp = nfp;
@@ -3647,6 +3717,14 @@ extern "C" int hams_ctx_set_field_points(hams_ctx* c, int32_t nfp, const double*
   }
   CU(cudaStreamSynchronize(c->st));
   return 0;
+}
+
+extern "C" int hams_ctx_set_field_points(hams_ctx* c, int32_t nfp, const double* xfp) {
+  g_err.clear();
+  if (!c || c->is_lane) return fail(HAMS_ERR_ARG, "null context");
+  if (nfp < 0 || (nfp > 0 && !xfp)) return fail(HAMS_ERR_ARG, "bad field points");
+  if (cudaSetDevice(c->dev) != cudaSuccess) return fail(HAMS_ERR_CUDA, "cudaSetDevice failed");
+  return with_memory(c, [&] { return set_field_points(c, nfp, xfp); });
 }
 
 extern "C" int hams_field_potentials(hams_ctx* c, int32_t k, double* pot) {

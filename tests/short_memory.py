@@ -16,7 +16,8 @@ SHIM = r"""
 typedef struct { void* p; size_t n; } Block;
 static pthread_mutex_t mu = PTHREAD_MUTEX_INITIALIZER;
 static Block blocks[1 << 16];
-static int nblocks, refused, pending, fail_launch = -1;
+static int nblocks, refused, fail_launch = -1;
+static __thread int pending;  /* the runtime's last error is a thread's own, too */
 static size_t used, peak, limit;
 static char log_[1 << 22];
 static size_t nlog;

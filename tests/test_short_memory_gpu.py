@@ -129,3 +129,53 @@ got, less = batch(held - size)
 answer(less=held - less, same=all(np.array_equal(a, b) for a, b in zip(got, want)))
 """)
     assert got["less"] >= 1 << 20 and got["same"]
+
+
+# bodies, depth, waves, field points, keywords, and the MB that the call needs without what only saves time,
+# 5 % above the least found by bisection
+DECKS = {
+    "batch": ("test_series._rough([meshgen.cylinder(4.0, 6.0, 24, 8, 4)], 0.02, 1)", 45.0, 4, 0, "", 44),
+    "mixed": ("test_series._rough([meshgen.cylinder(4.0, 6.0, 24, 8, 4)], 0.02, 1)", 45.0, 1, 0,
+              "precision=hams_b200.PREC_MIXED", 23),
+    "field points": ("[meshgen.cylinder(4.0, 6.0, 20, 9, 4)]", 45.0, 3, 4000, "", 140),
+    "gmres": ("[meshgen.cylinder(4.0, 6.0, 20, 9, 4, 20.0 * k, 0.0) for k in range(3)]", 45.0, 1, 0,
+              "solver=hams_b200.SOLVER_GMRES, gmres_tol=1e-11, gmres_dense=1", 71),
+}
+
+
+@pytest.mark.parametrize("name", list(DECKS))
+def test_tables_make_room(so, name):
+    """The buffers that a solve allocates as it goes find no room beside the tables: these are given back
+    and the call is repeated, down to the memory that it needs without them.  Every limit from there up
+    works, with the results of ample memory to the rounding of another order of sums."""
+    bodies, depth, nf, field, kw, need = DECKS[name]
+    got = short_memory.run(so, f"bodies, depth, nf, field, need, kw = \"{bodies}\", {depth}, {nf}, {field}, {need}, dict({kw})" + """
+import test_series
+geom = deck(eval(bodies))
+rng = np.random.default_rng(1)
+p = np.column_stack([rng.uniform(8.0, 30.0, field), rng.uniform(-20.0, 20.0, field), -rng.uniform(0.5, 12.0, field)])
+waves = [hams_b200.wave_properties(v, depth, 9.81) for v in np.linspace(0.6, 1.4, nf)]
+def solved(limit):
+    hams_b200.release_cached()
+    mem.short_memory_limit(limit)
+    ctx = hams_b200.Context(geom, depth, rho=1025.0, g=9.81, **kw)
+    if field: ctx.set_field_points(p)
+    out = list(ctx.solve_batch(waves, [0.3]) if nf > 1 else ctx.solve_frequency(waves[0], [0.3]))
+    if field: out += [ctx.field_potentials(1, k) for k in range(nf)]
+    mem.short_memory_limit(0)
+    ctx.close()
+    return out
+solved(0)
+hams_b200.release_cached()
+mem.short_memory_reset()
+want = solved(0)
+peak, errs, refused = mem.short_memory_peak(), [], []
+need = int(need * 2 ** 20)
+for limit in np.linspace(need, peak, 9).astype(int):
+    mem.short_memory_reset()
+    errs.append(max(rel(a, b) for a, b in zip(solved(int(limit)), want)))
+    refused.append(mem.short_memory_refused())
+answer(peak=peak, need=need, errs=errs, refused=refused)
+""")
+    assert got["need"] < 0.9 * got["peak"] and got["refused"][0] > 0, got
+    assert max(got["errs"]) < 1e-9, got
