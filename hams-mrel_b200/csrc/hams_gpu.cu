@@ -2941,7 +2941,8 @@ static int field_setup(hams_ctx* f, hams_ctx* of) {
 }
 // c's pair set for its field points; the caller's stream c->st is idle.  Left
 // out (k_field_pairs takes over) where the pairs exceed the 32-bit index or
-// memory runs out.
+// memory runs out; a lane that finds no memory for its part of one fails, so that
+// all frequencies of a batch take the same way.
 static int field_context(hams_ctx* c, hams_ctx* of) {
   field_free(c->field);
   c->field = nullptr;
@@ -2967,7 +2968,7 @@ static int field_context(hams_ctx* c, hams_ctx* of) {
   if (rc < 0) {
     cudaStreamSynchronize(f->st);  // a kernel of the set may still write the buffers that go back
     field_free(f);
-    if (rc != HAMS_ERR_NOMEM) return rc;
+    if (of || rc != HAMS_ERR_NOMEM) return rc;
     g_err.clear();
     return 0;
   }
@@ -3706,6 +3707,7 @@ static int set_field_points(hams_ctx* c, int32_t nfp, const double* xfp) {
     l->field = nullptr;
   }
   TRY(field_context(c, nullptr));
+  int rc = 0;
   for (hams_ctx* l : c->lanes) {
     l->nfp = nfp;
     l->fp_last.clear();
@@ -3713,7 +3715,19 @@ static int set_field_points(hams_ctx* c, int32_t nfp, const double* xfp) {
       l->fp_x.view(c->fp_x);
       l->fp_sld.view(c->fp_sld);
     }
-    if (c->field) TRY(field_context(l, c->field));
+    if (c->field && !rc) rc = field_context(l, c->field);
+  }
+  if (rc == HAMS_ERR_NOMEM) {  // none of them has it
+    cudaStreamSynchronize(c->st);  // which fills its Rankine tables
+    for (hams_ctx* l : c->lanes) {
+      field_free(l->field);
+      l->field = nullptr;
+    }
+    field_free(c->field);
+    c->field = nullptr;
+    g_err.clear();
+  } else {
+    TRY(rc);
   }
   CU(cudaStreamSynchronize(c->st));
   return 0;

@@ -179,3 +179,33 @@ answer(peak=peak, need=need, errs=errs, refused=refused)
 """)
     assert got["need"] < 0.9 * got["peak"] and got["refused"][0] > 0, got
     assert max(got["errs"]) < 1e-9, got
+
+
+def test_field_points_of_a_batch_take_one_way(so):
+    """A lane that finds no room for the mode tables of the points' pair set, though for the influences
+    themselves: every frequency has the bits of the pair set, or every one those of the pairs taken singly."""
+    got = short_memory.run(so, """
+geom = deck([meshgen.cylinder(4.0, 6.0, 6, 3, 1)])
+rng, m = np.random.default_rng(1), 20000
+p = np.column_stack([rng.uniform(8.0, 30.0, m), rng.uniform(-20.0, 20.0, m), -rng.uniform(0.5, 12.0, m)])
+waves = [hams_b200.wave_properties(v, 45.0, 9.81) for v in np.linspace(0.6, 1.4, 6)]
+def solved(room):
+    ctx = hams_b200.Context(geom, 45.0, rho=1025.0, g=9.81, batch_lanes=2)
+    ctx.set_field_points(p)
+    ctx.solve_frequency(waves[0], [0.3])
+    hams_b200.release_cached()
+    mem.short_memory_reset()
+    mem.short_memory_limit(mem.short_memory_used() + room if room else 0)
+    ctx.solve_batch(waves, [0.3])
+    mem.short_memory_limit(0)
+    out = [ctx.field_potentials(1, k) for k in range(len(waves))]
+    ctx.close()
+    hams_b200.release_cached()
+    return out
+want, ways = solved(0), []
+for mb in range(22, 62, 3):
+    ways.append([bool(np.array_equal(a, b)) for a, b in zip(solved(mb << 20), want)])
+answer(ways=ways)
+""")
+    assert all(all(w) or not any(w) for w in got["ways"]), got
+    assert any(all(w) for w in got["ways"]) and any(not any(w) for w in got["ways"]), got
