@@ -3456,9 +3456,17 @@ extern "C" int hams_eval_green(hams_ctx* c, const hams_wave* w, int32_t npts, co
     const bool series = c->opts.depth >= 0.0 && !wd.limit;
     if (series) CU(cudaMemcpyAsync(c->wvn.p, w->wvn, HAMS_NK * 8, cudaMemcpyHostToDevice, c->st));
     CU(cudaMemsetAsync(c->ovf.p, 0, sizeof(int), c->st));
+    bool singly = !series;  // a thread per point
     if (series) {
-      TRY(point_series(c, wd, npts, dp.p, df.p, dout.p, list, hist, key, work));
-    } else {
+      const int rc = point_series(c, wd, npts, dp.p, df.p, dout.p, list, hist, key, work);
+      if (rc == HAMS_ERR_NOMEM) {  // no room for the lists or tables
+        g_err.clear();
+        singly = true;
+      } else {
+        TRY(rc);
+      }
+    }
+    if (singly) {
       launch_eval_green((npts + 127) / 128, c->st, npts, dp.p, df.p, wd, c->wvn.p, dout.p, c->ovf.p);
       TRY(launch_check(c));
     }

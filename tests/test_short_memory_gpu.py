@@ -209,3 +209,27 @@ answer(ways=ways)
 """)
     assert all(all(w) or not any(w) for w in got["ways"]), got
     assert any(all(w) for w in got["ways"]) and any(not any(w) for w in got["ways"]), got
+
+
+def test_points_without_their_tables(so):
+    """hams_eval_green with room for the points and their results only: a thread per point, the same bits."""
+    got = short_memory.run(so, """
+ctx = hams_b200.Context(deck([meshgen.cylinder(4.0, 4.0, 8, 2, 2)]), 31.0, g=9.81)
+rng, n = np.random.default_rng(1), 5000
+r, th = 31.0 * np.exp(rng.uniform(np.log(1e-4), np.log(2.0), n)), rng.uniform(0.0, 6.28, n)
+pts = np.zeros((n, 6), order="F")
+pts[:, 3], pts[:, 4] = r * np.cos(th), r * np.sin(th)
+pts[:, 2], pts[:, 5] = rng.uniform(-12.0, -0.3, n), rng.uniform(-12.0, -0.3, n)
+flag, wave = (rng.uniform(size=n) < 0.5).astype(np.int32), ctx.wave(1.3)
+want = ctx.eval_green(wave, pts, flag)
+hams_b200.release_cached()
+same, refused = [], []
+for room in (n * (48 + 4 + 64) + 4096, 1 << 20, 4 << 20):
+    mem.short_memory_reset()
+    mem.short_memory_limit(mem.short_memory_used() + room)
+    same.append(bool(np.array_equal(ctx.eval_green(wave, pts, flag), want)))
+    refused.append(mem.short_memory_refused())
+    hams_b200.release_cached()
+answer(same=same, refused=refused)
+""")
+    assert all(got["same"]) and all(got["refused"]), got
