@@ -2522,6 +2522,12 @@ static int mixed_solve(hams_ctx* c, double2* M, const double2* rhs, int ldr, int
   return mixed_refine(c, M, rhs, ldr, nrhs);
 }
 
+// The error of a zlu_solve that returned rc.
+static int zlu_fail(const char* what, int rc) {
+  if (rc >= 10) return fail(HAMS_ERR_CUDA, "%s: cublas status %d", what, rc - 10);
+  return fail(HAMS_ERR_CUDA, "%s: %s", what, cudaGetErrorString(cudaGetLastError()));
+}
+
 // Most panels of a body whose block GMRES inverts.  An inverse takes four times
 // the operations of the factors and saves every step their triangular solves: two
 // bodies in infinite depth, five steps, factors against inverses 38.8 / 13.5 ms at
@@ -2633,7 +2639,7 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
                                (size_t)nn * nn, c->info.p, c->zwork.p, nullptr, &la, &lb);
       c->launches += la;
       c->lib_calls += lb;
-      if (rc) return fail(HAMS_ERR_CUDA, "GMRES preconditioner: LU failed (%d)", rc);
+      if (rc) return zlu_fail("GMRES preconditioner", rc);
       k_mark_singular<<<1, 32, 0, c->st>>>(c->info.p, c->gpre.p + boff[b], (size_t)nn * nn, e - b);
       TRY(launch_check(c));
     }
@@ -2853,7 +2859,7 @@ static int solve_dev(hams_ctx* c, int nrhs, int* info_host) {
       const int rc = zlu_solve(c->st, c->blas, 1, n, nrhs, M, 0, c->X.p, 0, c->info.p, c->zwork.p, c->evf, &la, &lb);
       c->launches += la;
       c->lib_calls += lb;
-      if (rc) return fail(HAMS_ERR_CUDA, "LU: %s", rc >= 10 ? "a cuBLAS product failed" : cudaGetErrorString(cudaGetLastError()));
+      if (rc) return zlu_fail("LU", rc);
       CU(cudaMemcpyAsync(info_host, c->info.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
       return 0;
     }

@@ -514,7 +514,7 @@ int zlu_solve(cudaStream_t st, cublasHandle_t blas, int batch, int n, int nrhs, 
                  nrhs, zb, work);
       *launches += 1;
     }
-    if (cudaGetLastError() != cudaSuccess) return 1;
+    if (cudaPeekAtLastError() != cudaSuccess) return 1;
     double2* Lk = A + (size_t)k0 * n + k1;
     int rc = gemm(right, right, kb, Lk, A + (size_t)k1 * n + k0, sa, A + (size_t)k1 * n + k1, sa);
     if (!rc) rc = gemm(right, nrhs, kb, Lk, X + k0, sx, X + k1, sx);
@@ -527,7 +527,7 @@ int zlu_solve(cudaStream_t st, cublasHandle_t blas, int batch, int n, int nrhs, 
     pdl_launch(k_zback, dim3(blocks(nrhs, kZBackCols), 1, batch), dim3(128), kZBackSmem, st, A, n, n, k0, kb, X, nrhs,
                zb);
     *launches += 1;
-    if (cudaGetLastError() != cudaSuccess) return 1;
+    if (cudaPeekAtLastError() != cudaSuccess) return 1;
     const int rc = gemm(k0, nrhs, kb, A + (size_t)k0 * n, X + k0, sx, X, sx);
     if (rc) return rc;
   }

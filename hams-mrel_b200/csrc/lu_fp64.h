@@ -18,7 +18,7 @@ int zlu_supported(int n);
 // in 16-column panels, rows ordered by pivot).  info[0] receives 1 + a column
 // with a zero pivot, the first one of a single system, or stays at 0.  evf, if
 // not null, is recorded after the last column is factored (the forward
-// substitution is part of the factorisation).  Returns 0, 1 on a CUDA error, or
-// 10 + a cuBLAS status.
+// substitution is part of the factorisation).  Returns 0, 1 on a CUDA error (left as
+// the thread's last error), or 10 + a cuBLAS status.
 int zlu_solve(cudaStream_t st, cublasHandle_t blas, int batch, int n, int nrhs, double2* A, size_t sa, double2* X,
               size_t sx, int* info, int* work, cudaEvent_t evf, long long* launches, long long* lib_calls);

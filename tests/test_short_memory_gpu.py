@@ -233,3 +233,27 @@ for room in (n * (48 + 4 + 64) + 4096, 1 << 20, 4 << 20):
 answer(same=same, refused=refused)
 """)
     assert all(got["same"]) and all(got["refused"]), got
+
+
+@pytest.mark.parametrize("solver", ["SOLVER_LU", "SOLVER_GMRES"])
+def test_a_refused_launch_of_the_lu_is_named(so, solver):
+    """The runtime refuses one launch of the complex128 LU: the call's error is the runtime's, and the next
+    call works."""
+    got = short_memory.run(so, f"solver = hams_b200.{solver}" + """
+geom = deck([meshgen.cylinder(5.0, 8.0, 10, 4, 4, 30.0 * k, 0.0) for k in range(2)])
+ctx = hams_b200.Context(geom, -1.0, rho=1025.0, g=9.81, solver=solver, gmres_dense=1)
+w, msgs = ctx.wave(0.9), []
+want = ctx.solve_frequency(w, [0.3])
+for k in (0, 1, 2, 3, 12):  # panel, its rows' exchange, update, and one of a later block of columns
+    mem.short_memory_fail_launch(k)
+    try:
+        ctx.solve_frequency(w, [0.3])
+        msgs.append("")
+    except hams_b200.HamsError as e:
+        msgs.append(str(e))
+    mem.short_memory_fail_launch(-1)
+    again = ctx.solve_frequency(w, [0.3])
+    msgs[-1] += "" if all(np.array_equal(a, b) for a, b in zip(again, want)) else " (and then wrong)"
+answer(msgs=msgs)
+""")
+    assert all("-2" in m and m.endswith("invalid configuration argument") for m in got["msgs"]), got
