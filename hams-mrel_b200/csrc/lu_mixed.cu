@@ -164,7 +164,9 @@ __global__ void __launch_bounds__(kLuThreads) k_diag_lu(const float2* __restrict
         const int j = j0 + s;
         if (j < nbk) {  // uniform
           // offer this warp's best row and the reciprocal of its entry
-          const uint32_t mine = taken ? 0u : __float_as_uint(fabsf(cur.x) + fabsf(cur.y)) + 1u;
+          // (an entry that is no number counts as zero: no pivot while there is another, and a
+          // column without one is reported)
+          const uint32_t mine = taken ? 0u : __float_as_uint(fmaxf(fabsf(cur.x) + fabsf(cur.y), 0.0f)) + 1u;
           const uint32_t best = __reduce_max_sync(0xffffffffu, mine);
           const float2 rcp = reciprocal(cur);
           float2* of = offer + ((j & 1) * kLuRowWarps + warp) * kNB;
