@@ -2609,9 +2609,8 @@ static int gmres_solve(hams_ctx* c, double2* M, const double2* rhs, int nrhs) {
     boff[b + 1] = boff[b] + (size_t)c->body_nelem[b] * c->body_nelem[b];
   }
   TRY(c->gpiv.alloc(n));
-  bool inv = nb > 1 && !c->lean;
-  for (int b = 0; b < nb && inv; ++b)
-    inv = c->body_nelem[b] > 0 && c->body_nelem[b] <= kInvRows && zlu_supported(c->body_nelem[b]) == 0;
+  const auto size = std::minmax_element(c->body_nelem.begin(), c->body_nelem.end());
+  bool inv = nb > 1 && !c->lean && *size.first > 0 && *size.second <= kInvRows && zlu_supported(*size.second) == 0;
   TRY(c->gpre.alloc(nb > 1 ? boff[nb] : (size_t)n));  // either way needs it
   if (inv && (c->gblk.alloc(boff[nb]) || c->gtmp.alloc((size_t)n * nrhs))) {
     inv = false;
