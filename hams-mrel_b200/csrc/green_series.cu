@@ -75,13 +75,14 @@ __global__ void __launch_bounds__(128) k_rad_series(DevGeom g, WaveDev w, const 
   }
 }
 
-void launch_rad_series(int br, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, const double* ur,
+void launch_rad_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, const double* ur,
                        const uint32_t* pairs, long long count, double* kt, double4* jy) {
+  const dim3 grid((unsigned)((count + 127) / 128), ntmax);
   if (br == hams::kPidcock)
-    k_rad_series<hams::kPidcock><<<dim3((unsigned)((count + 127) / 128), hams::kPidcockMax), 128, 0, st>>>(
+    k_rad_series<hams::kPidcock><<<grid, 128, 0, st>>>(
         g, w, wvn, ur, pairs, count, kt, jy);
   else
-    k_rad_series<hams::kEigenE><<<dim3((unsigned)((count + 127) / 128), hams::kEigenEMax), 128, 0, st>>>(
+    k_rad_series<hams::kEigenE><<<grid, 128, 0, st>>>(
         g, w, wvn, ur, pairs, count, kt, jy);
 }
 
@@ -559,7 +560,7 @@ void launch_point_series(int br, int ntmax, cudaStream_t st, int npts, const dou
   const int nmode = ntmax + 1;
   launch_mode_tables(st, g, w, wvn, nmode, pw.pm, pw.ac, pw.src, pw.srct, pw.fld, pw.fldt);
   const hams::ModeTab mt{m, m, nmode, pw.pm, pw.ac, pw.src, pw.srct, pw.fld, pw.fldt};
-  launch_rad_series(br, st, g, w, wvn, pw.r, nullptr, m, pw.kt, pw.jy);
+  launch_rad_series(br, ntmax, st, g, w, wvn, pw.r, nullptr, m, pw.kt, pw.jy);
   launch_series(br, ntmax, st, g, w, wvn, mt, RadTab{nullptr, 0, pw.kt, pw.jy}, PointIO{list, flag, out, (size_t)npts},
                 m, ovf);
 }

@@ -190,27 +190,33 @@ __global__ void k_distance_heads(const double* __restrict__ r, long long count, 
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < count) head[t] = t == 0 || r[t] != r[t - 1];
 }
-// rid of every pair, the distinct distances ur, and each branch's first and
-// last distance number (lim[2 br], lim[2 br + 1]); cut0..cut4 are the
-// positions where bins 2..6 start, counted from bin 1.
-__device__ __forceinline__ int series_class(long long pos, long long c2, long long c3, long long c4, long long c5) {
-  if (pos < c2) return hams::kPidcock;
-  if (pos < c3) return hams::kEigenE;
-  if (pos < c4) return hams::kEigen;
-  return pos < c5 ? hams::kEigenE : hams::kEigen;
-}
+// The number of each pair's distance (rid) and the distinct distances (ur) from
+// the sorted ones; entry idx of the sorted list is pair idx of the list's n1
+// first, or idx - n1 of its second part, which starts off2 further on.
 __global__ void k_distance_rows(const double* __restrict__ r, const uint32_t* __restrict__ idx,
-                                const uint32_t* __restrict__ rank, long long count, long long c2, long long c3,
-                                long long c4, long long c5, uint32_t* __restrict__ rid, double* __restrict__ ur,
-                                uint32_t* __restrict__ lim) {
+                                const uint32_t* __restrict__ rank, long long count, long long n1, long long off2,
+                                uint32_t* __restrict__ rid, double* __restrict__ ur) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const uint32_t k = rank[t] - 1;
-  rid[idx[t]] = k;
+  const long long i = idx[t];
+  rid[i < n1 ? i : off2 + i - n1] = k;
   if (t == 0 || rank[t - 1] != rank[t]) ur[k] = r[t];
-  const int br = series_class(idx[t], c2, c3, c4, c5);
-  if (t == 0 || series_class(idx[t - 1], c2, c3, c4, c5) != br) atomicMin(&lim[2 * br], k);
-  if (t == count - 1 || series_class(idx[t + 1], c2, c3, c4, c5) != br) atomicMax(&lim[2 * br + 1], k);
+}
+// The pairs in the order of their distances, with the numbers and the distinct
+// distances; cut: where every per-th distance starts.
+__global__ void k_distance_order(const double* __restrict__ r, const uint32_t* __restrict__ idx,
+                                 const uint32_t* __restrict__ rank, long long count, uint32_t per,
+                                 const uint32_t* __restrict__ pairs, uint32_t* __restrict__ ordered,
+                                 uint32_t* __restrict__ rid, double* __restrict__ ur, uint32_t* __restrict__ cut) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t k = rank[t] - 1;
+  ordered[t] = pairs[idx[t]];
+  rid[t] = k;
+  if (t > 0 && rank[t - 1] == rank[t]) return;
+  ur[k] = r[t];
+  if (k % per == 0) cut[k / per] = (uint32_t)t;
 }
 
 // ---------------------------------------------------------------------------
@@ -1226,13 +1232,20 @@ struct hams_ctx {
   // EIGEN), 4-5 (surrogate pairs of EIGENE, EIGEN), 6 (pairs of copied body
   // blocks); bin_off[7] = total
   long long bin_off[kBins + 1] = {};
-  // radial tables: the distance number of every pair of bins 1-5 (from bin 1
-  // on), the distinct distances, and each branch's first and number of
-  // distances; a branch without distance numbers (rad_n = 0) gives every pair
-  // its own row, a chunk of pairs at a time
-  DBuf<uint32_t> rid;
-  DBuf<double> ur;
-  uint32_t rad_base[4] = {}, rad_n[4] = {};
+  // radial tables (build_distances): the distance number of every pair of bins
+  // 1-5 (from bin 1 on) and the distinct distances, of a branch (rad_n of them,
+  // in ur[br]) or of one bin whose pairs are in the order of their distances
+  // (chunks not empty; ur[bin]); bins 4 and 5 have that order in a list of its
+  // own.  Pairs without numbers have a table row each, a chunk of them at a time
+  struct RadChunk {
+    long long pair;  // first pair of the bin, and its distance
+    double r;
+  };
+  DBuf<uint32_t> rid, far_pairs;
+  DBuf<double> ur[kBins];
+  uint32_t rad_n[4] = {};
+  std::vector<RadChunk> chunk[kBins];  // of kRadMin bytes of table each, and the end
+  uint32_t chunk_n[kBins] = {};        // distances of the bin
   // LINTON rows: the row of every pair of bin 0 and a pair of each row (none:
   // a row per pair), this frequency's rows
   DBuf<uint32_t> lrow, lrep;
@@ -1370,7 +1383,8 @@ extern "C" void hams_ctx_destroy(hams_ctx* c) {
   rel(c->fp_x, c->fp_sld, c->fp_S, c->fp_D, c->fp_bc, c->fp_pot, c->fp_out, c->hxp, c->hyp, c->hw);
   field_free(c->field);
   rel(c->xq, c->fxyz, c->ds, c->pnsz, c->nrm, c->vtx, c->ncn, c->body, c->bstart, c->rs, c->rd, c->pairs);
-  rel(c->rid, c->ur, c->lrow, c->lrep, c->lin_fg);
+  rel(c->rid, c->far_pairs, c->lrow, c->lrep, c->lin_fg);
+  for (auto& u : c->ur) rel(u);
   for (int br = 0; br < 4; ++br) rel(c->rad_k[br], c->rad_j[br]);
   rel(c->blk_copied, c->blk_list, c->chunks, c->bchunk, c->A, c->S, c->B, c->part, c->wd, c->C, c->D, c->X, c->R);
   rel(c->Af, c->Xf, c->luw, c->gv, c->gw, c->gz, c->gy, c->gpre, c->gblk, c->gtmp, c->gnrm, c->gpiv, c->perm,
@@ -1414,8 +1428,11 @@ static bool shed(hams_ctx* c) {
     x->lean = true;
     field_free(x->field);
     x->field = nullptr;
-    for (DBuf<uint32_t>* d : {&x->rid, &x->lrow, &x->lrep}) d->release(true);
-    x->ur.release(true);
+    for (DBuf<uint32_t>* d : {&x->rid, &x->far_pairs, &x->lrow, &x->lrep}) d->release(true);
+    for (int b = 0; b < kBins; ++b) {
+      x->ur[b].release(true);
+      x->chunk[b].clear();
+    }
     x->lin_fg.release(true);
     x->lin_rows = x->bin_off[1];
     for (int br = 0; br < 4; ++br) {
@@ -1453,83 +1470,129 @@ constexpr long long kLinChunk = 65536;  // LINTON pairs of a chunk without row n
 constexpr size_t kRadLean = (size_t)2 << 20;
 constexpr long long kLinLean = 4096, kRadLeast = 512;
 
-// The distinct distances of the series bins (RadTab): the pairs' distances
-// sorted, numbered where they change, the numbers scattered back to the
-// pairs.  A branch whose table would exceed half the bytes of A (a mesh
-// with few equal distances) keeps no numbers.
-static int build_distances(hams_ctx* c) {
-  const long long o1 = c->bin_off[1], ns = c->bin_off[6] - o1;
-  for (int br = 0; br < 4; ++br) c->rad_base[br] = c->rad_n[br] = 0;
-  c->rid.release(true);
-  if (ns <= 0 || c->lean) return 0;
+// The sorted distances of the pairs of one or two bins.
+struct DistSort {
   DBuf<double> r, r2;
-  DBuf<uint32_t> idx, idx2, rank, lim;
-  // without the memory for the sort, every pair has its own row
-  if (r.alloc(ns) || r2.alloc(ns) || idx.alloc(ns) || idx2.alloc(ns) || rank.alloc(ns) || lim.alloc(8) ||
-      c->rid.alloc(ns)) {
-    g_err.clear();
-    c->rid.release(true);
-    return 0;
+  DBuf<uint32_t> idx, idx2, rank;  // rank: 1 + the number of the distance
+  DBuf<char> tmp;
+  long long n1 = 0, count = 0;  // pairs of the first bin, of both
+  uint32_t nu = 0;              // distinct distances
+  void release() {  // after the stream has been waited for
+    r.release(true);
+    r2.release(true);
+    for (DBuf<uint32_t>* d : {&idx, &idx2, &rank}) d->release(true);
+    tmp.release(true);
   }
-  for (int b = 1; b < 6; ++b) {
-    const long long n = c->bin_off[b + 1] - c->bin_off[b];
-    if (n <= 0) continue;
-    const uint32_t* lst = c->pairs.p + c->bin_off[b];
-    double* out = r.p + (c->bin_off[b] - o1);
-    if (b == 3 || b == 5) k_eigen_distance<<<(unsigned)((n + 255) / 256), 256, 0, c->st>>>(c->g, lst, n, out);
-    else launch_series_distance(c->st, c->g, lst, n, out);
+};
+static int sort_distances(hams_ctx* c, int br, int b1, int b2, DistSort& d) {
+  const long long n1 = c->bin_off[b1 + 1] - c->bin_off[b1], n2 = b2 ? c->bin_off[b2 + 1] - c->bin_off[b2] : 0;
+  d.n1 = n1;
+  const long long n = d.count = n1 + n2;
+  size_t t1 = 0, t2 = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, t1, d.r.p, d.r2.p, d.idx.p, d.idx2.p, (size_t)n, 0, 64, c->st);
+  cub::DeviceScan::InclusiveSum(nullptr, t2, d.rank.p, d.rank.p, (size_t)n, c->st);
+  for (DBuf<double>* x : {&d.r, &d.r2}) TRY(x->alloc(n));
+  for (DBuf<uint32_t>* x : {&d.idx, &d.idx2, &d.rank}) TRY(x->alloc(n));
+  TRY(d.tmp.alloc(std::max(t1, t2)));
+  for (int q = 0; q < 2; ++q) {
+    const long long m = q ? n2 : n1;
+    if (m <= 0) continue;
+    const uint32_t* lst = c->pairs.p + c->bin_off[q ? b2 : b1];
+    double* out = d.r.p + (q ? n1 : 0);
+    if (br == hams::kEigen) k_eigen_distance<<<(unsigned)((m + 255) / 256), 256, 0, c->st>>>(c->g, lst, m, out);
+    else launch_series_distance(c->st, c->g, lst, m, out);
     TRY(launch_check(c));
   }
-  const unsigned nb = (unsigned)((ns + 255) / 256);
-  k_iota<<<nb, 256, 0, c->st>>>(idx.p, ns);
-  size_t t1 = 0, t2 = 0;
-  cub::DeviceRadixSort::SortPairs(nullptr, t1, r.p, r2.p, idx.p, idx2.p, (size_t)ns, 0, 64, c->st);
-  cub::DeviceScan::InclusiveSum(nullptr, t2, rank.p, rank.p, (size_t)ns, c->st);
-  DBuf<char> tbuf;
-  if (tbuf.alloc(std::max(t1, t2))) {
-    g_err.clear();
-    c->rid.release();
-    return 0;
-  }
-  CU(cub::DeviceRadixSort::SortPairs(tbuf.p, t1, r.p, r2.p, idx.p, idx2.p, (size_t)ns, 0, 64, c->st));
-  k_distance_heads<<<nb, 256, 0, c->st>>>(r2.p, ns, rank.p);
-  CU(cub::DeviceScan::InclusiveSum(tbuf.p, t2, rank.p, rank.p, (size_t)ns, c->st));
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  k_iota<<<nb, 256, 0, c->st>>>(d.idx.p, n);
+  CU(cub::DeviceRadixSort::SortPairs(d.tmp.p, t1, d.r.p, d.r2.p, d.idx.p, d.idx2.p, (size_t)n, 0, 64, c->st));
+  k_distance_heads<<<nb, 256, 0, c->st>>>(d.r2.p, n, d.rank.p);
+  CU(cub::DeviceScan::InclusiveSum(d.tmp.p, t2, d.rank.p, d.rank.p, (size_t)n, c->st));
   c->lib_calls += 2;
   TRY(launch_check(c, 2));
-  uint32_t nu = 0, l[8];
-  CU(cudaMemcpyAsync(&nu, rank.p + ns - 1, 4, cudaMemcpyDeviceToHost, c->st));
+  CU(cudaMemcpyAsync(&d.nu, d.rank.p + n - 1, 4, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
-  c->ur.release(true);
-  if (c->ur.alloc(nu)) {
-    g_err.clear();
-    c->rid.release(true);
-    return 0;
-  }
-  for (int q = 0; q < 8; ++q) l[q] = q % 2 ? 0u : 0xffffffffu;
-  CU(cudaMemcpyAsync(lim.p, l, sizeof l, cudaMemcpyHostToDevice, c->st));
-  k_distance_rows<<<nb, 256, 0, c->st>>>(r2.p, idx2.p, rank.p, ns, c->bin_off[2] - o1, c->bin_off[3] - o1,
-                                         c->bin_off[4] - o1, c->bin_off[5] - o1, c->rid.p, c->ur.p, lim.p);
+  return 0;
+}
+// Pairs whose tables fill kRadMin bytes.
+constexpr uint32_t rad_chunk(int br) { return (uint32_t)(kRadMin / (rad_stride(br) * 8)); }
+
+// One bin in the order of its distances (a sort of it alone in d).
+static int order_bin(hams_ctx* c, int br, int b, DistSort& d) {
+  const long long n = d.count, o = c->bin_off[b];
+  const uint32_t per = rad_chunk(br), nc = (d.nu + per - 1) / per;
+  DBuf<uint32_t> cut;
+  TRY(cut.alloc(nc));
+  TRY(c->ur[b].alloc(d.nu));
+  const bool far = b >= 4;
+  if (far) TRY(c->far_pairs.alloc(c->bin_off[6] - c->bin_off[4]));
+  // a list in place goes through idx, which is free again
+  uint32_t* to = far ? c->far_pairs.p + (o - c->bin_off[4]) : d.idx.p;
+  k_distance_order<<<(unsigned)((n + 255) / 256), 256, 0, c->st>>>(d.r2.p, d.idx2.p, d.rank.p, n, per, c->pairs.p + o,
+                                                                   to, c->rid.p + (o - c->bin_off[1]), c->ur[b].p,
+                                                                   cut.p);
   TRY(launch_check(c));
-  CU(cudaMemcpyAsync(l, lim.p, sizeof l, cudaMemcpyDeviceToHost, c->st));
+  if (!far) CU(cudaMemcpyAsync(c->pairs.p + o, to, (size_t)n * 4, cudaMemcpyDeviceToDevice, c->st));
+  std::vector<uint32_t> at(nc);
+  std::vector<double> r(nc);
+  CU(cudaMemcpyAsync(at.data(), cut.p, (size_t)nc * 4, cudaMemcpyDeviceToHost, c->st));
+  CU(cudaMemcpy2DAsync(r.data(), 8, c->ur[b].p, (size_t)per * 8, 8, nc, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
-  for (DBuf<uint32_t>* d : {&idx, &idx2, &rank, &lim}) d->release(true);
-  r.release(true);
-  r2.release(true);
-  tbuf.release(true);
+  cut.release(true);
+  for (uint32_t k = 0; k < nc; ++k) c->chunk[b].push_back({at[k], r[k]});
+  c->chunk[b].push_back({n, 0.0});
+  c->chunk_n[b] = d.nu;
+  return 0;
+}
+
+// The distinct distances of the series bins (RadTab): the pairs' distances
+// sorted and numbered where they change, the numbers given to the pairs.  A
+// branch whose table would exceed half the bytes of A (an irregular mesh: a
+// distance has two pairs, (i, j) and (j, i)) is worked off in the order of the
+// distances instead, bin by bin: a chunk's table holds each of its distances once,
+// its pairs follow one another, and its series are of like length.
+static int build_distances(hams_ctx* c) {
+  const long long o1 = c->bin_off[1], ns = c->bin_off[6] - o1;
+  for (uint32_t& n : c->rad_n) n = 0;
+  for (auto& q : c->chunk) q.clear();
+  for (auto& u : c->ur) u.release(true);
+  c->far_pairs.release(true);
+  c->rid.release(true);
+  if (ns <= 0 || c->lean) return 0;
   const size_t cap = std::max(kRadMin, (size_t)c->tn * c->n * 8);
-  bool numbered = false;
-  for (int br = 1; br < 4; ++br) {
-    if (l[2 * br] > l[2 * br + 1]) continue;  // no pair
-    const uint32_t n = l[2 * br + 1] - l[2 * br] + 1;
-    if ((size_t)n * rad_stride(br) * 8 > cap) continue;
-    c->rad_base[br] = l[2 * br];
-    c->rad_n[br] = n;
-    numbered = true;
-  }
-  if (!numbered) {
-    c->rid.release(true);
-    c->ur.release(true);
-  }
+  int used = 0;
+  auto branch = [&](int br, int b2) -> int {
+    DistSort d;
+    const int bins[2] = {br, b2};
+    auto size = [&](int b) { return b ? c->bin_off[b + 1] - c->bin_off[b] : 0; };
+    if (size(br) + size(b2) <= 0) return 0;
+    const bool two = size(br) > 0 && size(b2) > 0;
+    TRY(sort_distances(c, br, br, b2, d));
+    if ((size_t)d.nu * rad_stride(br) * 8 <= cap) {
+      TRY(c->ur[br].alloc(d.nu));
+      k_distance_rows<<<(unsigned)((d.count + 255) / 256), 256, 0, c->st>>>(
+          d.r2.p, d.idx2.p, d.rank.p, d.count, d.n1, (b2 ? c->bin_off[b2] : 0) - c->bin_off[br],
+          c->rid.p + (c->bin_off[br] - o1), c->ur[br].p);
+      TRY(launch_check(c));
+      CU(cudaStreamSynchronize(c->st));
+      c->rad_n[br] = d.nu;
+      ++used;
+    } else {
+      for (int b : bins) {
+        if (size(b) <= 0) continue;
+        if (two) TRY(sort_distances(c, br, b, 0, d));
+        TRY(order_bin(c, br, b, d));
+        ++used;
+      }
+    }
+    d.release();
+    return 0;
+  };
+  int rc = c->rid.alloc(ns);
+  for (int br = hams::kPidcock; br <= hams::kEigen && !rc; ++br) rc = branch(br, br == hams::kPidcock ? 0 : br + 2);
+  if (rc && rc != HAMS_ERR_NOMEM) return rc;
+  if (rc) g_err.clear();  // the bins that are not done go without numbers
+  if (!used) c->rid.release(true);
   return 0;
 }
 
@@ -1885,12 +1948,17 @@ static void view_pairs(hams_ctx* l, hams_ctx* c) {
   for (int b = 0; b <= kBins; ++b) l->bin_off[b] = c->bin_off[b];
   l->pairs.view(c->pairs);
   l->rid.view(c->rid);
-  l->ur.view(c->ur);
+  l->far_pairs.view(c->far_pairs);
+  for (int b = 0; b < kBins; ++b) {
+    l->ur[b].view(c->ur[b]);
+    l->chunk[b] = c->chunk[b];
+    l->chunk_n[b] = c->chunk_n[b];
+  }
   l->lrow.view(c->lrow);
   l->lrep.view(c->lrep);
   l->lin_rows = c->lin_rows;
   l->lean = c->lean;
-  for (int br = 0; br < 4; ++br) l->rad_base[br] = c->rad_base[br], l->rad_n[br] = c->rad_n[br];
+  for (int br = 0; br < 4; ++br) l->rad_n[br] = c->rad_n[br];
   for (int b = 0; b < kBins; ++b) l->nt_cut[b][0] = c->nt_cut[b][0], l->nt_cut[b][1] = c->nt_cut[b][1];
 }
 
@@ -2111,11 +2179,17 @@ static WaveDev wave_dev(const hams_ctx* c, const hams_wave* w) {
   return d;
 }
 
-// The pairs of one bin from the EIGENE / PIDCOCK / EIGEN series (br); pos is
-// the list's place in c->pairs, or -1 for a list without distance numbers.
-// bin is the bin the list is (its launch is split by series length), or 0.
-static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* lst, long long cnt, long long pos,
-                        int bin) {
+// Terms of a branch's series at the distance r (FinGreen3D.f90:434, :592).
+static int longest_series(int br, double r, double h) {
+  if (br == hams::kEigen || !(r >= 0.0)) return hams::kPidcockMax;
+  const double rhp = r / h, t = br == hams::kPidcock ? HAMS_F4(-1010.10) * rhp + HAMS_F4(100.50)
+                                                     : HAMS_F4(-88.89) * rhp + HAMS_F4(54.45);
+  return std::max(2, (int)std::min(t, 1000.0));
+}
+
+// Pairs from the EIGENE / PIDCOCK / EIGEN series (br): those of a bin, or (bin 0)
+// of a list of their own.
+static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* lst, long long cnt, int bin) {
   if (cnt <= 0) return 0;
   const int ntmax = br == hams::kPidcock ? hams::kPidcockMax : hams::kEigenEMax;
   auto launch = [&](RadTab rt, const uint32_t* l, long long n, int nt) {
@@ -2127,49 +2201,65 @@ static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* 
                           c->ovf.p);
     return launch_check(c);
   };
-  auto table = [&](const double* ur, const uint32_t* l, long long n) {
+  auto table = [&](const double* ur, const uint32_t* l, long long n, int nt) {
     if (br == hams::kEigen)
       k_rad_eigen<<<(unsigned)((n + 127) / 128), 128, 0, c->st>>>(c->g, c->wvn.p, c->mt, ur, l, n, c->rad_k[br].p,
                                                                   c->rad_j[br].p);
     else
-      launch_rad_series(br, c->st, c->g, wd, c->wvn.p, ur, l, n, c->rad_k[br].p, c->rad_j[br].p);
+      launch_rad_series(br, nt, c->st, c->g, wd, c->wvn.p, ur, l, n, c->rad_k[br].p, c->rad_j[br].p);
     return launch_check(c);
   };
   if (wd.limit) return launch(RadTab{}, lst, cnt, 8);
-  if (pos >= 0 && c->rad_n[br]) {
+  const uint32_t* rid = bin ? c->rid.p + (c->bin_off[bin] - c->bin_off[1]) : nullptr;
+  if (bin && c->rad_n[br]) {
     if (!c->rad_ready[br]) {
-      TRY(table(c->ur.p + c->rad_base[br], nullptr, c->rad_n[br]));
+      TRY(table(c->ur[br].p, nullptr, c->rad_n[br], ntmax));
       c->rad_ready[br] = true;
     }
-    const uint32_t* rid = c->rid.p + (pos - c->bin_off[1]);
     // the longest series first, each launch with the shared memory of its own
     // lengths (and one more: the keys round distances with fused multiply-adds);
     // a list that one wave of blocks holds stays one launch
     long long cut[4] = {0, 0, 0, cnt};
-    if (br != hams::kEigen && bin && cnt > (long long)c->sms * 32 * 16) {
+    if (br != hams::kEigen && cnt > (long long)c->sms * 32 * 16) {
       cut[1] = c->nt_cut[bin][0] - c->bin_off[bin];
       cut[2] = c->nt_cut[bin][1] - c->bin_off[bin];
     }
     for (int q = 2; q >= 0; --q) {
       const long long n = cut[q + 1] - cut[q];
       if (n <= 0) continue;
-      const RadTab rt{rid + cut[q], c->rad_base[br], c->rad_k[br].p, c->rad_j[br].p};
+      const RadTab rt{rid + cut[q], 0, c->rad_k[br].p, c->rad_j[br].p};
       TRY(launch(rt, lst + cut[q], n, q == 2 ? ntmax : kNtCut[br == hams::kPidcock][q] + 1));
     }
     return 0;
   }
+  const uint32_t per = rad_chunk(br);
+  if (bin && !c->chunk[bin].empty()) {
+    if (!c->rad_k[br].alloc((size_t)per * rad_stride(br)) && !c->rad_j[br].alloc(per)) {
+      const auto& q = c->chunk[bin];
+      for (size_t k = 0; k + 1 < q.size(); ++k) {
+        const uint32_t d0 = (uint32_t)k * per, dn = std::min(per, c->chunk_n[bin] - d0);
+        // the chunk's longest series is that of its first distance (and one more, as above)
+        const int nt = std::min(ntmax, longest_series(br, q[k].r, wd.h) + 1);
+        const RadTab rt{rid + q[k].pair, d0, c->rad_k[br].p, c->rad_j[br].p};
+        TRY(table(c->ur[bin].p + d0, nullptr, dn, nt));
+        TRY(launch(rt, lst + q[k].pair, q[k + 1].pair - q[k].pair, nt));
+      }
+      return 0;
+    }
+    g_err.clear();
+  }
   // a row per pair, a chunk of pairs at a time; c->rad_k may hold the table
   // of the numbered distances, which is then filled again
-  long long per = std::min<long long>(cnt, (c->lean ? kRadLean : kRadMin) / (rad_stride(br) * 8));
-  while (c->rad_k[br].alloc((size_t)per * rad_stride(br)) || c->rad_j[br].alloc(per)) {
-    if (per <= kRadLeast) return HAMS_ERR_NOMEM;
-    per /= 2;
+  long long rows = std::min<long long>(cnt, c->lean ? kRadLean / (rad_stride(br) * 8) : per);
+  while (c->rad_k[br].alloc((size_t)rows * rad_stride(br)) || c->rad_j[br].alloc(rows)) {
+    if (rows <= kRadLeast) return HAMS_ERR_NOMEM;
+    rows /= 2;
     g_err.clear();
   }
   c->rad_ready[br] = false;
-  for (long long t = 0; t < cnt; t += per) {
-    const long long n = std::min(per, cnt - t);
-    TRY(table(nullptr, lst + t, n));
+  for (long long t = 0; t < cnt; t += rows) {
+    const long long n = std::min(rows, cnt - t);
+    TRY(table(nullptr, lst + t, n, ntmax));
     TRY(launch(RadTab{nullptr, 0, c->rad_k[br].p, c->rad_j[br].p}, lst + t, n, ntmax));
   }
   return 0;
@@ -2177,8 +2267,9 @@ static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* 
 // The pairs of bin b (1-5) of the context's list.
 static int series_bin(hams_ctx* c, const WaveDev& wd, int b) {
   static const int branch[6] = {hams::kLinton, hams::kPidcock, hams::kEigenE, hams::kEigen, hams::kEigenE, hams::kEigen};
-  return series_pairs(c, wd, branch[b], c->pairs.p + c->bin_off[b], c->bin_off[b + 1] - c->bin_off[b], c->bin_off[b],
-                      b);
+  const uint32_t* lst = b >= 4 && !c->chunk[b].empty() ? c->far_pairs.p + (c->bin_off[b] - c->bin_off[4])
+                                                       : c->pairs.p + c->bin_off[b];
+  return series_pairs(c, wd, branch[b], lst, c->bin_off[b + 1] - c->bin_off[b], b);
 }
 
 // The LINTON pairs (bin 0): their rows, then A and S; without row numbers a
@@ -2284,8 +2375,8 @@ static int assemble_dev(hams_ctx* c, const hams_wave* w, int nbeta, bool force_s
           const unsigned gb = (unsigned)((ns + 255) / 256);
           k_gather_pairs<<<gb, 256, 0, c->st>>>(c->sg_samp.p, ns, c->A.p, c->S.p, c->sg_g1.p);
           TRY(launch_check(c));
-          TRY(series_pairs(c, wd, hams::kEigenE, c->sg_samp.p, c->sg_ns4, -1, 0));
-          TRY(series_pairs(c, wd, hams::kEigen, c->sg_samp.p + c->sg_ns4, c->sg_ns5, -1, 0));
+          TRY(series_pairs(c, wd, hams::kEigenE, c->sg_samp.p, c->sg_ns4, 0));
+          TRY(series_pairs(c, wd, hams::kEigen, c->sg_samp.p + c->sg_ns4, c->sg_ns5, 0));
           k_gather_pairs<<<gb, 256, 0, c->st>>>(c->sg_samp.p, ns, c->A.p, c->S.p, c->sg_g2.p);
           k_sample_err<<<1, 1024, 0, c->st>>>(c->sg_g1.p, c->sg_g2.p, ns, c->sg_red.p);
           TRY(c->sg_cells.alloc(4 * kJCells));
@@ -2920,7 +3011,8 @@ static int forces_dev(hams_ctx* c, const hams_wave* w, int nbeta) {
 static void field_free(hams_ctx* f) {
   if (!f) return;
   auto rel = [](auto&... b) { (b.release(true), ...); };
-  rel(f->rs, f->rd, f->pairs, f->rid, f->ur, f->lrow, f->lrep, f->lin_fg, f->A, f->S, f->wvn, f->ovf);
+  rel(f->rs, f->rd, f->pairs, f->rid, f->far_pairs, f->lrow, f->lrep, f->lin_fg, f->A, f->S, f->wvn, f->ovf);
+  for (auto& u : f->ur) rel(u);
   rel(f->mt_pm, f->mt_ac, f->mt_fld, f->mt_fldt, f->mt_src, f->mt_srct);
   for (int br = 0; br < 4; ++br) rel(f->rad_k[br], f->rad_j[br]);
   delete f;

@@ -83,7 +83,7 @@ __host__ __device__ constexpr int rad_stride(int br) {
 void launch_green_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn,
                          const hams::ModeTab& mt, RadTab rt, const uint32_t* pairs, long long count, const double* rs,
                          const double* rd, double2* A, double2* S, int* ovf);
-void launch_rad_series(int br, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, const double* ur,
+void launch_rad_series(int br, int ntmax, cudaStream_t st, DevGeom g, WaveDev w, const double* wvn, const double* ur,
                        const uint32_t* pairs, long long count, double* kt, double4* jy);
 void launch_series_distance(cudaStream_t st, DevGeom g, const uint32_t* pairs, long long count, double* r);
 int series_kernels_init();
