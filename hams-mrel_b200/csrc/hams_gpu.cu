@@ -506,13 +506,12 @@ __global__ void __launch_bounds__(128, 8) k_green_eigen(DevGeom g, WaveDev w, co
 // pairs lie in vertical columns of panels: a 5,400-panel array of cylinders has
 // 37,800 pairs of 101 different (R, z, zeta).  The different triples are found
 // once per geometry (build_linton_rows), evaluated here, a row (G and its R and
-// z derivatives) each, and the rows given to their pairs by k_linton_pairs.
+// z derivatives) each, and the rows given to their pairs by k_linton_pairs; an
+// irregular mesh has hardly any equal ones, and each pair its own row.
 // A row is a long FP64 chain: adaptive Gauss-Kronrod integrals of three
 // integrands and a mode sum.  Few rows: a block of four warps each, a warp per
-// integral (its fifteen nodes, two lanes a node) and one for the sums; many: a
-// thread each.  5,400
-// panels, every pair: 2.05 -> 0.14 ms; one body of 234 panels 0.31 -> 0.12 ms
-// (a warp or a thread per pair before).
+// integral (its fifteen nodes, two lanes a node) and one for the sums; more: a
+// warp each, then a thread each (kLintonBlocksPerSm).
 struct LintonPair {
   int i, j;
   double xpq, ypq, zq, zp, rr;
@@ -548,9 +547,36 @@ __global__ void __launch_bounds__(128) k_linton_rows_threads(DevGeom g, WaveDev 
   linton_store(fg, t, f);
 }
 
-// Below this many rows per SM a block per row; above a thread per row (the
-// blocks' lanes repeat the work outside the integrals).
-constexpr int kLintonRowsPerSm = 64;
+// Up to kLintonBlocksPerSm rows per SM, one wave, a block per row; below
+// kLintonWarpsPerSm a warp per row, which takes its integrals in turn and waits for
+// no longer one; from there a thread per row (the lanes of a warp repeat the work
+// outside the integrals, but a thread's chain is long at low frequencies).
+// Microseconds in 40 m of water at 0.3 and 1.0 rad/s by block, warp, thread:
+// 444 rows 109, 374, 3,889 and 123, 142, 463; 592 rows 184, 374, 3,889 and 225, 140,
+// 459; 2,368 rows 683, 733, 3,887 and 654, 289, 458; 9,472 rows 2,899, 2,120, 3,900
+// and 2,533, 914, 456; 18,944 rows 5,862, 3,919, 4,000 and 5,321, 1,807, 459.
+constexpr int kLintonBlocksPerSm = 3, kLintonWarpsPerSm = 64;
+constexpr int kLintonWarps = 4;
+__global__ void __launch_bounds__(32 * kLintonWarps) k_linton_rows_warps(DevGeom g, WaveDev w,
+                                                                         const double* __restrict__ wvn,
+                                                                         const uint32_t* __restrict__ pairs,
+                                                                         const uint32_t* __restrict__ rep,
+                                                                         long long rows, double2* __restrict__ fg,
+                                                                         int* ovf) {
+  __shared__ double stack[kLintonWarps][2][hams::kQuadStack];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const long long row = (long long)blockIdx.x * kLintonWarps + wl;
+  if (row >= rows) return;  // the whole warp
+  const LintonPair q = linton_pair(g, pairs[rep ? rep[row] : row]);
+  const hams::WarpQuad quad{stack[wl][0], stack[wl][1], lane};
+  cplx f[3];
+  int o = 0;
+  hams::linton(q.rr, q.zq, q.zp, w.v, wvn[0], wvn, w.h, f, &o, quad);
+  if (lane != 0) return;
+  if (o) atomicOr(ovf, 1);
+  linton_store(fg, row, f);
+}
+
 __global__ void __launch_bounds__(128) k_linton_rows(DevGeom g, WaveDev w, const double* __restrict__ wvn,
                                                      const uint32_t* __restrict__ pairs,
                                                      const uint32_t* __restrict__ rep, double2* __restrict__ fg,
@@ -604,7 +630,8 @@ __global__ void __launch_bounds__(128) k_linton_pairs(DevGeom g, WaveDev w, cons
   store_pair(g, p, q.i, q.j, G, rs, rd, A, S);
 }
 
-// A hash of a LINTON pair's (R, z, zeta); equal triples are neighbours once
+// A hash of a LINTON pair's (R, z, zeta), by the finaliser of SplitMix64 (G. L.
+// Steele, D. Lea, C. H. Flood, OOPSLA 2014); equal triples are neighbours once
 // sorted by its lower half (unless others share it: then a triple may get
 // more than one row).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
@@ -1625,7 +1652,8 @@ static int build_linton_rows(hams_ctx* c) {
   uint32_t rows = 0;
   CU(cudaMemcpyAsync(&rows, rank.p + n - 1, 4, cudaMemcpyDeviceToHost, c->st));
   CU(cudaStreamSynchronize(c->st));
-  if (c->lrep.alloc(rows)) {
+  // few equal ones: each pair its own row, in the order of the pairs
+  if (2 * (long long)rows > n || c->lrep.alloc(rows)) {
     g_err.clear();
     c->lrow.release();
     return 0;
@@ -2288,8 +2316,11 @@ static int linton_bin(hams_ctx* c, const WaveDev& wd) {
     const long long n = std::min(per, cnt - t), rows = numbered ? c->lin_rows : n;
     const uint32_t* lst = c->pairs.p + t;
     if (!wd.limit) {
-      if (rows < (long long)c->sms * kLintonRowsPerSm)
+      if (rows <= (long long)c->sms * kLintonBlocksPerSm)
         k_linton_rows<<<(unsigned)rows, 128, 0, c->st>>>(c->g, wd, c->wvn.p, lst, c->lrep.p, c->lin_fg.p, c->ovf.p);
+      else if (rows < (long long)c->sms * kLintonWarpsPerSm)
+        k_linton_rows_warps<<<(unsigned)((rows + kLintonWarps - 1) / kLintonWarps), 32 * kLintonWarps, 0, c->st>>>(
+            c->g, wd, c->wvn.p, lst, c->lrep.p, rows, c->lin_fg.p, c->ovf.p);
       else
         k_linton_rows_threads<<<(unsigned)((rows + 127) / 128), 128, 0, c->st>>>(c->g, wd, c->wvn.p, lst, c->lrep.p,
                                                                                  rows, c->lin_fg.p, c->ovf.p);
