@@ -546,7 +546,7 @@ void launch_point_linton(cudaStream_t st, int npts, const double* pts, const int
   k_point_linton<<<(count + kPointWarps - 1) / kPointWarps, 32 * kPointWarps, 0, st>>>(npts, pts, flag, w, wvn, list,
                                                                                        count, out, ovf);
 }
-void launch_point_eigen(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
+void launch_point_single(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
                         const uint32_t* list, int count, double2* out, int* ovf) {
   k_eval_green<<<(count + 127) / 128, 128, 0, st>>>(npts, pts, flag, w, wvn, out, ovf, list, count);
 }

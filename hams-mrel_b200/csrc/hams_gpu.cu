@@ -3490,14 +3490,17 @@ extern "C" int hams_assemble(hams_ctx* c, const hams_wave* w, int32_t nbeta, con
 }
 
 // The points of hams_eval_green at a regular frequency in finite depth, branch
-// by branch: LINTON a warp per point, EIGENE and PIDCOCK with the kernel of the
-// assembly (three warps for 32 points of like series length), EIGEN a thread
-// per point.  One thread per point for all of them let the longest chain of a
+// by branch: LINTON a warp per point (many: a thread), EIGENE and PIDCOCK with the
+// kernel of the assembly (three warps for 32 points of like series length), EIGEN a
+// thread per point.  One thread per point for all of them let the longest chain of a
 // warp decide: 64 points over all branches 4.8 -> 0.77 ms, 200,003 points at
-// R/h >= 0.05 9.3 -> 3.6 ms (host copies included).
+// R/h >= 0.05 9.3 -> 3.4 ms (host copies included).
+// LINTON points per SM from which a thread takes each, as k_linton_rows_threads does
+// rows: 5,000 points at 2.5 rad/s in 40 m take 1.65 ms by threads and 1.72 by warps,
+// 60,000 points 4.1 and 23.1; at 0.3 rad/s a thread's chain alone takes 4 ms.
+constexpr int kLintonPointsPerSm = 32;
 static int point_series(hams_ctx* c, const WaveDev& wd, int npts, const double* pts, const int* flag, double2* out,
                         DBuf<uint32_t>& list, DBuf<uint32_t>& hist, DBuf<unsigned short>& key, DBuf<double>& work) {
-  TRY(list.alloc(npts));
   TRY(key.alloc(npts));
   TRY(hist.alloc(kPointBins));
   CU(cudaMemsetAsync(hist.p, 0, kPointBins * 4, c->st));
@@ -3508,17 +3511,25 @@ static int point_series(hams_ctx* c, const WaveDev& wd, int npts, const double* 
   CU(cudaStreamSynchronize(c->st));
   off[0] = 0;
   for (int b = 0; b < kPointBins; ++b) off[b + 1] = off[b] + cnt[b];
+  auto first = [&](int br) { return off[br * kPointTerms]; };
+  if (first(hams::kEigen) == 0) {  // one branch: as they come
+    launch_eval_green((npts + 127) / 128, c->st, npts, pts, flag, wd, c->wvn.p, out, c->ovf.p);
+    return launch_check(c);
+  }
+  TRY(list.alloc(npts));
   CU(cudaMemcpyAsync(hist.p, off, kPointBins * 4, cudaMemcpyHostToDevice, c->st));
   launch_point_file(c->st, npts, key.p, hist.p, list.p);
   TRY(launch_check(c));
-  auto first = [&](int br) { return off[br * kPointTerms]; };
   const uint32_t* lst = list.p;
   if (const int n = (int)(first(1) - first(0))) {
-    launch_point_linton(c->st, npts, pts, flag, wd, c->wvn.p, lst, n, out, c->ovf.p);
+    if (n < c->sms * kLintonPointsPerSm)
+      launch_point_linton(c->st, npts, pts, flag, wd, c->wvn.p, lst, n, out, c->ovf.p);
+    else
+      launch_point_single(c->st, npts, pts, flag, wd, c->wvn.p, lst, n, out, c->ovf.p);
     TRY(launch_check(c));
   }
   if (const int n = (int)(first(4) - first(3))) {
-    launch_point_eigen(c->st, npts, pts, flag, wd, c->wvn.p, lst + first(3), n, out, c->ovf.p);
+    launch_point_single(c->st, npts, pts, flag, wd, c->wvn.p, lst + first(3), n, out, c->ovf.p);
     TRY(launch_check(c));
   }
   const int most = (int)std::min<uint32_t>(std::max(first(2) - first(1), first(3) - first(2)), kPointChunk);
@@ -3556,6 +3567,24 @@ static int point_series(hams_ctx* c, const WaveDev& wd, int npts, const double* 
   return 0;
 }
 
+// Every point is EIGEN's (R/h >= 0.5), whose points a thread each suits: then the
+// lists, whose lengths the host waits for, cost more than they save (one point 91
+// us, 70 without, 60,000 points 1.03 ms, 0.95 without).  Up to kPointScan points the
+// host looks itself (about 1 ns a point), above that at the lists' lengths.
+constexpr int kPointScan = 16384;
+static bool all_eigen(int npts, const double* pts, double h) {
+  const double *xq = pts, *yq = xq + npts, *xp = yq + 2 * (size_t)npts, *yp = xp + npts, lim = 0.25 * h * h;
+  for (int k0 = 0; k0 < npts; k0 += 256) {
+    int near = 0;
+    for (int k = k0; k < std::min(npts, k0 + 256); ++k) {
+      const double dx = xq[k] - xp[k], dy = yq[k] - yp[k];
+      near |= !(dx * dx + dy * dy >= lim);
+    }
+    if (near) return false;
+  }
+  return true;
+}
+
 extern "C" int hams_eval_green(hams_ctx* c, const hams_wave* w, int32_t npts, const double* pts, const int32_t* flag,
                                double* grn) {
   g_err.clear();
@@ -3584,8 +3613,8 @@ extern "C" int hams_eval_green(hams_ctx* c, const hams_wave* w, int32_t npts, co
     const bool series = c->opts.depth >= 0.0 && !wd.limit;
     if (series) CU(cudaMemcpyAsync(c->wvn.p, w->wvn, HAMS_NK * 8, cudaMemcpyHostToDevice, c->st));
     CU(cudaMemsetAsync(c->ovf.p, 0, sizeof(int), c->st));
-    bool singly = !series;  // a thread per point
-    if (series) {
+    bool singly = !series || (npts <= kPointScan && all_eigen(npts, pts, wd.h));  // a thread per point
+    if (!singly) {
       const int rc = point_series(c, wd, npts, dp.p, df.p, dout.p, list, hist, key, work);
       if (rc == HAMS_ERR_NOMEM) {  // no room for the lists or tables
         g_err.clear();

@@ -105,7 +105,7 @@ void launch_point_bins(cudaStream_t st, int npts, const double* pts, double h, u
 void launch_point_file(cudaStream_t st, int npts, const unsigned short* key, uint32_t* next, uint32_t* list);
 void launch_point_linton(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
                          const uint32_t* list, int count, double2* out, int* ovf);
-void launch_point_eigen(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
+void launch_point_single(cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w, const double* wvn,
                         const uint32_t* list, int count, double2* out, int* ovf);
 void launch_point_series(int br, int ntmax, cudaStream_t st, int npts, const double* pts, const int* flag, WaveDev w,
                          const double* wvn, const uint32_t* list, int m, const PointWork& pw, double2* out, int* ovf);
