@@ -106,14 +106,15 @@ EPS_FN float eps_top_of(const double (&v)[kEpsRows], int from) {
 //     d has a significand of all ones (P. Markstein, IBM J. Res. Dev. 34, 1990);
 //   - there 1/d lies just above the middle of two numbers, and that step stays at
 //     the lower one, a power of two, but ends at the upper one from the upper
-//     one.  So the seed is raised by one unit of its upper word: e is then
-//     -2^-20, and the error of the three terms is upwards.
+//     one.  So the seed, whose lower word is zero, gets one of all ones (for the
+//     price of the zero): e is then -2^-20, and the error of the three terms is
+//     upwards.
 // tests/test_epsilon_gpu.py compares the bits with __drcp_rn.
 EPS_FN double eps_rcp(double d) {
 #if defined(__CUDA_ARCH__)
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = __hiloint2double(__double2hiint(y) + 1, __double2loint(y));
+  y = __hiloint2double(__double2hiint(y), -1);
   const double e = __fma_rn(-d, y, 1.0);
   y = __fma_rn(__fma_rn(y, e, y), e, y);
   return __fma_rn(y, __fma_rn(-d, y, 1.0), y);
