@@ -1488,12 +1488,6 @@ static int with_memory(hams_ctx* c, const F& f) {
 // Series lengths (EIGENE, then PIDCOCK) at which a bin's launch is split, so
 // that its shared memory fits the lengths it holds (launch_series).
 constexpr int kNtCut[2][2] = {{26, 38}, {66, 82}};
-// Pairs per SM from which it is: three launches hold more blocks per SM (two of 99
-// terms, five of 50), but each has a tail of its own.  PIDCOCK in one launch and in
-// three: 69,520 pairs 0.99 and 1.28 ms, 119,520 1.67 and 1.72, 165,984 2.57 and 2.78,
-// 192,800 2.87 and 2.66, 710,460 11.1 and 10.3; EIGENE 190,800 0.42 and 0.45, 1.23 M
-// 3.08 and 3.10, 11.4 M 14.0 and 13.6.
-constexpr int kSplitPairsPerSm = 1280;
 // Least cap on the radial table of a numbered branch (otherwise half the bytes
 // of A), and the table bytes of a chunk of pairs where distances are not
 // numbered: small enough to stay in L2 between the two kernels.
@@ -2252,9 +2246,9 @@ static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* 
     }
     // the longest series first, each launch with the shared memory of its own
     // lengths (and one more: the keys round distances with fused multiply-adds);
-    // a list below kSplitPairsPerSm stays one launch
+    // a list that one wave of blocks holds stays one launch
     long long cut[4] = {0, 0, 0, cnt};
-    if (br != hams::kEigen && cnt > (long long)c->sms * kSplitPairsPerSm) {
+    if (br != hams::kEigen && cnt > (long long)c->sms * 32 * 16) {
       cut[1] = c->nt_cut[bin][0] - c->bin_off[bin];
       cut[2] = c->nt_cut[bin][1] - c->bin_off[bin];
     }
