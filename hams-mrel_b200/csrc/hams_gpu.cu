@@ -190,18 +190,27 @@ __global__ void k_distance_heads(const double* __restrict__ r, long long count, 
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < count) head[t] = t == 0 || r[t] != r[t - 1];
 }
-// The number of each pair's distance (rid) and the distinct distances (ur) from
-// the sorted ones; entry idx of the sorted list is pair idx of the list's n1
-// first, or idx - n1 of its second part, which starts off2 further on.
+// rid of every pair, the distinct distances ur, and each branch's first and
+// last distance number (lim[2 br], lim[2 br + 1]); c2..c5 are the positions where
+// bins 2..5 start, counted from bin 1.
+__device__ __forceinline__ int series_class(long long pos, long long c2, long long c3, long long c4, long long c5) {
+  if (pos < c2) return hams::kPidcock;
+  if (pos < c3) return hams::kEigenE;
+  if (pos < c4) return hams::kEigen;
+  return pos < c5 ? hams::kEigenE : hams::kEigen;
+}
 __global__ void k_distance_rows(const double* __restrict__ r, const uint32_t* __restrict__ idx,
-                                const uint32_t* __restrict__ rank, long long count, long long n1, long long off2,
-                                uint32_t* __restrict__ rid, double* __restrict__ ur) {
+                                const uint32_t* __restrict__ rank, long long count, long long c2, long long c3,
+                                long long c4, long long c5, uint32_t* __restrict__ rid, double* __restrict__ ur,
+                                uint32_t* __restrict__ lim) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const uint32_t k = rank[t] - 1;
-  const long long i = idx[t];
-  rid[i < n1 ? i : off2 + i - n1] = k;
+  rid[idx[t]] = k;
   if (t == 0 || rank[t - 1] != rank[t]) ur[k] = r[t];
+  const int br = series_class(idx[t], c2, c3, c4, c5);
+  if (t == 0 || series_class(idx[t - 1], c2, c3, c4, c5) != br) atomicMin(&lim[2 * br], k);
+  if (t == count - 1 || series_class(idx[t + 1], c2, c3, c4, c5) != br) atomicMax(&lim[2 * br + 1], k);
 }
 // The pairs in the order of their distances, with the numbers and the distinct
 // distances; cut: where every per-th distance starts.
@@ -1260,17 +1269,18 @@ struct hams_ctx {
   // blocks); bin_off[7] = total
   long long bin_off[kBins + 1] = {};
   // radial tables (build_distances): the distance number of every pair of bins
-  // 1-5 (from bin 1 on) and the distinct distances, of a branch (rad_n of them,
-  // in ur[br]) or of one bin whose pairs are in the order of their distances
-  // (chunks not empty; ur[bin]); bins 4 and 5 have that order in a list of its
-  // own.  Pairs without numbers have a table row each, a chunk of them at a time
+  // 1-5 (from bin 1 on) and the distinct distances, of all branches together (ur[0];
+  // a branch's are rad_n from rad_base on, 0: its table is too large) or of one bin
+  // whose pairs are in the order of their distances (chunk not empty; ur[bin]); bins
+  // 4 and 5 have that order in a list of its own.  Pairs without numbers have a table
+  // row each, a chunk of them at a time
   struct RadChunk {
     long long pair;  // first pair of the bin, and its distance
     double r;
   };
   DBuf<uint32_t> rid, far_pairs;
   DBuf<double> ur[kBins];
-  uint32_t rad_n[4] = {};
+  uint32_t rad_base[4] = {}, rad_n[4] = {};
   std::vector<RadChunk> chunk[kBins];  // of kRadMin bytes of table each, and the end
   uint32_t chunk_n[kBins] = {};        // distances of the bin
   // LINTON rows: the row of every pair of bin 0 and a pair of each row (none:
@@ -1488,6 +1498,14 @@ static int with_memory(hams_ctx* c, const F& f) {
 // Series lengths (EIGENE, then PIDCOCK) at which a bin's launch is split, so
 // that its shared memory fits the lengths it holds (launch_series).
 constexpr int kNtCut[2][2] = {{26, 38}, {66, 82}};
+// Pairs per SM from which it is: three launches hold more blocks per SM (two of 99
+// terms, five of 50), but each has a tail of its own.  One frequency alone, PIDCOCK
+// in one launch and in three: 69,520 pairs 0.99 and 1.28 ms, 119,520 1.67 and 1.72,
+// 165,984 2.57 and 2.78, 192,800 2.87 and 2.66, 710,460 11.1 and 10.3; EIGENE 11.4 M
+// 14.0 and 13.6.  With other frequencies in flight, which fill the tails, three pay
+// earlier: a sweep whose lists are at 80,000-150,000 pairs takes 15.6 ms with the line
+// here and 16.3 with the line at 189,440.
+constexpr int kSplitPairsPerSm = 512;
 // Least cap on the radial table of a numbered branch (otherwise half the bytes
 // of A), and the table bytes of a chunk of pairs where distances are not
 // numbered: small enough to stay in L2 between the two kernels.
@@ -1497,13 +1515,13 @@ constexpr long long kLinChunk = 65536;  // LINTON pairs of a chunk without row n
 constexpr size_t kRadLean = (size_t)2 << 20;
 constexpr long long kLinLean = 4096, kRadLeast = 512;
 
-// The sorted distances of the pairs of one or two bins.
+// The sorted distances of the pairs of bins b0 to b1 - 1.
 struct DistSort {
   DBuf<double> r, r2;
   DBuf<uint32_t> idx, idx2, rank;  // rank: 1 + the number of the distance
   DBuf<char> tmp;
-  long long n1 = 0, count = 0;  // pairs of the first bin, of both
-  uint32_t nu = 0;              // distinct distances
+  long long count = 0;  // pairs
+  uint32_t nu = 0;      // distinct distances
   void release() {  // after the stream has been waited for
     r.release(true);
     r2.release(true);
@@ -1511,22 +1529,20 @@ struct DistSort {
     tmp.release(true);
   }
 };
-static int sort_distances(hams_ctx* c, int br, int b1, int b2, DistSort& d) {
-  const long long n1 = c->bin_off[b1 + 1] - c->bin_off[b1], n2 = b2 ? c->bin_off[b2 + 1] - c->bin_off[b2] : 0;
-  d.n1 = n1;
-  const long long n = d.count = n1 + n2;
+static int sort_distances(hams_ctx* c, int b0, int b1, DistSort& d) {
+  const long long n = d.count = c->bin_off[b1] - c->bin_off[b0];
   size_t t1 = 0, t2 = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, t1, d.r.p, d.r2.p, d.idx.p, d.idx2.p, (size_t)n, 0, 64, c->st);
   cub::DeviceScan::InclusiveSum(nullptr, t2, d.rank.p, d.rank.p, (size_t)n, c->st);
   for (DBuf<double>* x : {&d.r, &d.r2}) TRY(x->alloc(n));
   for (DBuf<uint32_t>* x : {&d.idx, &d.idx2, &d.rank}) TRY(x->alloc(n));
   TRY(d.tmp.alloc(std::max(t1, t2)));
-  for (int q = 0; q < 2; ++q) {
-    const long long m = q ? n2 : n1;
+  for (int b = b0; b < b1; ++b) {
+    const long long m = c->bin_off[b + 1] - c->bin_off[b];
     if (m <= 0) continue;
-    const uint32_t* lst = c->pairs.p + c->bin_off[q ? b2 : b1];
-    double* out = d.r.p + (q ? n1 : 0);
-    if (br == hams::kEigen) k_eigen_distance<<<(unsigned)((m + 255) / 256), 256, 0, c->st>>>(c->g, lst, m, out);
+    const uint32_t* lst = c->pairs.p + c->bin_off[b];
+    double* out = d.r.p + (c->bin_off[b] - c->bin_off[b0]);
+    if (b == 3 || b == 5) k_eigen_distance<<<(unsigned)((m + 255) / 256), 256, 0, c->st>>>(c->g, lst, m, out);
     else launch_series_distance(c->st, c->g, lst, m, out);
     TRY(launch_check(c));
   }
@@ -1578,48 +1594,55 @@ static int order_bin(hams_ctx* c, int br, int b, DistSort& d) {
 // distance has two pairs, (i, j) and (j, i)) is worked off in the order of the
 // distances instead, bin by bin: a chunk's table holds each of its distances once,
 // its pairs follow one another, and its series are of like length.
+static int number_distances(hams_ctx* c) {
+  const long long o1 = c->bin_off[1];
+  DistSort d;
+  DBuf<uint32_t> lim;
+  TRY(c->rid.alloc(c->bin_off[6] - o1));
+  TRY(lim.alloc(8));
+  TRY(sort_distances(c, 1, 6, d));
+  TRY(c->ur[0].alloc(d.nu));
+  uint32_t l[8];
+  for (int q = 0; q < 8; ++q) l[q] = q % 2 ? 0u : 0xffffffffu;
+  CU(cudaMemcpyAsync(lim.p, l, sizeof l, cudaMemcpyHostToDevice, c->st));
+  k_distance_rows<<<(unsigned)((d.count + 255) / 256), 256, 0, c->st>>>(
+      d.r2.p, d.idx2.p, d.rank.p, d.count, c->bin_off[2] - o1, c->bin_off[3] - o1, c->bin_off[4] - o1,
+      c->bin_off[5] - o1, c->rid.p, c->ur[0].p, lim.p);
+  TRY(launch_check(c));
+  CU(cudaMemcpyAsync(l, lim.p, sizeof l, cudaMemcpyDeviceToHost, c->st));
+  CU(cudaStreamSynchronize(c->st));
+  lim.release(true);
+  const size_t cap = std::max(kRadMin, (size_t)c->tn * c->n * 8);
+  bool numbered = false;
+  for (int br = hams::kPidcock; br <= hams::kEigen; ++br) {
+    if (l[2 * br] > l[2 * br + 1]) continue;  // no pair
+    const uint32_t n = l[2 * br + 1] - l[2 * br] + 1;
+    if ((size_t)n * rad_stride(br) * 8 <= cap) {
+      c->rad_base[br] = l[2 * br];
+      c->rad_n[br] = n;
+      numbered = true;
+      continue;
+    }
+    for (int b : {br, br + 2}) {
+      if ((br == hams::kPidcock && b != br) || c->bin_off[b + 1] <= c->bin_off[b]) continue;
+      TRY(sort_distances(c, b, b + 1, d));
+      TRY(order_bin(c, br, b, d));
+    }
+  }
+  d.release();
+  if (!numbered) c->ur[0].release(true);
+  return 0;
+}
 static int build_distances(hams_ctx* c) {
-  const long long o1 = c->bin_off[1], ns = c->bin_off[6] - o1;
-  for (uint32_t& n : c->rad_n) n = 0;
+  for (int br = 0; br < 4; ++br) c->rad_base[br] = c->rad_n[br] = 0;
   for (auto& q : c->chunk) q.clear();
   for (auto& u : c->ur) u.release(true);
   c->far_pairs.release(true);
   c->rid.release(true);
-  if (ns <= 0 || c->lean) return 0;
-  const size_t cap = std::max(kRadMin, (size_t)c->tn * c->n * 8);
-  int used = 0;
-  auto branch = [&](int br, int b2) -> int {
-    DistSort d;
-    const int bins[2] = {br, b2};
-    auto size = [&](int b) { return b ? c->bin_off[b + 1] - c->bin_off[b] : 0; };
-    if (size(br) + size(b2) <= 0) return 0;
-    const bool two = size(br) > 0 && size(b2) > 0;
-    TRY(sort_distances(c, br, br, b2, d));
-    if ((size_t)d.nu * rad_stride(br) * 8 <= cap) {
-      TRY(c->ur[br].alloc(d.nu));
-      k_distance_rows<<<(unsigned)((d.count + 255) / 256), 256, 0, c->st>>>(
-          d.r2.p, d.idx2.p, d.rank.p, d.count, d.n1, (b2 ? c->bin_off[b2] : 0) - c->bin_off[br],
-          c->rid.p + (c->bin_off[br] - o1), c->ur[br].p);
-      TRY(launch_check(c));
-      CU(cudaStreamSynchronize(c->st));
-      c->rad_n[br] = d.nu;
-      ++used;
-    } else {
-      for (int b : bins) {
-        if (size(b) <= 0) continue;
-        if (two) TRY(sort_distances(c, br, b, 0, d));
-        TRY(order_bin(c, br, b, d));
-        ++used;
-      }
-    }
-    d.release();
-    return 0;
-  };
-  int rc = c->rid.alloc(ns);
-  for (int br = hams::kPidcock; br <= hams::kEigen && !rc; ++br) rc = branch(br, br == hams::kPidcock ? 0 : br + 2);
-  if (rc && rc != HAMS_ERR_NOMEM) return rc;
-  if (rc) g_err.clear();  // the bins that are not done go without numbers
-  if (!used) c->rid.release(true);
+  if (c->bin_off[6] <= c->bin_off[1] || c->lean) return 0;
+  const int rc = number_distances(c);
+  if (rc != HAMS_ERR_NOMEM) return rc;
+  g_err.clear();  // what is not done goes without numbers
   return 0;
 }
 
@@ -1986,7 +2009,7 @@ static void view_pairs(hams_ctx* l, hams_ctx* c) {
   l->lrep.view(c->lrep);
   l->lin_rows = c->lin_rows;
   l->lean = c->lean;
-  for (int br = 0; br < 4; ++br) l->rad_n[br] = c->rad_n[br];
+  for (int br = 0; br < 4; ++br) l->rad_base[br] = c->rad_base[br], l->rad_n[br] = c->rad_n[br];
   for (int b = 0; b < kBins; ++b) l->nt_cut[b][0] = c->nt_cut[b][0], l->nt_cut[b][1] = c->nt_cut[b][1];
 }
 
@@ -2241,21 +2264,21 @@ static int series_pairs(hams_ctx* c, const WaveDev& wd, int br, const uint32_t* 
   const uint32_t* rid = bin ? c->rid.p + (c->bin_off[bin] - c->bin_off[1]) : nullptr;
   if (bin && c->rad_n[br]) {
     if (!c->rad_ready[br]) {
-      TRY(table(c->ur[br].p, nullptr, c->rad_n[br], ntmax));
+      TRY(table(c->ur[0].p + c->rad_base[br], nullptr, c->rad_n[br], ntmax));
       c->rad_ready[br] = true;
     }
     // the longest series first, each launch with the shared memory of its own
     // lengths (and one more: the keys round distances with fused multiply-adds);
-    // a list that one wave of blocks holds stays one launch
+    // a list below kSplitPairsPerSm stays one launch
     long long cut[4] = {0, 0, 0, cnt};
-    if (br != hams::kEigen && cnt > (long long)c->sms * 32 * 16) {
+    if (br != hams::kEigen && cnt > (long long)c->sms * kSplitPairsPerSm) {
       cut[1] = c->nt_cut[bin][0] - c->bin_off[bin];
       cut[2] = c->nt_cut[bin][1] - c->bin_off[bin];
     }
     for (int q = 2; q >= 0; --q) {
       const long long n = cut[q + 1] - cut[q];
       if (n <= 0) continue;
-      const RadTab rt{rid + cut[q], 0, c->rad_k[br].p, c->rad_j[br].p};
+      const RadTab rt{rid + cut[q], c->rad_base[br], c->rad_k[br].p, c->rad_j[br].p};
       TRY(launch(rt, lst + cut[q], n, q == 2 ? ntmax : kNtCut[br == hams::kPidcock][q] + 1));
     }
     return 0;
