@@ -164,8 +164,10 @@ __device__ __noinline__ double pidcock_image(int table, double r, double zf, dou
 // Issue-bound: about 18 instructions per table entry, 8 of them FP64 (the FP64
 // pipe is at half its rate).  Against one thread per pair with the Bessel
 // functions in the loop and the tables column by column in local memory
-// (5,400 panels, every pair): EIGENE 36.8 -> 13.3 ms for 11.2 M pairs, PIDCOCK
-// 16.0 -> 7.8 ms for 0.63 M.  Blocks of 4 or 6 rows (more warps, more columns
+// (5,400 panels, every pair): EIGENE 36.8 -> 13.9 ms for 11.2 M pairs, PIDCOCK
+// 16.0 -> 7.9 ms for 0.63 M; an irregular mesh of 5,400 panels in 150 m, its pairs in
+// the order of their distances, EIGENE 124.5 -> 92.9 ms for 26.8 M pairs and PIDCOCK
+// 59.4 -> 48.9 ms for 2.29 M with their tables.  Blocks of 4 or 6 rows (more warps, more columns
 // read and written per entry) measured the same within 3 %, one loop body for
 // all columns (less code, idle rows computed) 6-20 % slower.
 constexpr int kSerThreads = 96;
